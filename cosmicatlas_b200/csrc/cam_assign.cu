@@ -233,6 +233,12 @@ __global__ void brick_starts_kernel(const uint32_t *__restrict__ scanned, int nb
     }
 }
 
+// Pass 4: one CTA per brick, two CTAs of 512 threads per SM.  Bound by the
+// shared-memory atomics (one per stencil cell, 3.7 wavefronts each: 32 random
+// cells on 32 banks) and, for NGP and CIC, by the latency of the record
+// loads.  256^3, 16.8 M weighted particles: TSC 417 -> 341 us, CIC 200 ->
+// 156, NGP 136 -> 122 with the stencil on constant offsets from one address
+// (508 warp instructions per 32 TSC records before; 78% issue).
 template <int SCHEME, typename OutT>
 __global__ void __launch_bounds__(kDepositThreads, 2)
 deposit_kernel(const uint4 *__restrict__ payload, const uint32_t *__restrict__ start, uint32_t nrec,
@@ -240,7 +246,7 @@ deposit_kernel(const uint4 *__restrict__ payload, const uint32_t *__restrict__ s
                OutT *__restrict__ mesh, double *__restrict__ brick_sum, uint32_t slab,
                const uint32_t *__restrict__ slab_count)
 {
-    extern __shared__ uint32_t tile32[];
+    extern __shared__ __align__(16) uint32_t tile32[];
     __shared__ long long red[kDepositThreads / 32];
     const int B = blockIdx.x;
     const int B2 = B % g.nb[2];
@@ -249,19 +255,9 @@ deposit_kernel(const uint4 *__restrict__ payload, const uint32_t *__restrict__ s
     const int o[3] = {B0 * g.b[0], B1 * g.b[1], B2 * g.b[2]};
     const int e[3] = {min(g.b[0], g.n[0] - o[0]), min(g.b[1], g.n[1] - o[1]),
                       min(g.b[2], g.n[2] - o[2])};
-    const bool whole[3] = {g.nb[0] == 1, g.nb[1] == 1, g.nb[2] == 1};
-    // haloed tile: (b0 + 2) x (b1 + 2) x (b2 + 2) cells, low words then high words
-    const int T2 = g.b[2] + 2, T1 = g.b[1] + 2;
-    const int S1 = T2, S0 = T1 * T2;
-    const int cap = (g.b[0] + 2) * S0;
-    uint32_t *lo = tile32;
-    uint32_t *hi = tile32 + cap;
-    {
-        const int nw = 2 * cap;
-        uint4 *t4 = reinterpret_cast<uint4 *>(tile32);
-        for (int i = threadIdx.x; i < nw / 4; i += blockDim.x) t4[i] = make_uint4(0u, 0u, 0u, 0u);
-        for (int i = (nw & ~3) + threadIdx.x; i < nw; i += blockDim.x) tile32[i] = 0u;
-    }
+    const unsigned fold = (g.nb[0] == 1 ? 1u : 0u) | (g.nb[1] == 1 ? 2u : 0u) | (g.nb[2] == 1 ? 4u : 0u);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    zero_tile(tile32, e, threadIdx.x, kDepositThreads);
     __syncthreads();
 
     // records beyond the payload's capacity nrec were not written (overflow
@@ -273,38 +269,11 @@ deposit_kernel(const uint4 *__restrict__ payload, const uint32_t *__restrict__ s
     const int s = fixed_scale(wstat, weighted, end - beg);
     // 2^s as two exact factors (s may exceed the float exponent range)
     const float f1 = scalbnf(1.0f, s / 2), f2 = scalbnf(1.0f, s - s / 2);
-    // one record per iteration, the next one's load in flight meanwhile; a
-    // single inlined copy of the stencil (three conversion paths of up to 27
-    // cells each) keeps the loop within the instruction cache
-    uint32_t p = beg + threadIdx.x;
-    uint4 v = p < end ? payload[p] : make_uint4(0u, 0u, 0u, 0u);
-    for (; p < end; p += blockDim.x) {
-        const uint32_t pn = p + blockDim.x;
-        const uint4 vn = pn < end ? payload[pn] : make_uint4(0u, 0u, 0u, 0u);
-        deposit_record<SCHEME>(v, e, whole, S0, S1, f1, f2, nonneg, lo, hi);
-        v = vn;
-    }
+    deposit_records<SCHEME>(payload, beg, end, e, f1, f2, nonneg, tile32, warp, kDepositThreads / 32, lane);
     __syncthreads();
 
-    long long acc = 0;
     const double sc = ldexp(1.0, -s);
-    // interior cell i = (li * e1 + lj) * e2 + lk; a brick holds < 2^16 cells
-    const int ncell = e[0] * e[1] * e[2];
-    const unsigned e2 = (unsigned)e[2], e12 = (unsigned)(e[1] * e[2]);
-    const unsigned m2 = e2 > 1u ? (unsigned)((0x100000000ull + e2 - 1) / e2) : 0u;
-    const unsigned m12 = e12 > 1u ? (unsigned)((0x100000000ull + e12 - 1) / e12) : 0u;
-    const unsigned e1 = (unsigned)e[1];
-    for (int i = threadIdx.x; i < ncell; i += blockDim.x) {
-        const unsigned row = div_small((unsigned)i, e2, m2);  // li * e1 + lj
-        const unsigned lk = (unsigned)i - row * e2;
-        const unsigned lii = div_small((unsigned)i, e12, m12);
-        const unsigned lj = row - lii * e1;
-        const int c = (int)(lii + 1) * S0 + (int)(lj + 1) * S1 + (int)lk + 1;
-        const long long q = (long long)(((unsigned long long)hi[c] << 32) | lo[c]);
-        acc += q;
-        const int64_t gidx = ((int64_t)(o[0] + (int)lii) * g.n[1] + (o[1] + (int)lj)) * g.n[2] + (o[2] + (int)lk);
-        mesh[gidx] = convert_out<OutT>(q, s, sc);
-    }
+    long long acc = store_tile<OutT>(tile32, o, e, g.n, fold, s, sc, mesh, warp, kDepositThreads / 32, lane);
     // Deterministic block sum of the integer cell sums.
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, off);
@@ -519,8 +488,7 @@ static void assign_impl(cam_ctx *ctx, const float *x, const float *y, const floa
     CAM_LAUNCH_NAMED(ctx, "assign_bin_scatter", scatter_k, G2, kScatterThreads, 0, x, y, z, w, np, chunk2, g, (int)nb,
                      table, payload, d_lost, d_wmax, total, d_ovf, slab);
 
-    const size_t smem = (size_t)(g.b[0] + 2) * (g.b[1] + 2) * (g.b[2] + 2) * 2 * sizeof(uint32_t);
-    CAM_REQUIRE(smem <= 110 * 1024, CAM_E_UNSUPPORTED, "brick tile too large");
+    const size_t smem = (size_t)tile_words(g.b[0]) * sizeof(uint32_t);
     const int weighted = w != nullptr;
     auto launch_dep = [&](auto kern, auto *mesh) {
         smem_at_least(kern, smem);

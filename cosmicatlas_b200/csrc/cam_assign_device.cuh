@@ -286,12 +286,135 @@ __device__ __forceinline__ unsigned div_small(unsigned i, unsigned d, unsigned m
     return d == 1u ? i : __umulhi(i, m);
 }
 
-// Adds round(v) to the 64-bit fixed-point cell (lo, hi) with 32-bit shared
-// atomics: the low word's old value tells whether the add carried, and the
-// high word takes the upper 32 bits of the two's complement plus the carry.
-// |v| < 2^31 converts in 32 bits (the common case); larger contributions
-// (heavy particles when light ones set the scale) convert in 64 bits.
-__device__ __forceinline__ void add_fixed(uint32_t *lo, uint32_t *hi, float v)
+// ---- the deposit tile ------------------------------------------------------
+// Brick cell (li, lj, lk), each in [-1, e], has its 64-bit fixed-point sum in
+// two 32-bit words of shared memory: the low word at slot
+// (li + 1) kTileS0 + (lj + 1) kTileS1 + lk + 1 and the high word kTileHi
+// slots further.  The strides are those of the largest brick whatever the
+// brick's extent, so a record's whole stencil is one address plus constant
+// offsets.  The cells at -1 and e are a halo: a record deposits its stencil
+// with no per-cell test, and what lands in the halo belongs to neighbouring
+// bricks (which hold the particle's own record) and is dropped -- or, along
+// an axis that one brick spans, is the periodic image of the opposite edge
+// and is folded back when the tile is stored.
+constexpr int kTileS1 = 34;
+constexpr int kTileS0 = 18 * kTileS1;
+constexpr int kTileHi = 18 * kTileS0;
+// Shared-memory words of the tile of a brick of extent b0 along x.
+__host__ __device__ constexpr int tile_words(int b0) { return kTileHi + (b0 + 2) * kTileS0; }
+
+// Zeroes the slots of a brick of extents e; tid of nthr threads.
+__device__ __forceinline__ void zero_tile(uint32_t *tile, const int e[3], int tid, int nthr)
+{
+    const unsigned pw = (unsigned)((e[1] + 2) * kTileS1 + 3) / 4u;  // 16-byte words per plane
+    const unsigned m = (unsigned)((0x100000000ull + pw - 1) / pw);
+    const unsigned tot = (unsigned)(e[0] + 2) * pw;
+    uint4 *lo = reinterpret_cast<uint4 *>(tile), *hi = reinterpret_cast<uint4 *>(tile + kTileHi);
+    for (unsigned i = tid; i < tot; i += nthr) {
+        const unsigned pl = div_small(i, pw, m);
+        const unsigned at = pl * (kTileS0 / 4) + (i - pl * pw);
+        lo[at] = make_uint4(0u, 0u, 0u, 0u);
+        hi[at] = make_uint4(0u, 0u, 0u, 0u);
+    }
+}
+
+// One axis of a record: the stencil weights and the tile coordinate of the
+// first of its W consecutive cells.  A TSC stencil centred on a halo cell
+// (home cell -1 or e) would reach one cell past the halo: its weights are
+// moved by one so that the three cells lie inside, the one that left the
+// tile being replaced by a zero on the other side.
+template <int SCHEME>
+__device__ __forceinline__ int axis_base(uint32_t word, int e, float wa[3])
+{
+    int cl;
+    float t;
+    unpack_axis(word, cl, t);
+    if (SCHEME == CAM_NGP) return min(cl, e - 1) + 1;
+    if (SCHEME == CAM_CIC) {
+        wa[0] = 1.0f - t;
+        wa[1] = t;
+        return min(cl, e - 1) + 1;
+    }
+    const float hm = 0.5f - t, hp = 0.5f + t;
+    const float w0 = 0.5f * hm * hm, w1 = 0.75f - t * t, w2 = 0.5f * hp * hp;
+    const bool below = cl < 0, above = cl >= e;
+    wa[0] = below ? w1 : (above ? 0.0f : w0);
+    wa[1] = below ? w2 : (above ? w0 : w1);
+    wa[2] = below ? 0.0f : (above ? w1 : w2);
+    return below ? 0 : (above ? e - 1 : cl);
+}
+
+// Adds W consecutive non-negative contributions (units of the quantum) to
+// the cells at byte address a + OFF: one 32-bit shared atomic each, whose
+// old value tells whether the low word wrapped; a wrap adds one to the high
+// word.  Written as predicated instructions on immediate offsets: as C++
+// (pointer arithmetic per cell, a branch around the carry) a TSC cell cost
+// 18.8 warp instructions; see deposit_kernel.
+template <int W, int OFF>
+__device__ __forceinline__ void add_run(uint32_t a, uint32_t m0, uint32_t m1, uint32_t m2)
+{
+    constexpr int HI = OFF + 4 * kTileHi;
+    if constexpr (W == 1) {
+        asm volatile(
+            "{\n\t.reg .u32 o0;\n\t.reg .pred p0;\n\t"
+            "atom.shared.add.u32 o0, [%0+%2], %1;\n\t"
+            "add.u32 o0, o0, %1;\n\t"
+            "setp.lt.u32 p0, o0, %1;\n\t"
+            "@p0 red.shared.add.u32 [%0+%3], 1;\n\t}"
+            ::"r"(a), "r"(m0), "n"(OFF), "n"(HI) : "memory");
+    } else if constexpr (W == 2) {
+        asm volatile(
+            "{\n\t.reg .u32 o0, o1;\n\t.reg .pred p0, p1;\n\t"
+            "atom.shared.add.u32 o0, [%0+%3], %1;\n\t"
+            "atom.shared.add.u32 o1, [%0+%4], %2;\n\t"
+            "add.u32 o0, o0, %1;\n\t"
+            "add.u32 o1, o1, %2;\n\t"
+            "setp.lt.u32 p0, o0, %1;\n\t"
+            "setp.lt.u32 p1, o1, %2;\n\t"
+            "@p0 red.shared.add.u32 [%0+%5], 1;\n\t"
+            "@p1 red.shared.add.u32 [%0+%6], 1;\n\t}"
+            ::"r"(a), "r"(m0), "r"(m1), "n"(OFF), "n"(OFF + 4), "n"(HI), "n"(HI + 4) : "memory");
+    } else {
+        asm volatile(
+            "{\n\t.reg .u32 o0, o1, o2;\n\t.reg .pred p0, p1, p2;\n\t"
+            "atom.shared.add.u32 o0, [%0+%4], %1;\n\t"
+            "atom.shared.add.u32 o1, [%0+%5], %2;\n\t"
+            "atom.shared.add.u32 o2, [%0+%6], %3;\n\t"
+            "add.u32 o0, o0, %1;\n\t"
+            "add.u32 o1, o1, %2;\n\t"
+            "add.u32 o2, o2, %3;\n\t"
+            "setp.lt.u32 p0, o0, %1;\n\t"
+            "setp.lt.u32 p1, o1, %2;\n\t"
+            "setp.lt.u32 p2, o2, %3;\n\t"
+            "@p0 red.shared.add.u32 [%0+%7], 1;\n\t"
+            "@p1 red.shared.add.u32 [%0+%8], 1;\n\t"
+            "@p2 red.shared.add.u32 [%0+%9], 1;\n\t}"
+            ::"r"(a), "r"(m0), "r"(m1), "r"(m2), "n"(OFF), "n"(OFF + 4), "n"(OFF + 8), "n"(HI), "n"(HI + 4),
+            "n"(HI + 8) : "memory");
+    }
+}
+
+// The rows (i, j) of a non-negative stencil, unrolled at compile time.
+template <int SCHEME, int I, int J>
+__device__ __forceinline__ void add_rows(uint32_t a, float ws, float wi, const float w0[3], const float w1[3],
+                                         const float w2[3])
+{
+    constexpr int W = Stencil<SCHEME>::W;
+    const float ni = J == 0 ? ws * w0[I] : wi;
+    const float wij = ni * w1[J];
+    const uint32_t m0 = __float2uint_rn(wij * w2[0]);
+    const uint32_t m1 = W > 1 ? __float2uint_rn(wij * w2[1]) : 0u;
+    const uint32_t m2 = W > 2 ? __float2uint_rn(wij * w2[2]) : 0u;
+    add_run<W, 4 * (I * kTileS0 + J * kTileS1)>(a, m0, m1, m2);
+    if constexpr (J + 1 < W) add_rows<SCHEME, I, J + 1>(a, ws, ni, w0, w1, w2);
+    else if constexpr (I + 1 < W) add_rows<SCHEME, I + 1, 0>(a, ws, ni, w0, w1, w2);
+}
+
+// Any contribution: signed, or of 2^32 quanta and more (a particle much
+// heavier than the lightest, which sets the quantum).  |v| < 2^31 converts
+// in 32 bits, the rest in 64.  The high word takes the upper 32 bits of the
+// two's complement plus the carry of the low word.
+__device__ __forceinline__ void add_fixed(uint32_t *lo, float v)
 {
     uint32_t ql, qh;
     if (fabsf(v) < 2147483648.0f) {
@@ -306,122 +429,125 @@ __device__ __forceinline__ void add_fixed(uint32_t *lo, uint32_t *hi, float v)
     const uint32_t old = atomicAdd(lo, ql);
     const uint32_t carry = (uint32_t)(old + ql) < old ? 1u : 0u;
     const uint32_t hadd = qh + carry;
-    if (hadd) atomicAdd(hi, hadd);
+    if (hadd) atomicAdd(lo + kTileHi, hadd);
 }
 
-// The brick's tile has a one-cell halo on every side: tile cell
-// (li + 1, lj + 1, lk + 1) holds brick cell (li, lj, lk), li in [-1, e].  A
-// record deposits its whole stencil with no per-cell test; the halo cells
-// take the contributions that belong to neighbouring bricks (which get the
-// particle's own record) and are discarded.  Per axis, a stencil point
-// further out than the halo (TSC only: home cell -1 or e) gets weight zero
-// and the nearest halo index, so it adds nothing.  Along an axis that one
-// brick spans (nb = 1) the stencil wraps periodically inside the brick.
+// The record's stencil by add_fixed.  Not inlined: few records need it, and
+// its 27 general conversions would crowd the common path out of the
+// instruction cache.
+struct RecordWeights {
+    float w[3][3];
+};
 template <int SCHEME>
-__device__ __forceinline__ void axis_stencil(uint32_t word, int e, bool whole, float wa[3], int ia[3])
+__device__ __noinline__ void deposit_general(RecordWeights r, float ws, uint32_t *at)
 {
-    using St = Stencil<SCHEME>;
-    int cl;
-    float t;
-    unpack_axis(word, cl, t);
-    if (SCHEME == CAM_NGP) {
-        wa[0] = 1.0f;
-    } else if (SCHEME == CAM_CIC) {
-        wa[0] = 1.0f - t;
-        wa[1] = t;
-    } else {
-        const float hm = 0.5f - t, hp = 0.5f + t;
-        wa[0] = 0.5f * hm * hm;
-        wa[1] = 0.75f - t * t;
-        wa[2] = 0.5f * hp * hp;
-    }
-#pragma unroll
-    for (int i = 0; i < St::W; ++i) {
-        int lc = cl + St::FIRST + i;
-        if (whole) {
-            lc += lc < 0 ? e : (lc >= e ? -e : 0);
-        } else if (lc < -1 || lc > e) {
-            wa[i] = 0.0f;
-            lc = lc < -1 ? -1 : e;
+    constexpr int W = Stencil<SCHEME>::W;
+#pragma unroll 1
+    for (int i = 0; i < W; ++i)
+#pragma unroll 1
+        for (int j = 0; j < W; ++j) {
+            const float wij = SCHEME == CAM_NGP ? ws : ws * r.w[0][i] * r.w[1][j];
+#pragma unroll 1
+            for (int k = 0; k < W; ++k)
+                add_fixed(at + i * kTileS0 + j * kTileS1 + k, SCHEME == CAM_NGP ? wij : wij * r.w[2][k]);
         }
-        ia[i] = lc + 1;
+}
+
+// The payload records [beg, end) of one brick into its tile; whole warps
+// take 32 consecutive records (warp `warp` of nwarp), the next 32 already
+// on their way.  Lanes past the end deposit zeros.  ws = weight * 2^s; the
+// stencil weights are <= 1 and, up to a rounding next to a cell face (CIC),
+// non-negative, so |ws| < 2^32 bounds every contribution; a warp with any
+// record that this does not hold for takes the general form (the same
+// integers).
+template <int SCHEME>
+__device__ __forceinline__ void deposit_records(const uint4 *__restrict__ payload, uint32_t beg, uint32_t end,
+                                                const int e[3], float f1, float f2, bool nonneg, uint32_t *tile,
+                                                int warp, int nwarp, int lane)
+{
+    const uint32_t tile_addr = (uint32_t)__cvta_generic_to_shared(tile);
+    const uint32_t zero_word = (8u << 26) | (1u << 24);  // home cell 0, offset 0
+    const uint4 none = make_uint4(zero_word, zero_word, zero_word, 0u);
+    const uint32_t step = 32u * (uint32_t)nwarp;
+    uint32_t p = beg + 32u * (uint32_t)warp + (uint32_t)lane;
+    uint4 v = p < end ? payload[p] : none;
+    for (uint32_t left = beg + 32u * (uint32_t)warp; left < end; left += step) {
+        p += step;
+        const uint4 vn = p < end ? payload[p] : none;
+        float w0[3] = {1.f, 1.f, 1.f}, w1[3] = {1.f, 1.f, 1.f}, w2[3] = {1.f, 1.f, 1.f};
+        const int i0 = axis_base<SCHEME>(v.x, e[0], w0);
+        const int i1 = axis_base<SCHEME>(v.y, e[1], w1);
+        const int i2 = axis_base<SCHEME>(v.z, e[2], w2);
+        const float ws = (__uint_as_float(v.w) * f1) * f2;
+        const int slot = i0 * kTileS0 + i1 * kTileS1 + i2;
+        bool fast = nonneg && ws < 4294967296.0f;
+        if (SCHEME == CAM_CIC)
+            fast = fast && w0[0] >= 0.f && w0[1] >= 0.f && w1[0] >= 0.f && w1[1] >= 0.f && w2[0] >= 0.f && w2[1] >= 0.f;
+        if (__all_sync(0xffffffffu, fast)) {
+            add_rows<SCHEME, 0, 0>(tile_addr + 4u * (uint32_t)slot, ws, ws, w0, w1, w2);
+        } else {
+            const RecordWeights r = {{{w0[0], w0[1], w0[2]}, {w1[0], w1[1], w1[2]}, {w2[0], w2[1], w2[2]}}};
+            deposit_general<SCHEME>(r, ws, tile + slot);
+        }
+        v = vn;
     }
 }
 
-// Adds the non-negative contribution v < 2^32 (units of the quantum) to the
-// cell (lo, hi): one 32-bit atomic, and a carry into the high word when the
-// low word wraps.  v < 2^22 converts by adding 2^23 (the float's mantissa
-// then holds round(v)); larger values convert with cvt.
-template <bool SMALL>
-__device__ __forceinline__ void add_nonneg(uint32_t *lo, uint32_t *hi, float v)
+// Sum of the tile's images of interior coordinates (li, lj, lk): itself and,
+// along axes that one brick spans, the halo cells that are its periodic
+// images (fold: bit a set for such an axis).
+__device__ __forceinline__ long long folded_cell(const uint32_t *tile, int li, int lj, int lk, const int e[3],
+                                                 unsigned fold)
 {
-    uint32_t m;
-    if (SMALL) m = __float_as_uint(__fadd_rn(v, 8388608.0f)) - 0x4b000000u;
-    else m = __float2uint_rn(v);
-    const uint32_t old = atomicAdd(lo, m);
-    if (old + m < old) atomicAdd(hi, 1u);
-}
-
-// TIER 0: every contribution < 2^22 and >= 0; 1: < 2^32 and >= 0; 2: any.
-// The whole stencil is written, halo cells included (they are discarded):
-// skipping the stencil rows that lie in the halo along x or y saved
-// atomics but cost more in branches (TSC deposit 0.257 -> 0.304 ms per
-// 256^3 job with the skip).
-template <int SCHEME, int TIER>
-__device__ __forceinline__ void deposit_stencil(const float wa[3][3], const int ia[3][3], int S0, int S1, float ws,
-                                                uint32_t *lo, uint32_t *hi)
-{
-    using St = Stencil<SCHEME>;
+    const int l[3] = {li, lj, lk};
+    int img[3][3], cnt[3];
 #pragma unroll
-    for (int i = 0; i < St::W; ++i) {
-#pragma unroll
-        for (int j = 0; j < St::W; ++j) {
-            const float wij = ws * wa[0][i] * wa[1][j];
-            const int row = ia[0][i] * S0 + ia[1][j] * S1;
-#pragma unroll
-            for (int k = 0; k < St::W; ++k) {
-                const int c = row + ia[2][k];
-                const float v = wij * wa[2][k];
-                if (TIER == 0) add_nonneg<true>(lo + c, hi + c, v);
-                else if (TIER == 1) add_nonneg<false>(lo + c, hi + c, v);
-                else add_fixed(lo + c, hi + c, v);
+    for (int a = 0; a < 3; ++a) {
+        cnt[a] = 1;
+        img[a][0] = l[a] + 1;
+        img[a][1] = img[a][2] = 0;
+        if ((fold >> a) & 1u) {
+            if (l[a] == 0) img[a][cnt[a]++] = e[a] + 1;
+            if (l[a] == e[a] - 1) {
+                if (cnt[a] == 1) img[a][1] = 0;
+                else img[a][2] = 0;
+                ++cnt[a];
             }
         }
     }
+    unsigned long long q = 0;
+    for (int i = 0; i < cnt[0]; ++i)
+        for (int j = 0; j < cnt[1]; ++j)
+            for (int k = 0; k < cnt[2]; ++k) {
+                const int c = img[0][i] * kTileS0 + img[1][j] * kTileS1 + img[2][k];
+                q += ((unsigned long long)tile[c + kTileHi] << 32) | tile[c];
+            }
+    return (long long)q;
 }
 
-// One payload record into the haloed tile.  ws = weight * 2^s; the stencil
-// weights are <= 1 (a TSC weight can dip below zero by ~1e-7 next to a cell
-// face: such records take the signed path), so |ws| bounds every
-// contribution and picks the conversion once per record.
-template <int SCHEME>
-__device__ __forceinline__ void deposit_record(const uint4 v, const int e[3], const bool whole[3], int S0, int S1,
-                                               float f1, float f2, bool nonneg, uint32_t *lo, uint32_t *hi)
+// The tile's interior cells as OutT into the mesh (o: the brick's first
+// cell, n: mesh sides), one row along z per warp; returns this thread's sum
+// of the integer cell sums.
+template <typename OutT>
+__device__ __forceinline__ long long store_tile(const uint32_t *tile, const int o[3], const int e[3], const int n[3],
+                                                unsigned fold, int s, double sc, OutT *__restrict__ mesh, int warp,
+                                                int nwarp, int lane)
 {
-    float wa[3][3];
-    int ia[3][3];
-    axis_stencil<SCHEME>(v.x, e[0], whole[0], wa[0], ia[0]);
-    axis_stencil<SCHEME>(v.y, e[1], whole[1], wa[1], ia[1]);
-    axis_stencil<SCHEME>(v.z, e[2], whole[2], wa[2], ia[2]);
-    const float ws = (__uint_as_float(v.w) * f1) * f2;
-    bool pos = nonneg;
-    if (SCHEME == CAM_TSC) {
-#pragma unroll
-        for (int a = 0; a < 3; ++a) pos = pos && wa[a][0] >= 0.0f && wa[a][2] >= 0.0f;
-    } else if (SCHEME == CAM_CIC) {
-#pragma unroll
-        for (int a = 0; a < 3; ++a) pos = pos && wa[a][0] >= 0.0f && wa[a][1] >= 0.0f;
+    long long acc = 0;
+    const unsigned e1 = (unsigned)e[1];
+    const unsigned m1 = e1 > 1u ? (unsigned)((0x100000000ull + e1 - 1) / e1) : 0u;
+    if (lane < e[2]) {
+        for (int r = warp; r < e[0] * e[1]; r += nwarp) {
+            const int li = (int)div_small((unsigned)r, e1, m1), lj = r - li * e[1];
+            const int c = (li + 1) * kTileS0 + (lj + 1) * kTileS1 + lane + 1;
+            long long q;
+            if (fold == 0u) q = (long long)(((unsigned long long)tile[c + kTileHi] << 32) | tile[c]);
+            else q = folded_cell(tile, li, lj, lane, e, fold);
+            acc += q;
+            mesh[((int64_t)(o[0] + li) * n[1] + (o[1] + lj)) * n[2] + o[2] + lane] = convert_out<OutT>(q, s, sc);
+        }
     }
-    // One conversion path for all lanes of the warp here (the most general
-    // one any of them needs): lanes of a warp hold unrelated records, and
-    // per-lane paths would run one after the other.  Every path gives the
-    // same integer sums.
-    const int tier = (pos && ws < 4194304.0f) ? 0 : ((pos && ws < 4294967296.0f) ? 1 : 2);
-    const unsigned act = __activemask();
-    const int wt = __reduce_max_sync(act, (unsigned)tier);
-    if (wt == 0) deposit_stencil<SCHEME, 0>(wa, ia, S0, S1, ws, lo, hi);
-    else if (wt == 1) deposit_stencil<SCHEME, 1>(wa, ia, S0, S1, ws, lo, hi);
-    else deposit_stencil<SCHEME, 2>(wa, ia, S0, S1, ws, lo, hi);
+    return acc;
 }
 
 // Pass 4: one CTA per brick, cell sums in 64-bit fixed point of quantum

@@ -210,14 +210,10 @@ __device__ void dl_assign(const DlJob &J, const DlScratch &S, uint4 *payload, fl
         bin_one<SCHEME, true, false, 1>(J.x[p], J.y[p], J.z[p], weighted ? J.w[p] : 1.0f, weighted, g, 1, 0, nullptr,
                                         sh.hist, payload, S.pcap, sh.ovf, dummy_lost, dummy_wmax, dummy_neg);
     __syncthreads();
-    // deposit, brick by brick (the same tile layout as deposit_kernel)
-    const int T2 = g.b[2] + 2, T1 = g.b[1] + 2;
-    const int S1 = T2, S0 = T1 * T2;
-    const int cap = (g.b[0] + 2) * S0;
-    uint32_t *lo = reinterpret_cast<uint32_t *>(sh.big);
-    uint32_t *hi = lo + cap;
-    long long *red = reinterpret_cast<long long *>(hi + cap);
-    const bool whole[3] = {g.nb[0] == 1, g.nb[1] == 1, g.nb[2] == 1};
+    // deposit, brick by brick (the tile of deposit_kernel)
+    uint32_t *tile = reinterpret_cast<uint32_t *>(sh.big);
+    long long *red = reinterpret_cast<long long *>(tile + tile_words(g.b[0]));
+    const unsigned fold = (g.nb[0] == 1 ? 1u : 0u) | (g.nb[1] == 1 ? 2u : 0u) | (g.nb[2] == 1 ? 4u : 0u);
     const bool nonneg = !weighted || sh.wstat[1] == 0u;
     for (int B = 0; B < nb; ++B) {
         const int B2 = B % g.nb[2];
@@ -225,30 +221,15 @@ __device__ void dl_assign(const DlJob &J, const DlScratch &S, uint4 *payload, fl
         const int B0 = B / (g.nb[2] * g.nb[1]);
         const int o[3] = {B0 * g.b[0], B1 * g.b[1], B2 * g.b[2]};
         const int e[3] = {min(g.b[0], g.n[0] - o[0]), min(g.b[1], g.n[1] - o[1]), min(g.b[2], g.n[2] - o[2])};
-        {
-            uint4 *t4 = reinterpret_cast<uint4 *>(lo);
-            const int nw = 2 * cap;
-            for (int i = tid; i < nw / 4; i += kDlThreads) t4[i] = make_uint4(0u, 0u, 0u, 0u);
-            for (int i = (nw & ~3) + tid; i < nw; i += kDlThreads) lo[i] = 0u;
-        }
+        zero_tile(tile, e, tid, kDlThreads);
         __syncthreads();
         const uint32_t beg = sh.start[B], end = sh.start[B + 1];
         const int s = fixed_scale(sh.wstat, weighted ? 1 : 0, end - beg);
         const float f1 = scalbnf(1.0f, s / 2), f2 = scalbnf(1.0f, s - s / 2);
-        for (uint32_t p = beg + tid; p < end; p += kDlThreads)
-            deposit_record<SCHEME>(payload[p], e, whole, S0, S1, f1, f2, nonneg, lo, hi);
+        deposit_records<SCHEME>(payload, beg, end, e, f1, f2, nonneg, tile, tid >> 5, kDlWarps, tid & 31);
         __syncthreads();
-        long long acc = 0;
         const double sc = ldexp(1.0, -s);
-        const int ncell = e[0] * e[1] * e[2];
-        for (int i = tid; i < ncell; i += kDlThreads) {
-            const int lk = i % e[2], row = i / e[2];
-            const int lj = row % e[1], li = row / e[1];
-            const int c = (li + 1) * S0 + (lj + 1) * S1 + lk + 1;
-            const long long q = (long long)(((unsigned long long)hi[c] << 32) | lo[c]);
-            acc += q;
-            mesh[((int64_t)(o[0] + li) * g.n[1] + (o[1] + lj)) * g.n[2] + (o[2] + lk)] = convert_out<float>(q, s, sc);
-        }
+        long long acc = store_tile<float>(tile, o, e, g.n, fold, s, sc, mesh, tid >> 5, kDlWarps, tid & 31);
 #pragma unroll
         for (int off = 16; off > 0; off >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, off);
         if ((tid & 31) == 0) red[tid >> 5] = acc;

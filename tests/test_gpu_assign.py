@@ -276,3 +276,28 @@ def test_mesh_384_vs_oracle(ctx, scheme):
     ref, lost = orc.assign_f64_mt(scheme, x, y, z, w, orc.Grid.cubic(n, box))
     assert got.n_lost == lost
     assert rel_err_cells(got.mesh, ref, float(np.mean(w, dtype=np.float64))) <= 1e-5
+
+
+@pytest.mark.parametrize("scheme", SCHEMES)
+@pytest.mark.parametrize("signed", [False, True])
+@pytest.mark.parametrize("n", [(1, 5, 33), (16, 1, 64), (2, 40, 31), (17, 34, 65), (3, 3, 3)])
+def test_deposit_tile_edges(ctx, scheme, signed, n):
+    # axes that one brick spans (the tile's halo is folded back, down to one
+    # cell per axis), bricks of 2 and 15 cells, rows of 2 to 32 cells, both
+    # forms of the deposit (signed weights take the general one)
+    rng = np.random.default_rng(100 * n[0] + n[2] + scheme)
+    L = tuple(10.0 * k for k in n)
+    npart = 20_000
+    xs = [rng.uniform(0.0, side, npart).astype(np.float32) for side in L]
+    for a in range(3):
+        e = edge_positions(L[a], n[a])
+        xs[a][a * 20:a * 20 + len(e)] = e
+    w = synth.halo_masses(npart, seed=12) if signed else None
+    if signed:
+        w[::3] *= -1.0
+    g = make_grid(n, L)
+    r = ctx.assign(*xs, w, g, scheme, F64)
+    ref, lost = orc.assign_f64(scheme, *xs, w, orc.Grid(n, L, tuple(g.d), (0.0, 0.0, 0.0)))
+    assert r.n_lost == lost
+    unit = 1.0 if w is None else float(np.mean(np.abs(w)))
+    assert rel_err_cells(r.mesh, ref, unit) <= 1e-5
