@@ -42,108 +42,294 @@ constexpr int kSmemBricks = 16384;  // per-CTA brick histogram in shared memory 
 using namespace asg;
 
 
-// Calls one(x, y, z, w) for the particles [p0, p1), the threads of the CTA
-// taking consecutive particles; with VEC (16-byte aligned arrays, p0 a
-// multiple of 4) four per thread per iteration from float4 loads.  Unit
-// weights when w is null.
-template <bool VEC, typename F>
-__device__ __forceinline__ void for_chunk(const float *__restrict__ x, const float *__restrict__ y,
-                                          const float *__restrict__ z, const float *__restrict__ w, int64_t p0,
-                                          int64_t p1, F &one)
+// Calls one(i, x, y, z, w) for the particles p0 + i, i in [0, count), the
+// threads of the CTA taking consecutive particles, the next one's loads in
+// flight meanwhile.  Scalar loads: 128 bytes per warp and array either way,
+// and no selects to pick a particle out of a float4.  Unit weights when w is
+// null.
+template <typename F>
+__device__ __forceinline__ void for_particles(const float *__restrict__ x, const float *__restrict__ y,
+                                              const float *__restrict__ z, const float *__restrict__ w, int64_t p0,
+                                              int64_t count, F &&one)
 {
     const bool weighted = w != nullptr;
-    int64_t ptail = p0;
-    if (VEC) {
-        const int64_t q1 = p0 + ((p1 - p0) & ~(int64_t)3);
-        for (int64_t p = p0 + 4 * (int64_t)threadIdx.x; p < q1; p += 4 * (int64_t)blockDim.x) {
-            const float4 X = __ldcs(reinterpret_cast<const float4 *>(x + p));
-            const float4 Y = __ldcs(reinterpret_cast<const float4 *>(y + p));
-            const float4 Z = __ldcs(reinterpret_cast<const float4 *>(z + p));
-            const float4 Wt = weighted ? __ldcs(reinterpret_cast<const float4 *>(w + p)) : make_float4(1.f, 1.f, 1.f, 1.f);
-            // one copy of the particle body, not four: the inlined body is
-            // large and four copies overflowed the instruction cache
-#pragma unroll 1
-            for (int k = 0; k < 4; ++k) {
-                const float px = k == 0 ? X.x : (k == 1 ? X.y : (k == 2 ? X.z : X.w));
-                const float py = k == 0 ? Y.x : (k == 1 ? Y.y : (k == 2 ? Y.z : Y.w));
-                const float pz = k == 0 ? Z.x : (k == 1 ? Z.y : (k == 2 ? Z.z : Z.w));
-                const float pw = k == 0 ? Wt.x : (k == 1 ? Wt.y : (k == 2 ? Wt.z : Wt.w));
-                one(px, py, pz, pw);
-            }
-        }
-        ptail = q1;
+    int64_t i = threadIdx.x;
+    float ax = 0.f, ay = 0.f, az = 0.f, aw = 1.f;
+    if (i < count) {
+        ax = __ldcs(x + p0 + i);
+        ay = __ldcs(y + p0 + i);
+        az = __ldcs(z + p0 + i);
+        if (weighted) aw = __ldcs(w + p0 + i);
     }
-    for (int64_t p = ptail + threadIdx.x; p < p1; p += blockDim.x)
-        one(__ldcs(x + p), __ldcs(y + p), __ldcs(z + p), weighted ? __ldcs(w + p) : 1.0f);
+#pragma unroll 1
+    while (i < count) {
+        const int64_t j = i + blockDim.x;
+        float bx = 0.f, by = 0.f, bz = 0.f, bw = 1.f;
+        if (j < count) {
+            bx = __ldcs(x + p0 + j);
+            by = __ldcs(y + p0 + j);
+            bz = __ldcs(z + p0 + j);
+            if (weighted) bw = __ldcs(w + p0 + j);
+        }
+        one((int)i, ax, ay, az, aw);
+        ax = bx;
+        ay = by;
+        az = bz;
+        aw = bw;
+        i = j;
+    }
 }
 
+// Adds the CTA's lost count and weight statistics, one atomic per warp.
+__device__ __forceinline__ void flush_stats(unsigned long long lost_n, unsigned int wmax, unsigned int neg,
+                                            unsigned int wminc, unsigned long long *__restrict__ lost,
+                                            unsigned int *__restrict__ wstat)
+{
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) {
+        lost_n += __shfl_down_sync(0xffffffffu, lost_n, off);
+        wmax = max(wmax, __shfl_down_sync(0xffffffffu, wmax, off));
+        neg |= __shfl_down_sync(0xffffffffu, neg, off);
+        wminc = max(wminc, __shfl_down_sync(0xffffffffu, wminc, off));
+    }
+    if ((threadIdx.x & 31) == 0) {
+        if (lost_n) atomicAdd(lost, lost_n);
+        if (wmax) atomicMax(wstat, wmax);
+        if (neg) atomicOr(wstat + 1, 1u);  // some weight is negative
+        if (wminc) atomicMax(wstat + 6, wminc);  // smallest nonzero |w|
+    }
+}
 
-// Passes 1 and 3.  Block `blk` handles particles [blk * chunk, (blk+1) * chunk)
-// (chunk a multiple of 4).
-//   COUNT   : table[brick * kCursorStride] += number of payloads for the
-//             brick (through a per-CTA shared-memory histogram when SMEM,
-//             nb <= kSmemBricks), plus lost particles and max |w|.
-//   SCATTER : table[brick * kCursorStride] is the brick's append cursor (the
-//             exclusive scan of the counts); every payload takes the next
-//             slot of its brick with one global atomic, and its words are
-//             packed while the atomic is in flight.  A brick's records are appended
-//             contiguously by all CTAs, so its few open 128-byte lines fill
-//             in L2 and are written back whole.  The order of records inside
-//             a brick varies from run to run; the deposit's integer sums do
-//             not depend on it.
-// VEC: 16-byte aligned arrays, four particles per thread per iteration
-// (float4 loads).
-// SLAB (scatter only): records into per-brick slabs of `slab` records, the
-// weight statistics and lost count gathered here (no count pass).
-template <int SCHEME, bool SCATTER, bool SMEM, bool VEC, bool SLAB = false>
+// Pass 1.  Block b counts the records of particles [b chunk, (b+1) chunk)
+// per brick into table[brick * kCursorStride] (through a shared-memory
+// histogram when SMEM, nb <= kSmemBricks), plus lost particles and the
+// weight statistics.
+template <int SCHEME, bool SMEM>
 __global__ void __launch_bounds__(kBinThreads)
-bin_kernel(const float *__restrict__ x, const float *__restrict__ y, const float *__restrict__ z,
-           const float *__restrict__ w, int64_t np, int64_t chunk, AssignGeom g, int nb,
-           uint32_t *__restrict__ table, uint4 *__restrict__ payload, unsigned long long *__restrict__ lost,
-           unsigned int *__restrict__ wmax_bits, uint64_t cap, unsigned int *__restrict__ ovf, uint32_t slab)
+count_kernel(const float *__restrict__ x, const float *__restrict__ y, const float *__restrict__ z,
+             const float *__restrict__ w, int64_t np, int64_t chunk, const __grid_constant__ AssignGeom g, int nb,
+             uint32_t *__restrict__ table, unsigned long long *__restrict__ lost, unsigned int *__restrict__ wstat)
 {
     extern __shared__ uint32_t hist[];
-    constexpr bool kHist = SMEM && !SCATTER;
-    const int G = gridDim.x, blk = blockIdx.x;
-    const int lane = threadIdx.x & 31;
-    if (kHist) {
+    if (SMEM) {
         for (int i = threadIdx.x; i < nb; i += blockDim.x) hist[i] = 0u;
         __syncthreads();
     }
     unsigned long long my_lost = 0;
     unsigned int my_wmax = 0, my_neg = 0, my_wminc = 0;
     const bool weighted = w != nullptr;
-    auto one = [&](float px, float py, float pz, float wt) {
-        if (SCATTER)
-            bin_one<SCHEME, true, false>(px, py, pz, wt, weighted, g, G, blk, hist, table, payload, cap, ovf,
-                                         my_lost, my_wmax, my_neg, SLAB ? &my_wminc : nullptr, SLAB ? slab : 0u);
-        else
-            count_one<SCHEME, kHist>(px, py, pz, wt, weighted, g, hist, table, my_lost, my_wmax, my_neg,
-                                     my_wminc);
-    };
-    for_chunk<VEC>(x, y, z, w, (int64_t)blk * chunk, min(np, (int64_t)blk * chunk + chunk), one);
-    if (!SCATTER || SLAB) {
-        // Warp reductions, one atomic per warp (the scatter's when it writes
-        // slabs: there is no count pass then).
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) {
-            my_lost += __shfl_down_sync(0xffffffffu, my_lost, off);
-            my_wmax = max(my_wmax, __shfl_down_sync(0xffffffffu, my_wmax, off));
-            my_neg |= __shfl_down_sync(0xffffffffu, my_neg, off);
-            my_wminc = max(my_wminc, __shfl_down_sync(0xffffffffu, my_wminc, off));
-        }
-        if (lane == 0) {
-            if (my_lost) atomicAdd(lost, my_lost);
-            if (my_wmax) atomicMax(wmax_bits, my_wmax);
-            if (my_neg) atomicOr(wmax_bits + 1, 1u);  // some weight is negative
-            if (my_wminc) atomicMax(wmax_bits + 6, my_wminc);  // smallest nonzero |w|
-        }
-        if (kHist) {
-            __syncthreads();
-            for (int i = threadIdx.x; i < nb; i += blockDim.x)
-                if (hist[i]) atomicAdd(table + (int64_t)i * kCursorStride, hist[i]);
-        }
+    const int64_t p0 = (int64_t)blockIdx.x * chunk;
+    for_particles(x, y, z, w, p0, min(chunk, np - p0), [&](int, float px, float py, float pz, float wt) {
+        count_one<SCHEME, SMEM>(px, py, pz, wt, weighted, g, hist, table, my_lost, my_wmax, my_neg, my_wminc);
+    });
+    flush_stats(my_lost, my_wmax, my_neg, my_wminc, lost, wstat);
+    if (SMEM) {
+        __syncthreads();
+        for (int i = threadIdx.x; i < nb; i += blockDim.x)
+            if (hist[i]) atomicAdd(table + (int64_t)i * kCursorStride, hist[i]);
     }
+}
+
+// Pass 3 for meshes with more bricks than a staged tile sorts (kStageBricks):
+// every record takes the next slot of its brick's cursor (table, the
+// exclusive scan of the counts or zero for slabs) with one global atomic.  A
+// brick's records are appended contiguously by all CTAs, so its few open
+// 128-byte lines fill in L2 and are written back whole.  The order of records
+// inside a brick varies from run to run; the deposit's integer sums do not
+// depend on it.  SLAB: records into per-brick slabs, with the weight
+// statistics and lost count gathered here (no count pass).
+template <int SCHEME, bool SLAB>
+__global__ void __launch_bounds__(kScatterThreads, 2)
+append_kernel(const float *__restrict__ x, const float *__restrict__ y, const float *__restrict__ z,
+              const float *__restrict__ w, int64_t np, int64_t chunk, const __grid_constant__ AssignGeom g,
+              uint32_t *__restrict__ table, uint4 *__restrict__ payload, unsigned long long *__restrict__ lost,
+              unsigned int *__restrict__ wstat, uint64_t cap, unsigned int *__restrict__ ovf, uint32_t slab)
+{
+    unsigned long long my_lost = 0;
+    unsigned int my_wmax = 0, my_neg = 0, my_wminc = 0;
+    const bool weighted = w != nullptr;
+    const int64_t p0 = (int64_t)blockIdx.x * chunk;
+    for_particles(x, y, z, w, p0, min(chunk, np - p0), [&](int, float px, float py, float pz, float wt) {
+        const unsigned long long before = my_lost;
+        append_one<SCHEME, kCursorStride>(px, py, pz, wt, g, table, payload, cap, ovf, my_lost, SLAB ? slab : 0u);
+        if (SLAB && weighted && my_lost == before) weight_stats(wt, my_wmax, my_neg, my_wminc);
+    });
+    if (SLAB) flush_stats(my_lost, my_wmax, my_neg, my_wminc, lost, wstat);
+}
+
+// Pass 3, staged: each CTA sorts a tile of particles' records by brick in
+// shared memory and appends every brick's run with one cursor atomic and
+// consecutive 16-byte stores.
+//   1. each particle's record for its first brick goes to its stage slot; a
+//      shared counter per brick gives its rank in the tile.  Particles whose
+//      stencil crosses brick faces are queued;
+//   2. the queue's further records (next bricks) are staged the same way,
+//      by full warps; past the stage's capacity a record is appended on its
+//      own, as append_kernel does;
+//   3. per brick: the cursor is advanced by the tile's count (one atomic),
+//      and an exclusive scan of the counts orders the stage by brick (perm);
+//   4. records leave in that order: neighbouring threads write neighbouring
+//      slots of a brick's run.
+// Shared memory: stage [recs] 16 bytes, key and rank [recs] (18 + 14 bits),
+// bricks [nb], perm [recs] 16 bits (the queue lives there before step 3).
+// tile <= 8192, recs <= 16384, nb <= kStageBricks.
+constexpr int kStageThreads = 1024;
+constexpr int kStageBricks = 4096;
+constexpr int kStagePer = kStageBricks / kStageThreads;
+constexpr int kStageTile = 8192;
+constexpr size_t kStageSmem = 226 * 1024;
+__host__ __device__ constexpr size_t stage_bytes(int recs, int nb)
+{
+    return (size_t)recs * 22 + (size_t)nb * 4 + 16;
+}
+
+template <int SCHEME, bool SLAB>
+__global__ void __launch_bounds__(kStageThreads, 1)
+staged_kernel(const float *__restrict__ x, const float *__restrict__ y, const float *__restrict__ z,
+              const float *__restrict__ w, int64_t np, int tile, int recs, const __grid_constant__ AssignGeom g, int nb,
+              uint32_t *__restrict__ table, uint4 *__restrict__ payload, unsigned long long *__restrict__ lost,
+              unsigned int *__restrict__ wstat, uint64_t cap, unsigned int *__restrict__ ovf, uint32_t slab)
+{
+    extern __shared__ __align__(16) unsigned char stage_smem[];
+    __shared__ uint32_t warp_sums[kStageThreads / 32];
+    __shared__ uint32_t s_queued, s_extra, s_total;
+    uint4 *const stage = reinterpret_cast<uint4 *>(stage_smem);
+    uint32_t *const kr = reinterpret_cast<uint32_t *>(stage + recs);  // key << 14 | rank; ~0: no record
+    uint32_t *const bin = kr + recs;                                  // [nb]
+    uint16_t *const perm = reinterpret_cast<uint16_t *>(bin + nb);    // [recs]
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    const bool weighted = w != nullptr;
+    unsigned long long my_lost = 0;
+    unsigned int my_wmax = 0, my_neg = 0, my_wminc = 0;
+    const uint32_t slab_v = SLAB ? slab : 0u;
+    const int per = (nb + kStageThreads - 1) / kStageThreads;  // bricks per thread in step 3
+    for (int b = tid; b < nb; b += kStageThreads) bin[b] = 0u;
+    if (tid == 0) s_queued = s_extra = 0u;
+    __syncthreads();
+    for (int64_t p0 = (int64_t)blockIdx.x * tile; p0 < np; p0 += (int64_t)gridDim.x * tile) {
+        const int count = (int)min((int64_t)tile, np - p0);
+        // 1. first bricks
+        for_particles(x, y, z, w, p0, count, [&](int i, float px, float py, float pz, float wt) {
+            const float pos[3] = {px, py, pz};
+            int c[3], bl[3], cl[3];
+            float t[3] = {0.f, 0.f, 0.f};
+            if (!locate<SCHEME, true>(pos, g, c, t)) {
+                if (SLAB) ++my_lost;
+                kr[i] = ~0u;
+                return;
+            }
+            if (SLAB && weighted) weight_stats(wt, my_wmax, my_neg, my_wminc);
+            unsigned cross = 0;
+#pragma unroll
+            for (int a = 0; a < 3; ++a) cross |= brick_axis<SCHEME>(g, a, c[a], bl[a], cl[a]) ? 1u << a : 0u;
+            const int key = (bl[0] * g.nb[1] + bl[1]) * g.nb[2] + bl[2];
+            const uint32_t rank = atomicAdd(bin + key, 1u);
+            stage[i] = make_uint4(pack_axis(cl[0], t[0]), pack_axis(cl[1], t[1]), pack_axis(cl[2], t[2]),
+                                  __float_as_uint(wt));
+            kr[i] = ((uint32_t)key << 14) | rank;
+            if (SCHEME != CAM_NGP && cross) perm[atomicAdd(&s_queued, 1u)] = (uint16_t)(i | (cross << 13));
+        });
+        __syncthreads();
+        // 2. the next bricks of the queued particles
+        if (SCHEME != CAM_NGP) {
+            const int nq = (int)s_queued;
+            for (int q = tid; q < nq; q += kStageThreads) {
+                const unsigned ent = perm[q];
+                const int i = (int)(ent & 8191u);
+                const unsigned cross = ent >> 13;
+                const uint4 rec = stage[i];
+                const int key = (int)(kr[i] >> 14);
+                int bl[3], step[3];
+                const int r = g.nb[2] == 1 ? key : (int)__umulhi((unsigned)key, g.kmagic[0]);
+                bl[2] = key - r * g.nb[2];
+                bl[0] = g.nb[1] == 1 ? r : (int)__umulhi((unsigned)r, g.kmagic[1]);
+                bl[1] = r - bl[0] * g.nb[1];
+                key_steps(g, bl, step);
+                for (unsigned m = cross; m; m = (m - 1u) & cross) {
+                    const int k = key + (m & 1u ? step[0] : 0) + (m & 2u ? step[1] : 0) + (m & 4u ? step[2] : 0);
+                    const uint4 nrec = next_brick_record(g, rec, bl, m);
+                    const int at = tile + (int)atomicAdd(&s_extra, 1u);
+                    if (at < recs) {
+                        const uint32_t rank = atomicAdd(bin + k, 1u);
+                        stage[at] = nrec;
+                        kr[at] = ((uint32_t)k << 14) | rank;
+                    } else {
+                        put_record(payload, nrec, k, atomicAdd(table + (int64_t)k * kCursorStride, 1u), slab_v, cap, ovf);
+                    }
+                }
+            }
+            __syncthreads();
+        }
+        // 3. cursors and the order by brick
+        const int extra = min((int)s_extra, recs - tile);
+        uint32_t base[kStagePer];
+        {
+            uint32_t cnt[kStagePer], sum = 0;
+#pragma unroll
+            for (int j = 0; j < kStagePer; ++j) {
+                const int b = tid * per + j;
+                cnt[j] = j < per && b < nb ? bin[b] : 0u;
+                base[j] = cnt[j] ? atomicAdd(table + (int64_t)b * kCursorStride, cnt[j]) : 0u;
+                sum += cnt[j];
+            }
+            uint32_t incl = sum;
+#pragma unroll
+            for (int off = 1; off < 32; off <<= 1) {
+                const uint32_t v = __shfl_up_sync(0xffffffffu, incl, off);
+                if (lane >= off) incl += v;
+            }
+            if (lane == 31) warp_sums[wid] = incl;
+            __syncthreads();
+            if (wid == 0) {
+                const uint32_t ws = warp_sums[lane];
+                uint32_t wi = ws;
+#pragma unroll
+                for (int off = 1; off < 32; off <<= 1) {
+                    const uint32_t v = __shfl_up_sync(0xffffffffu, wi, off);
+                    if (lane >= off) wi += v;
+                }
+                warp_sums[lane] = wi - ws;
+                if (lane == 31) s_total = wi;
+            }
+            __syncthreads();
+            uint32_t run = warp_sums[wid] + incl - sum;
+#pragma unroll
+            for (int j = 0; j < kStagePer; ++j) {
+                const int b = tid * per + j;
+                if (j < per && b < nb) bin[b] = run;
+                run += cnt[j];
+            }
+        }
+        __syncthreads();
+        for (int i = tid; i < count; i += kStageThreads) {
+            const uint32_t k = kr[i];
+            if (k != ~0u) perm[bin[k >> 14] + (k & 16383u)] = (uint16_t)i;
+        }
+        for (int i = tile + tid; i < tile + extra; i += kStageThreads) {
+            const uint32_t k = kr[i];
+            perm[bin[k >> 14] + (k & 16383u)] = (uint16_t)i;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int j = 0; j < kStagePer; ++j) {
+            const int b = tid * per + j;
+            if (j < per && b < nb) bin[b] = base[j];
+        }
+        __syncthreads();
+        // 4. out, in brick order
+        const int total = (int)s_total;
+#pragma unroll 2
+        for (int i = tid; i < total; i += kStageThreads) {
+            const int at = perm[i];
+            const uint32_t k = kr[at];
+            put_record(payload, stage[at], (int)(k >> 14), bin[k >> 14] + (k & 16383u), slab_v, cap, ovf);
+        }
+        __syncthreads();
+        for (int b = tid; b < nb; b += kStageThreads) bin[b] = 0u;
+        if (tid == 0) s_queued = s_extra = 0u;
+        __syncthreads();
+    }
+    if (SLAB) flush_stats(my_lost, my_wmax, my_neg, my_wminc, lost, wstat);
 }
 
 // Brick starts in one CTA (nb <= kOffThreads * kOffItems): thread t scans
@@ -348,7 +534,15 @@ AssignGeom make_geom(const cam_grid &gr, int scheme, int64_t np)
         g.nb[a] = (g.n[a] + g.b[a] - 1) / g.b[a];
         g.bmagic[a] = (unsigned)(((1ull << 32) + (uint64_t)g.b[a] - 1) / (uint64_t)g.b[a]);
         g.inv_d[a] = 1.0f / g.d[a];
+        g.e_last[a] = g.n[a] - (g.nb[a] - 1) * g.b[a];
+        g.nf[a] = (float)g.n[a];
+        // home_cell divides exactly when a quotient u <= n lies within
+        // 4e-7 max(u, 1) of an integer; a little more is set aside here
+        g.safe[a] = 0.5f - (4.2e-7f * (float)(g.n[a] + 1) + 1e-6f);
+        g.origin |= g.mn[a] != 0.0f;
     }
+    for (int a = 0; a < 2; ++a)
+        g.kmagic[a] = g.nb[2 - a] > 1 ? (unsigned)(((1ull << 32) + (uint64_t)g.nb[2 - a] - 1) / (uint64_t)g.nb[2 - a]) : 0u;
     (void)scheme;
     return g;
 }
@@ -360,14 +554,9 @@ static void assign_impl(cam_ctx *ctx, const float *x, const float *y, const floa
     const int64_t nb = (int64_t)g.nb[0] * g.nb[1] * g.nb[2];
     CAM_REQUIRE(nb < (1ll << 31), CAM_E_UNSUPPORTED, "too many mesh bricks");
     // Count pass: one CTA of 1024 threads per SM (its brick histogram in
-    // shared memory); scatter pass: two CTAs of 512 threads per SM.  Both
-    // take contiguous chunks of >= 4096 particles.
+    // shared memory), contiguous chunks of >= 4096 particles.
     const int G = (int)std::max<int64_t>(1, std::min<int64_t>(kNumSMs, (np + 4095) / 4096));
-    const int64_t chunk = std::max<int64_t>(4, ((np + G - 1) / G + 3) & ~(int64_t)3);
-    const int G2 = (int)std::max<int64_t>(1, std::min<int64_t>(2 * kNumSMs, (np + 4095) / 4096));
-    const int64_t chunk2 = std::max<int64_t>(4, ((np + G2 - 1) / G2 + 3) & ~(int64_t)3);
-    auto aligned = [](const void *p) { return p == nullptr || ((uintptr_t)p & 15u) == 0; };
-    const bool vec = aligned(x) && aligned(y) && aligned(z) && aligned(w);
+    const int64_t chunk = std::max<int64_t>(1, (np + G - 1) / G);
     const bool smem_hist = nb <= kSmemBricks;
     // per-brick counters, one per 128-byte line (counts, then cursors)
     auto *table = static_cast<uint32_t *>(scratch(ctx, "asg.cursor", (size_t)nb * kCursorStride * sizeof(uint32_t)));
@@ -414,14 +603,11 @@ static void assign_impl(cam_ctx *ctx, const float *x, const float *y, const floa
     }
 
     const size_t hsmem = smem_hist ? (size_t)nb * sizeof(uint32_t) : 0;
-    auto count_k = smem_hist ? (vec ? bin_kernel<SCHEME, false, true, true> : bin_kernel<SCHEME, false, true, false>)
-                             : (vec ? bin_kernel<SCHEME, false, false, true> : bin_kernel<SCHEME, false, false, false>);
-    auto scatter_k = slab ? (vec ? bin_kernel<SCHEME, true, false, true, true> : bin_kernel<SCHEME, true, false, false, true>)
-                          : (vec ? bin_kernel<SCHEME, true, false, true> : bin_kernel<SCHEME, true, false, false>);
+    auto count_k = smem_hist ? count_kernel<SCHEME, true> : count_kernel<SCHEME, false>;
     if (!slab) {
         smem_at_least(count_k, hsmem);
         CAM_LAUNCH_NAMED(ctx, "assign_bin_count", count_k, G, kBinThreads, hsmem, x, y, z, w, np, chunk, g, (int)nb,
-                         table, (uint4 *)nullptr, d_lost, d_wmax, (uint64_t)0, d_ovf, 0u);
+                         table, d_lost, d_wmax);
         if (nb <= (int64_t)kOffThreads * kOffItems) {
             CAM_LAUNCH_NAMED(ctx, "assign_starts", brick_offsets_kernel, 1, kOffThreads, 0, table, (int)nb, start,
                              d_total);
@@ -485,8 +671,29 @@ static void assign_impl(cam_ctx *ctx, const float *x, const float *y, const floa
     }
 
     uint4 *payload = static_cast<uint4 *>(scratch(ctx, "asg.payload", std::max<size_t>(total, 1) * sizeof(uint4)));
-    CAM_LAUNCH_NAMED(ctx, "assign_bin_scatter", scatter_k, G2, kScatterThreads, 0, x, y, z, w, np, chunk2, g, (int)nb,
-                     table, payload, d_lost, d_wmax, total, d_ovf, slab);
+    if (nb <= kStageBricks) {
+        // Tiles as large as the stage holds with the expected records (15%
+        // margin on the extra ones), split evenly over the SMs.
+        const int recs = (int)std::min<size_t>(16384, (kStageSmem - 16 - (size_t)nb * 4) / 22);
+        const double room = (double)recs / (1.0 + 1.15 * (f - 1.0));
+        const int64_t most = std::max<int64_t>(1024, std::min<int64_t>(kStageTile, (int64_t)room));
+        const int64_t rounds = std::max<int64_t>(1, (np + kNumSMs * most - 1) / (kNumSMs * most));
+        const int64_t even = (np + kNumSMs * rounds - 1) / (kNumSMs * rounds);
+        const int tile = (int)std::min<int64_t>(most, std::max<int64_t>(1024, (even + 31) & ~(int64_t)31));
+        const int64_t tiles = (np + tile - 1) / tile;
+        const unsigned grid_s = (unsigned)std::max<int64_t>(1, std::min<int64_t>(kNumSMs, tiles));
+        const size_t ssmem = stage_bytes(recs, (int)nb);
+        auto k = slab ? staged_kernel<SCHEME, true> : staged_kernel<SCHEME, false>;
+        smem_at_least(k, ssmem);
+        CAM_LAUNCH_NAMED(ctx, "assign_bin_scatter", k, grid_s, kStageThreads, ssmem, x, y, z, w, np, tile, recs, g,
+                         (int)nb, table, payload, d_lost, d_wmax, total, d_ovf, slab);
+    } else {
+        const int G2 = (int)std::max<int64_t>(1, std::min<int64_t>(2 * kNumSMs, (np + 4095) / 4096));
+        const int64_t chunk2 = std::max<int64_t>(1, (np + G2 - 1) / G2);
+        auto k = slab ? append_kernel<SCHEME, true> : append_kernel<SCHEME, false>;
+        CAM_LAUNCH_NAMED(ctx, "assign_bin_scatter", k, G2, kScatterThreads, 0, x, y, z, w, np, chunk2, g, table, payload,
+                         d_lost, d_wmax, total, d_ovf, slab);
+    }
 
     const size_t smem = (size_t)tile_words(g.b[0]) * sizeof(uint32_t);
     const int weighted = w != nullptr;

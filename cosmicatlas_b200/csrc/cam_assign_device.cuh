@@ -67,21 +67,27 @@ __device__ __forceinline__ int brick_of(int cell, int b, unsigned magic)
     return b == 1 ? cell : (int)__umulhi((unsigned)cell, magic);
 }
 
-// Exact offset t = (x - min)/d - 1/2 - c in cells, nearest periodic image,
-// in FP32 with error-free transformations: TwoSum for x - min and a fused
-// multiply-add for the subtraction of (c + 1/2) d (the product is exact
+// Cell centre (in cells) nearest to the position u = (x - min) / d: c + 1/2 of
+// the home cell c or its periodic image.
+__device__ __forceinline__ float nearest_centre(float u, float ci, float nf)
+{
+    const float diff = u - ci;
+    if (diff > 0.5f * nf) ci += nf;
+    else if (diff < -0.5f * nf) ci -= nf;
+    return ci;
+}
+
+// Exact offset t = (x - min)/d - ci in cells, in FP32 with error-free
+// transformations: TwoSum for x - min (nothing to do for min = 0) and a
+// fused multiply-add for the subtraction of ci d (the product is exact
 // inside the FMA); the residual (|r| <= 1.5 d) is scaled by 1/d.
 // |error| <= ~2e-7 cells.
-__device__ __forceinline__ float exact_offset(float x, float mn, float d, float inv_d, int c, int n)
+__device__ __forceinline__ float exact_offset(float x, float mn, float d, float inv_d, float ci, bool origin)
 {
+    if (!origin) return __fmaf_rn(-ci, d, x) * inv_d;
     const float hi = __fsub_rn(x, mn);
     const float bb = __fsub_rn(hi, x);
     const float lo = __fadd_rn(__fsub_rn(x, __fsub_rn(hi, bb)), __fsub_rn(-mn, bb));
-    const float u = hi * inv_d;
-    float ci = (float)c + 0.5f;
-    const float diff = u - ci;
-    if (diff > 0.5f * (float)n) ci += (float)n;
-    else if (diff < -0.5f * (float)n) ci -= (float)n;
     const float r = __fadd_rn(__fmaf_rn(-ci, d, hi), lo);
     return r * inv_d;
 }
@@ -92,17 +98,80 @@ struct Stencil {
     static constexpr int FIRST = SCHEME == CAM_TSC ? -1 : 0;
 };
 
-// First and last stencil cells of a home cell c in [0, n), wrapped
-// periodically: the stencil reaches at most one cell below 0 (TSC) and at
-// most one cell at or above n, so one conditional add or subtract each.
-template <int SCHEME>
-__device__ __forceinline__ void stencil_ends(int c, int n, int &lo, int &hi)
+// Home cell c[] of a particle as home_cell gives it (false: lost) and, with
+// OFFSETS, its exact offsets t[] from the cell centre.  The common case --
+// every quotient well inside [0, n) and away from an integer -- takes the
+// floor by one addition of 2^23 rounded down (the float then holds the
+// integer in its low bits); any other particle goes through home_cell.
+template <int SCHEME, bool OFFSETS>
+__device__ __forceinline__ bool locate(const float p[3], const AssignGeom &g, int c[3], float t[3])
 {
-    using St = Stencil<SCHEME>;
-    lo = c + St::FIRST;
-    hi = c + St::FIRST + St::W - 1;
-    if constexpr (St::FIRST < 0) lo = lo < 0 ? lo + n : lo;
-    if constexpr (St::FIRST + St::W - 1 > 0) hi = hi >= n ? hi - n : hi;
+    float ci[3];
+    bool ok = true, rare = false;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        float v = p[a];
+        if (SCHEME == CAM_CIC) {
+            v = __fsub_rn(v, __fmul_rn(0.5f, g.d[a]));
+            if (v < 0.0f) v = __fadd_rn(v, g.L[a]);
+            if (v >= g.L[a]) v = __fsub_rn(v, g.L[a]);
+        }
+        const float hi = __fadd_rn(g.mn[a], g.L[a]);
+        ok = ok && (SCHEME == CAM_TSC ? (v >= g.mn[a] && v <= hi) : (v >= g.mn[a] && v < hi));
+        const float u = __fmul_rn(__fsub_rn(v, g.mn[a]), g.inv_d[a]);
+        const float f = __fadd_rd(u, 8388608.0f);
+        const float fl = f - 8388608.0f;
+        c[a] = __float_as_int(f) - 0x4b000000;
+        ci[a] = fl + 0.5f;
+        rare = rare || !(fabsf(u - ci[a]) < g.safe[a]) || !(u < g.nf[a]);
+    }
+    if (!ok) return false;
+    if (rare) {
+        home_cell<SCHEME>(p, g, c);
+#pragma unroll
+        for (int a = 0; a < 3; ++a) ci[a] = (float)c[a] + 0.5f;
+    }
+    if (OFFSETS && SCHEME != CAM_NGP) {
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            // TSC: only a quotient that rounded up to n has its home cell
+            // wrapped; CIC: the half-cell shift can wrap any particle
+            if (SCHEME == CAM_CIC || rare)
+                ci[a] = nearest_centre(__fsub_rn(p[a], g.mn[a]) * g.inv_d[a], ci[a], g.nf[a]);
+            t[a] = exact_offset(p[a], g.mn[a], g.d[a], g.inv_d[a], ci[a], g.origin != 0);
+        }
+    }
+    return true;
+}
+
+// The brick of a particle's first stencil cell along axis a: its coordinate
+// bl, the home cell relative to it (cl in [0, e], e its extent), and whether
+// the stencil reaches into the next brick (periodic; never along an axis
+// that one brick spans).
+template <int SCHEME>
+__device__ __forceinline__ bool brick_axis(const AssignGeom &g, int a, int c, int &bl, int &cl)
+{
+    if (g.nb[a] == 1) {
+        bl = 0;
+        cl = c;
+        return false;
+    }
+    int lo = c;
+    if (SCHEME == CAM_TSC) lo = c == 0 ? g.n[a] - 1 : c - 1;
+    bl = brick_of(lo, g.b[a], g.bmagic[a]);
+    cl = lo - bl * g.b[a] + (SCHEME == CAM_TSC ? 1 : 0);
+    if (SCHEME == CAM_NGP) return false;
+    const int e = bl == g.nb[a] - 1 ? g.e_last[a] : g.b[a];
+    return cl + 1 >= e;
+}
+
+// Step of the brick number to the next brick along each axis (periodic).
+__device__ __forceinline__ void key_steps(const AssignGeom &g, const int bl[3], int step[3])
+{
+    const int s1 = g.nb[2], s0 = g.nb[1] * g.nb[2];
+    step[0] = (bl[0] + 1 == g.nb[0] ? -bl[0] : 1) * s0;
+    step[1] = (bl[1] + 1 == g.nb[1] ? -bl[1] : 1) * s1;
+    step[2] = bl[2] + 1 == g.nb[2] ? -bl[2] : 1;
 }
 
 // Payload word per axis: bits 26..31 = home cell relative to the brick + 8,
@@ -119,143 +188,97 @@ __device__ __forceinline__ void unpack_axis(uint32_t v, int &cl, float &t)
     t = (float)((int)(v & 0x3FFFFFFu) - 16777216) * (1.0f / 16777216.0f);
 }
 
-__device__ __forceinline__ int brick_linear(const AssignGeom &g, int b0, int b1, int b2)
+// A record as the next brick along the axes of mask m sees it: the home
+// cell relative to a brick falls by the extent of the brick before it.
+__device__ __forceinline__ uint4 next_brick_record(const AssignGeom &g, uint4 r, const int bl[3], unsigned m)
 {
-    return (b0 * g.nb[1] + b1) * g.nb[2] + b2;
+    auto ext = [&](int a) { return (uint32_t)(bl[a] == g.nb[a] - 1 ? g.e_last[a] : g.b[a]) << 26; };
+    if (m & 1u) r.x -= ext(0);
+    if (m & 2u) r.y -= ext(1);
+    if (m & 4u) r.z -= ext(2);
+    return r;
 }
 
-// One particle of pass 1: the bricks its stencil touches (the brick of its
-// first stencil cell and, along each axis whose stencil crosses a brick
-// face, the next brick, periodically) each get one count.
+// The weight statistics of one particle (wstat of fixed_scale).
+__device__ __forceinline__ void weight_stats(float wt, unsigned int &wmax, unsigned int &neg, unsigned int &wminc)
+{
+    wmax = max(wmax, __float_as_uint(fabsf(wt)));
+    neg |= wt < 0.0f;
+    if (wt != 0.0f) wminc = max(wminc, 0x7fffffffu - __float_as_uint(fabsf(wt)));
+}
+
+// One particle of the count pass: the bricks its stencil touches (the brick
+// of its first stencil cell and, along each axis whose stencil crosses a
+// brick face, the next brick, periodically) each get one count.
 template <int SCHEME, bool SMEM>
 __device__ __forceinline__ void count_one(float px, float py, float pz, float wt, bool weighted, const AssignGeom &g,
                                           uint32_t *hist, uint32_t *__restrict__ table, unsigned long long &my_lost,
                                           unsigned int &my_wmax, unsigned int &my_neg, unsigned int &my_wminc)
 {
-    using St = Stencil<SCHEME>;
     const float pos[3] = {px, py, pz};
-    int c[3] = {0, 0, 0};
-    if (!home_cell<SCHEME>(pos, g, c)) {
+    int c[3], bl[3], cl, step[3];
+    float t[3];
+    if (!locate<SCHEME, false>(pos, g, c, t)) {
         ++my_lost;
         return;
     }
-    if (weighted) {
-        my_wmax = max(my_wmax, __float_as_uint(fabsf(wt)));
-        my_neg |= wt < 0.0f;
-        if (wt != 0.0f) my_wminc = max(my_wminc, 0x7fffffffu - __float_as_uint(fabsf(wt)));
-    }
-    int bl[3];
-    bool two[3];
+    if (weighted) weight_stats(wt, my_wmax, my_neg, my_wminc);
+    unsigned cross = 0;
 #pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        int lo, hi;
-        stencil_ends<SCHEME>(c[a], g.n[a], lo, hi);
-        bl[a] = brick_of(lo, g.b[a], g.bmagic[a]);
-        two[a] = St::W > 1 && brick_of(hi, g.b[a], g.bmagic[a]) != bl[a];
-    }
-    const int s1 = g.nb[2], s0 = g.nb[1] * g.nb[2];
-    const int k0 = bl[0] * s0 + bl[1] * s1 + bl[2];
-    // key step to the next brick along each axis (periodic)
-    const int d2 = bl[2] + 1 == g.nb[2] ? -bl[2] : 1;
-    const int d1 = (bl[1] + 1 == g.nb[1] ? -bl[1] : 1) * s1;
-    const int d0 = (bl[0] + 1 == g.nb[0] ? -bl[0] : 1) * s0;
-    auto add = [&](int key) {
-        if (SMEM) atomicAdd(hist + key, 1u);
-        else atomicAdd(table + (int64_t)key * kCursorStride, 1u);
+    for (int a = 0; a < 3; ++a) cross |= brick_axis<SCHEME>(g, a, c[a], bl[a], cl) ? 1u << a : 0u;
+    const int key = (bl[0] * g.nb[1] + bl[1]) * g.nb[2] + bl[2];
+    auto add = [&](int k) {
+        if (SMEM) atomicAdd(hist + k, 1u);
+        else atomicAdd(table + (int64_t)k * kCursorStride, 1u);
     };
-    add(k0);
-    if (two[2]) add(k0 + d2);
-    if (two[1]) {
-        add(k0 + d1);
-        if (two[2]) add(k0 + d1 + d2);
-    }
-    if (two[0]) {
-        add(k0 + d0);
-        if (two[2]) add(k0 + d0 + d2);
-        if (two[1]) {
-            add(k0 + d0 + d1);
-            if (two[2]) add(k0 + d0 + d1 + d2);
-        }
-    }
+    add(key);
+    if (SCHEME == CAM_NGP || cross == 0u) return;
+    key_steps(g, bl, step);
+    for (unsigned m = cross; m; m = (m - 1u) & cross)
+        add(key + (m & 1u ? step[0] : 0) + (m & 2u ? step[1] : 0) + (m & 4u ? step[2] : 0));
 }
 
-// One particle of pass 3 (see bin_kernel).  slab > 0: the brick's records
-// go to its own slab of `slab` records (payload[key * slab + slot], the
-// counter starting at 0), and the weight statistics are gathered here
-// (there is no count pass); my_wminc then receives the smallest nonzero
-// |w| as count_one keeps it.
-template <int SCHEME, bool SCATTER, bool SMEM, int CSTRIDE = kCursorStride>
-__device__ __forceinline__ void bin_one(float px, float py, float pz, float wt, bool weighted,
-                                        const AssignGeom &g, int G, int blk, uint32_t *hist,
-                                        uint32_t *__restrict__ table, uint4 *__restrict__ payload, uint64_t cap,
-                                        unsigned int *ovf, unsigned long long &my_lost, unsigned int &my_wmax,
-                                        unsigned int &my_neg, unsigned int *my_wminc = nullptr, uint32_t slab = 0)
+// Writes one record at `slot` of brick `key`: slab > 0, its own slab of
+// `slab` records (payload[key * slab + slot]); otherwise payload[slot].
+// Records past a full slab or past the payload's capacity (a deferred
+// estimate that fell short) are flagged, not written.
+__device__ __forceinline__ void put_record(uint4 *__restrict__ payload, uint4 rec, int key, uint32_t slot,
+                                           uint32_t slab, uint64_t cap, unsigned int *ovf)
 {
-    using St = Stencil<SCHEME>;
+    const bool fits = slab ? slot < slab : slot < cap;
+    const uint64_t at = slab ? (uint64_t)key * slab + slot : (uint64_t)slot;
+    if (fits) payload[at] = rec;
+    else atomicOr(ovf, 1u);
+}
+
+// One particle appended record by record: every touched brick's cursor
+// (cursor[key * CSTRIDE]) gives the next slot.
+template <int SCHEME, int CSTRIDE>
+__device__ __forceinline__ void append_one(float px, float py, float pz, float wt, const AssignGeom &g,
+                                           uint32_t *__restrict__ cursor, uint4 *__restrict__ payload, uint64_t cap,
+                                           unsigned int *ovf, unsigned long long &my_lost, uint32_t slab)
+{
     const float pos[3] = {px, py, pz};
-    int c[3] = {0, 0, 0};
-    if (!home_cell<SCHEME>(pos, g, c)) {
+    int c[3], bl[3], cl[3], step[3];
+    float t[3] = {0.f, 0.f, 0.f};
+    if (!locate<SCHEME, true>(pos, g, c, t)) {
         ++my_lost;
         return;
     }
-    if (weighted && (!SCATTER || my_wminc)) {
-        my_wmax = max(my_wmax, __float_as_uint(fabsf(wt)));
-        my_neg |= wt < 0.0f;
-        if (SCATTER && wt != 0.0f) *my_wminc = max(*my_wminc, 0x7fffffffu - __float_as_uint(fabsf(wt)));
-    }
-    // Bricks touched along each axis: 1 or 2.
-    int bl[3], nbx[3];
-    float t[3] = {0.f, 0.f, 0.f};
+    unsigned cross = 0;
 #pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        int lo, hi;
-        stencil_ends<SCHEME>(c[a], g.n[a], lo, hi);
-        bl[a] = brick_of(lo, g.b[a], g.bmagic[a]);
-        nbx[a] = (brick_of(hi, g.b[a], g.bmagic[a]) == bl[a]) ? 1 : 2;
-        if (SCHEME != CAM_NGP && SCATTER) t[a] = exact_offset(pos[a], g.mn[a], g.d[a], g.inv_d[a], c[a], g.n[a]);
-    }
-#pragma unroll
-    for (int i0 = 0; i0 < 2; ++i0) {
-        if (i0 >= nbx[0]) break;
-        const int b0 = (bl[0] + i0 == g.nb[0]) ? 0 : bl[0] + i0;
-#pragma unroll
-        for (int i1 = 0; i1 < 2; ++i1) {
-            if (i1 >= nbx[1]) break;
-            const int b1 = (bl[1] + i1 == g.nb[1]) ? 0 : bl[1] + i1;
-#pragma unroll
-            for (int i2 = 0; i2 < 2; ++i2) {
-                if (i2 >= nbx[2]) break;
-                const int b2 = (bl[2] + i2 == g.nb[2]) ? 0 : bl[2] + i2;
-                const int key = brick_linear(g, b0, b1, b2);
-                // SMEM: the CTA's shared counters (count: its histogram;
-                // scatter: its own cursors into each brick's range);
-                // otherwise the global counts / the brick's append cursor
-                const uint32_t slot = SMEM ? atomicAdd(hist + key, 1u)
-                                           : atomicAdd(table + (int64_t)key * CSTRIDE, 1u);
-                if (SCATTER) {
-                    const int o[3] = {b0 * g.b[0], b1 * g.b[1], b2 * g.b[2]};
-                    uint32_t word[3];
-#pragma unroll
-                    for (int a = 0; a < 3; ++a) {
-                        // Home cell relative to the brick origin: the periodic
-                        // image in [-1, e], e = brick extent, which holds
-                        // whenever the stencil touches the brick.
-                        const int e = min(g.b[a], g.n[a] - o[a]);
-                        int cl = c[a] - o[a];
-                        if (cl < -1) cl += g.n[a];
-                        else if (cl > e) cl -= g.n[a];
-                        word[a] = pack_axis(cl, t[a]);
-                    }
-                    // records past the payload's capacity (a deferred
-                    // estimate that fell short) or past a full slab are
-                    // flagged, not written
-                    const bool fits = slab ? slot < slab : slot < cap;
-                    const uint64_t at = slab ? (uint64_t)key * slab + slot : (uint64_t)slot;
-                    if (fits) payload[at] = make_uint4(word[0], word[1], word[2], __float_as_uint(wt));
-                    else atomicOr(ovf, 1u);
-                }
-            }
-        }
+    for (int a = 0; a < 3; ++a) cross |= brick_axis<SCHEME>(g, a, c[a], bl[a], cl[a]) ? 1u << a : 0u;
+    const int key = (bl[0] * g.nb[1] + bl[1]) * g.nb[2] + bl[2];
+    const uint32_t slot = atomicAdd(cursor + (int64_t)key * CSTRIDE, 1u);
+    const uint4 rec = make_uint4(pack_axis(cl[0], t[0]), pack_axis(cl[1], t[1]), pack_axis(cl[2], t[2]),
+                                 __float_as_uint(wt));
+    put_record(payload, rec, key, slot, slab, cap, ovf);
+    if (SCHEME == CAM_NGP || cross == 0u) return;
+    key_steps(g, bl, step);
+    for (unsigned m = cross; m; m = (m - 1u) & cross) {
+        const int k = key + (m & 1u ? step[0] : 0) + (m & 2u ? step[1] : 0) + (m & 4u ? step[2] : 0);
+        const uint32_t sl = atomicAdd(cursor + (int64_t)k * CSTRIDE, 1u);
+        put_record(payload, next_brick_record(g, rec, bl, m), k, sl, slab, cap, ovf);
     }
 }
 

@@ -204,11 +204,10 @@ __device__ void dl_assign(const DlJob &J, const DlScratch &S, uint4 *payload, fl
     // append cursors (the counts are not needed any more)
     for (int b = tid; b < nb; b += kDlThreads) sh.hist[b] = sh.start[b];
     __syncthreads();
-    unsigned dummy_wmax = 0, dummy_neg = 0;
     unsigned long long dummy_lost = 0;
     for (int64_t p = tid; p < J.np; p += kDlThreads)
-        bin_one<SCHEME, true, false, 1>(J.x[p], J.y[p], J.z[p], weighted ? J.w[p] : 1.0f, weighted, g, 1, 0, nullptr,
-                                        sh.hist, payload, S.pcap, sh.ovf, dummy_lost, dummy_wmax, dummy_neg);
+        append_one<SCHEME, 1>(J.x[p], J.y[p], J.z[p], weighted ? J.w[p] : 1.0f, g, sh.hist, payload, S.pcap, sh.ovf,
+                              dummy_lost, 0u);
     __syncthreads();
     // deposit, brick by brick (the tile of deposit_kernel)
     uint32_t *tile = reinterpret_cast<uint32_t *>(sh.big);

@@ -184,6 +184,12 @@ struct AssignGeom {
     int b[3];            // brick extent (cells)
     int nb[3];           // bricks per axis
     unsigned bmagic[3];  // ceil(2^32 / b): cell / b = umulhi(cell, bmagic)
+    int e_last[3];       // extent of the last brick
+    unsigned kmagic[2];  // ceil(2^32 / nb[2]), ceil(2^32 / nb[1]) (0 for 1): brick number -> coordinates
+    float nf[3];         // (float)n
+    float safe[3];       // a quotient (x - min) * inv_d in [0, n) whose fraction lies within `safe` of 1/2
+                         // has the floor of the IEEE quotient
+    int origin;          // some min is not zero
 };
 
 struct AssignOut {
