@@ -43,57 +43,45 @@ using namespace asg;
 
 
 // Calls one(i, x, y, z, w) for the particles p0 + i, i in [0, count), the
-// threads of the CTA taking consecutive particles, the next one's loads in
-// flight meanwhile.  Scalar loads: 128 bytes per warp and array either way,
-// and no selects to pick a particle out of a float4.  Unit weights when w is
-// null.
-template <typename F>
+// NT threads of the CTA taking consecutive particles, two per iteration with
+// all their loads ahead of the work.  Scalar loads: 128 bytes per warp and
+// array either way, and no selects to pick a particle out of a float4.  Unit
+// weights when w is null.
+template <int NT, typename F>
 __device__ __forceinline__ void for_particles(const float *__restrict__ x, const float *__restrict__ y,
                                               const float *__restrict__ z, const float *__restrict__ w, int64_t p0,
-                                              int64_t count, F &&one)
+                                              int count, F &&one)
 {
-    const bool weighted = w != nullptr;
-    int64_t i = threadIdx.x;
-    float ax = 0.f, ay = 0.f, az = 0.f, aw = 1.f;
-    if (i < count) {
-        ax = __ldcs(x + p0 + i);
-        ay = __ldcs(y + p0 + i);
-        az = __ldcs(z + p0 + i);
-        if (weighted) aw = __ldcs(w + p0 + i);
-    }
+    x += p0;
+    y += p0;
+    z += p0;
+    if (w) w += p0;
+    int i = threadIdx.x;
 #pragma unroll 1
-    while (i < count) {
-        const int64_t j = i + blockDim.x;
-        float bx = 0.f, by = 0.f, bz = 0.f, bw = 1.f;
-        if (j < count) {
-            bx = __ldcs(x + p0 + j);
-            by = __ldcs(y + p0 + j);
-            bz = __ldcs(z + p0 + j);
-            if (weighted) bw = __ldcs(w + p0 + j);
+    for (; i + NT < count; i += 2 * NT) {
+        const float ax = __ldcs(x + i), ay = __ldcs(y + i), az = __ldcs(z + i);
+        const float bx = __ldcs(x + i + NT), by = __ldcs(y + i + NT), bz = __ldcs(z + i + NT);
+        float aw = 1.0f, bw = 1.0f;
+        if (w) {
+            aw = __ldcs(w + i);
+            bw = __ldcs(w + i + NT);
         }
-        one((int)i, ax, ay, az, aw);
-        ax = bx;
-        ay = by;
-        az = bz;
-        aw = bw;
-        i = j;
+        one(i, ax, ay, az, aw);
+        one(i + NT, bx, by, bz, bw);
     }
+    if (i < count) one(i, __ldcs(x + i), __ldcs(y + i), __ldcs(z + i), w ? __ldcs(w + i) : 1.0f);
 }
 
 // Adds the CTA's lost count and weight statistics, one atomic per warp.
-__device__ __forceinline__ void flush_stats(unsigned long long lost_n, unsigned int wmax, unsigned int neg,
-                                            unsigned int wminc, unsigned long long *__restrict__ lost,
-                                            unsigned int *__restrict__ wstat)
+__device__ __forceinline__ void flush_stats(unsigned int lost_n, const WeightStats &ws,
+                                            unsigned long long *__restrict__ lost, unsigned int *__restrict__ wstat)
 {
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
-        lost_n += __shfl_down_sync(0xffffffffu, lost_n, off);
-        wmax = max(wmax, __shfl_down_sync(0xffffffffu, wmax, off));
-        neg |= __shfl_down_sync(0xffffffffu, neg, off);
-        wminc = max(wminc, __shfl_down_sync(0xffffffffu, wminc, off));
-    }
+    lost_n = __reduce_add_sync(0xffffffffu, lost_n);
+    const unsigned wmax = __reduce_max_sync(0xffffffffu, ws.wmax);
+    const unsigned neg = __reduce_or_sync(0xffffffffu, ws.neg());
+    const unsigned wminc = __reduce_max_sync(0xffffffffu, ws.wminc());
     if ((threadIdx.x & 31) == 0) {
-        if (lost_n) atomicAdd(lost, lost_n);
+        if (lost_n) atomicAdd(lost, (unsigned long long)lost_n);
         if (wmax) atomicMax(wstat, wmax);
         if (neg) atomicOr(wstat + 1, 1u);  // some weight is negative
         if (wminc) atomicMax(wstat + 6, wminc);  // smallest nonzero |w|
@@ -101,36 +89,37 @@ __device__ __forceinline__ void flush_stats(unsigned long long lost_n, unsigned 
 }
 
 // Pass 1.  Block b counts the records of particles [b chunk, (b+1) chunk)
-// per brick into table[brick * kCursorStride] (through a shared-memory
+// per brick into table[brick * g.cstride] (through a shared-memory
 // histogram when SMEM, nb <= kSmemBricks), plus lost particles and the
 // weight statistics.
 template <int SCHEME, bool SMEM>
 __global__ void __launch_bounds__(kBinThreads)
 count_kernel(const float *__restrict__ x, const float *__restrict__ y, const float *__restrict__ z,
-             const float *__restrict__ w, int64_t np, int64_t chunk, const __grid_constant__ AssignGeom g, int nb,
+             const float *__restrict__ w, int64_t np, unsigned chunk, const __grid_constant__ AssignGeom g, int nb,
              uint32_t *__restrict__ table, unsigned long long *__restrict__ lost, unsigned int *__restrict__ wstat)
 {
     extern __shared__ uint32_t hist[];
     if (SMEM) {
-        for (int i = threadIdx.x; i < nb; i += blockDim.x) hist[i] = 0u;
+        for (int i = threadIdx.x; i < nb; i += kBinThreads) hist[i] = 0u;
         __syncthreads();
     }
-    unsigned long long my_lost = 0;
-    unsigned int my_wmax = 0, my_neg = 0, my_wminc = 0;
+    unsigned int my_lost = 0;
+    WeightStats ws;
     const bool weighted = w != nullptr;
     const int64_t p0 = (int64_t)blockIdx.x * chunk;
-    for_particles(x, y, z, w, p0, min(chunk, np - p0), [&](int, float px, float py, float pz, float wt) {
-        count_one<SCHEME, SMEM>(px, py, pz, wt, weighted, g, hist, table, my_lost, my_wmax, my_neg, my_wminc);
+    const int count = (int)max((int64_t)0, min((int64_t)chunk, np - p0));
+    for_particles<kBinThreads>(x, y, z, w, p0, count, [&](int, float px, float py, float pz, float wt) {
+        count_one<SCHEME, SMEM>(px, py, pz, wt, weighted, g, hist, table, my_lost, ws);
     });
-    flush_stats(my_lost, my_wmax, my_neg, my_wminc, lost, wstat);
+    flush_stats(my_lost, ws, lost, wstat);
     if (SMEM) {
         __syncthreads();
-        for (int i = threadIdx.x; i < nb; i += blockDim.x)
-            if (hist[i]) atomicAdd(table + (int64_t)i * kCursorStride, hist[i]);
+        for (int i = threadIdx.x; i < nb; i += kBinThreads)
+            if (hist[i]) atomicAdd(table + (int64_t)i * g.cstride, hist[i]);
     }
 }
 
-// Pass 3 for meshes with more bricks than a staged tile sorts (kStageBricks):
+// Pass 3 for meshes with more bricks than a staged tile counts (kStageBins):
 // every record takes the next slot of its brick's cursor (table, the
 // exclusive scan of the counts or zero for slabs) with one global atomic.  A
 // brick's records are appended contiguously by all CTAs, so its few open
@@ -141,135 +130,420 @@ count_kernel(const float *__restrict__ x, const float *__restrict__ y, const flo
 template <int SCHEME, bool SLAB>
 __global__ void __launch_bounds__(kScatterThreads, 2)
 append_kernel(const float *__restrict__ x, const float *__restrict__ y, const float *__restrict__ z,
-              const float *__restrict__ w, int64_t np, int64_t chunk, const __grid_constant__ AssignGeom g,
+              const float *__restrict__ w, int64_t np, unsigned chunk, const __grid_constant__ AssignGeom g,
               uint32_t *__restrict__ table, uint4 *__restrict__ payload, unsigned long long *__restrict__ lost,
               unsigned int *__restrict__ wstat, uint64_t cap, unsigned int *__restrict__ ovf, uint32_t slab)
 {
-    unsigned long long my_lost = 0;
-    unsigned int my_wmax = 0, my_neg = 0, my_wminc = 0;
+    unsigned int my_lost = 0;
+    WeightStats ws;
     const bool weighted = w != nullptr;
     const int64_t p0 = (int64_t)blockIdx.x * chunk;
-    for_particles(x, y, z, w, p0, min(chunk, np - p0), [&](int, float px, float py, float pz, float wt) {
-        const unsigned long long before = my_lost;
-        append_one<SCHEME, kCursorStride>(px, py, pz, wt, g, table, payload, cap, ovf, my_lost, SLAB ? slab : 0u);
-        if (SLAB && weighted && my_lost == before) weight_stats(wt, my_wmax, my_neg, my_wminc);
+    const int count = (int)max((int64_t)0, min((int64_t)chunk, np - p0));
+    for_particles<kScatterThreads>(x, y, z, w, p0, count, [&](int, float px, float py, float pz, float wt) {
+        const bool in = append_one<SCHEME>(px, py, pz, wt, g, table, payload, cap, ovf, SLAB ? slab : 0u);
+        if (SLAB && !in) ++my_lost;
+        if (SLAB && in && weighted) ws.add(wt);
     });
-    if (SLAB) flush_stats(my_lost, my_wmax, my_neg, my_wminc, lost, wstat);
+    if (SLAB) flush_stats(my_lost, ws, lost, wstat);
 }
 
-// Pass 3, staged: each CTA sorts a tile of particles' records by brick in
-// shared memory and appends every brick's run with one cursor atomic and
-// consecutive 16-byte stores.
-//   1. each particle's record for its first brick goes to its stage slot; a
-//      shared counter per brick gives its rank in the tile.  Particles whose
-//      stencil crosses brick faces are queued;
+// ---- staged scatter ---------------------------------------------------------
+// A CTA sorts a tile of particles by bin in shared memory and appends every
+// bin's run with one cursor atomic and consecutive 16-byte stores.
+//   LEVEL 0: particles straight into bricks (bins: all bricks);
+//   LEVEL 1: particles (x, y, z, w) into super-bricks, boxes of s.gs bricks,
+//            by an approximate home cell; anything outside the box or not
+//            finite goes to a last bin (bins: s.count + 1);
+//   LEVEL 2: the particles of one super-brick into bricks (bins: its bricks
+//            and one more on every side); a brick outside them and the last
+//            bin's particles are appended one by one.
+// One level costs a cursor atomic and a run of a few records per brick and
+// tile (4.6 records at 256^3 with tiles of 8192); two levels write the
+// particles once more but both in long runs.  16.8 M particles onto 256^3
+// (2048 bricks), NGP, CIC, TSC: one level 216, 284, 325 us, two levels 316,
+// 410, 443, record by record 345, 441, 530.  134 M CIC particles onto 512^3
+// (16384 bricks, more than a tile counts): two levels 3.09 ms, record by
+// record 4.64.
+// Steps of a tile:
+//   1. each particle's record for its first brick (LEVEL 1: the particle)
+//      goes to its stage slot, and a shared counter per bin gives its rank
+//      among the tile's.  Particles whose stencil crosses brick faces are
+//      queued;
 //   2. the queue's further records (next bricks) are staged the same way,
 //      by full warps; past the stage's capacity a record is appended on its
 //      own, as append_kernel does;
-//   3. per brick: the cursor is advanced by the tile's count (one atomic),
-//      and an exclusive scan of the counts orders the stage by brick (perm);
-//   4. records leave in that order: neighbouring threads write neighbouring
-//      slots of a brick's run.
-// Shared memory: stage [recs] 16 bytes, key and rank [recs] (18 + 14 bits),
-// bricks [nb], perm [recs] 16 bits (the queue lives there before step 3).
-// tile <= 8192, recs <= 16384, nb <= kStageBricks.
-constexpr int kStageThreads = 1024;
-constexpr int kStageBricks = 4096;
-constexpr int kStagePer = kStageBricks / kStageThreads;
-constexpr int kStageTile = 8192;
-constexpr size_t kStageSmem = 226 * 1024;
-__host__ __device__ constexpr size_t stage_bytes(int recs, int nb)
+//   3. per bin the cursor is advanced by the tile's count (one atomic, its
+//      latency behind the next steps), and an exclusive scan of the counts
+//      gives the bin's place in the order;
+//   4. slot and bin of every record are written to its place in the order
+//      (over its bin and rank, which every thread has read by then);
+//   5. records leave in that order: neighbouring threads write neighbouring
+//      slots of a bin's run.
+// What bounds it is the shared-memory pipe (two passes of 16 bytes per record
+// and a random 4-byte access per count, rank and place) and the instructions
+// of step 1.  Shared memory: stage [recs] 16 bytes, bins, order [recs] 4 bytes
+// (bin << 14 | rank, then bin << 14 | slot), the queue, LEVEL 2 the tile starts.
+constexpr int kStageBins = 4096;   // bins of a tile sort, LEVEL 0
+constexpr int kMaxSupers = 1023;
+constexpr int kMaxLocal = 1024;    // bricks around one super-brick, LEVEL 2 (10 bits in the queue)
+constexpr int kStageTile = 8192;   // particles per tile (13 bits in the queue)
+
+// One CTA of 1024 threads per SM for LEVEL 0, whose runs are the longer the
+// larger its tile (two of 512: 216 -> 221, 284 -> 296, 325 -> 335 us for NGP,
+// CIC, TSC as above); four of 256 for the others, whose runs are long anyway
+// (two of 512 at 512^3: LEVEL 1 0.98 -> 0.95 ms, LEVEL 2 2.16 -> 2.14).
+constexpr int stage_threads(int level) { return level == 0 ? 1024 : 256; }
+constexpr int stage_ctas(int level) { return 1024 / stage_threads(level); }
+constexpr size_t stage_budget(int level) { return (226 / stage_ctas(level) - 1) * 1024; }
+// bytes besides the 20 per record
+// Two levels where one level's tiles cannot count the bricks, for jobs with
+// tiles enough to fill the GPU twice.
+constexpr int64_t kTwoLevelParticles = 1000000;
+inline size_t stage_fixed(int level, int nbins)
 {
-    return (size_t)recs * 22 + (size_t)nb * 4 + 16;
+    return (size_t)nbins * 4 + (level == 2 ? (size_t)nbins * 8 + (kMaxSupers + 2) * 4 : 0);
 }
 
-template <int SCHEME, bool SLAB>
-__global__ void __launch_bounds__(kStageThreads, 1)
-staged_kernel(const float *__restrict__ x, const float *__restrict__ y, const float *__restrict__ z,
-              const float *__restrict__ w, int64_t np, int tile, int recs, const __grid_constant__ AssignGeom g, int nb,
-              uint32_t *__restrict__ table, uint4 *__restrict__ payload, unsigned long long *__restrict__ lost,
-              unsigned int *__restrict__ wstat, uint64_t cap, unsigned int *__restrict__ ovf, uint32_t slab)
+// Super-bricks: gs bricks per axis (the last may have fewer), ns per axis.
+struct SuperGeom {
+    int gs[3], ns[3];
+    int count;       // ns[0] ns[1] ns[2]
+    int D[3];        // LEVEL 2 bins per axis: gs + 2, or all bricks when ns = 1
+    float inv[3];    // 1 / (cells per super-brick)
+    unsigned dmagic[2];  // ceil(2^32 / D[2]), ceil(2^32 / D[1])
+    uint32_t cap;    // slots per super-brick (slabs), 0: dense ranges from beg
+};
+
+struct SortArgs {
+    const float *x, *y, *z, *w;  // LEVEL 0 and 1
+    int64_t np;
+    int tile, recs, nbins;
+    uint32_t *cursor;            // of the bricks (LEVEL 0, 2)
+    uint32_t *scursor;           // of the super-bricks (LEVEL 1, 2)
+    const uint32_t *sbeg;        // dense super-brick ranges [count + 2]
+    float4 *part;                // particles by super-brick
+    uint64_t part_cap;
+    uint4 *payload;
+    uint64_t cap;
+    uint32_t slab;
+    unsigned long long *lost;
+    unsigned int *wstat, *ovf;
+    int weighted;
+};
+
+__device__ __forceinline__ int super_of(const AssignGeom &g, const SuperGeom &s, float px, float py, float pz)
 {
-    extern __shared__ __align__(16) unsigned char stage_smem[];
-    __shared__ uint32_t warp_sums[kStageThreads / 32];
-    __shared__ uint32_t s_queued, s_extra, s_total;
-    uint4 *const stage = reinterpret_cast<uint4 *>(stage_smem);
-    uint32_t *const kr = reinterpret_cast<uint32_t *>(stage + recs);  // key << 14 | rank; ~0: no record
-    uint32_t *const bin = kr + recs;                                  // [nb]
-    uint16_t *const perm = reinterpret_cast<uint16_t *>(bin + nb);    // [recs]
+    const float p[3] = {px, py, pz};
+    int c[3];
+    bool in = true;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        const float u = (p[a] - g.mn[a]) * g.inv_d[a];
+        in = in && u >= 0.0f && u < g.nf[a];
+        c[a] = min((int)(u * s.inv[a]), s.ns[a] - 1);
+    }
+    return in ? (c[0] * s.ns[1] + c[1]) * s.ns[2] + c[2] : s.count;
+}
+
+// First slot of super-brick k and the particles it holds.
+__device__ __forceinline__ void super_range(const SortArgs &A, const SuperGeom &s, int k, uint32_t &beg, uint32_t &cnt)
+{
+    if (s.cap) {
+        beg = (uint32_t)k * s.cap;
+        cnt = min(A.scursor[k], k == s.count ? (uint32_t)(A.part_cap - beg) : s.cap);
+    } else {
+        beg = A.sbeg[k];
+        cnt = A.sbeg[k + 1] - beg;
+    }
+}
+
+// Tiles of LEVEL 2: tstart[k] = tiles of the super-bricks before k, for k in
+// [0, count + 1]; returns all tiles.  Called by every thread.
+template <int NT>
+__device__ __forceinline__ int tile_starts(const SortArgs &A, const SuperGeom &s, uint32_t *tstart, uint32_t *warp_sums)
+{
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-    const bool weighted = w != nullptr;
-    unsigned long long my_lost = 0;
-    unsigned int my_wmax = 0, my_neg = 0, my_wminc = 0;
-    const uint32_t slab_v = SLAB ? slab : 0u;
-    const int per = (nb + kStageThreads - 1) / kStageThreads;  // bricks per thread in step 3
-    for (int b = tid; b < nb; b += kStageThreads) bin[b] = 0u;
+    constexpr int PER = (kMaxSupers + 1 + NT - 1) / NT;
+    uint32_t n[PER], sum = 0;
+#pragma unroll
+    for (int j = 0; j < PER; ++j) {
+        const int k = tid * PER + j;
+        n[j] = 0;
+        if (k <= s.count) {
+            uint32_t beg, cnt;
+            super_range(A, s, k, beg, cnt);
+            n[j] = (cnt + (uint32_t)A.tile - 1u) / (uint32_t)A.tile;
+        }
+        sum += n[j];
+    }
+    uint32_t incl = sum;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+        const uint32_t v = __shfl_up_sync(0xffffffffu, incl, off);
+        if (lane >= off) incl += v;
+    }
+    if (lane == 31) warp_sums[wid] = incl;
+    __syncthreads();
+    uint32_t before = 0;
+    for (int k = 0; k < wid; ++k) before += warp_sums[k];
+    uint32_t run = before + incl - sum;
+#pragma unroll
+    for (int j = 0; j < PER; ++j) {
+        const int k = tid * PER + j;
+        if (k <= s.count) tstart[k] = run;
+        run += n[j];
+        if (k == s.count) tstart[k + 1] = run;
+    }
+    __syncthreads();
+    return (int)tstart[s.count + 1];
+}
+
+// The super-brick of tile t: the last k with tstart[k] <= t (and a tile).
+__device__ __forceinline__ int super_of_tile(const uint32_t *tstart, int count, int t)
+{
+    int lo = 0, hi = count;
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (tstart[mid] <= (uint32_t)t) lo = mid;
+        else hi = mid - 1;
+    }
+    return lo;
+}
+
+// First brick of super-brick k's bins along each axis.
+__device__ __forceinline__ void local_origin(const SuperGeom &s, int k, int o[3])
+{
+    const int c2 = k % s.ns[2], r = k / s.ns[2];
+    const int c1 = r % s.ns[1], c0 = r / s.ns[1];
+    o[0] = s.ns[0] == 1 ? 0 : c0 * s.gs[0] - 1;
+    o[1] = s.ns[1] == 1 ? 0 : c1 * s.gs[1] - 1;
+    o[2] = s.ns[2] == 1 ? 0 : c2 * s.gs[2] - 1;
+}
+// Brick coordinate bl as a coordinate of those bins (>= D: not among them),
+// and back.
+__device__ __forceinline__ int to_local(const AssignGeom &g, int a, int o, int bl)
+{
+    const int l = bl - o;
+    return l < 0 ? l + g.nb[a] : (l >= g.nb[a] ? l - g.nb[a] : l);
+}
+__device__ __forceinline__ int to_brick(const AssignGeom &g, int a, int o, int l)
+{
+    int b = o + l;
+    if (b < 0) b += g.nb[a];
+    if (b >= g.nb[a]) b -= g.nb[a];
+    return b;
+}
+
+// As for_particles, for particles stored as (x, y, z, w).
+template <int NT, typename F>
+__device__ __forceinline__ void for_packed(const float4 *__restrict__ in, int count, F &&one)
+{
+    int i = threadIdx.x;
+#pragma unroll 1
+    for (; i + NT < count; i += 2 * NT) {
+        const float4 a = __ldcs(in + i), b = __ldcs(in + i + NT);
+        one(i, a.x, a.y, a.z, a.w);
+        one(i + NT, b.x, b.y, b.z, b.w);
+    }
+    if (i < count) {
+        const float4 a = __ldcs(in + i);
+        one(i, a.x, a.y, a.z, a.w);
+    }
+}
+
+template <int SCHEME, bool SLAB, int LEVEL>
+__global__ void __launch_bounds__(stage_threads(LEVEL), stage_ctas(LEVEL))
+sort_kernel(const __grid_constant__ SortArgs A, const __grid_constant__ AssignGeom g, const __grid_constant__ SuperGeom s)
+{
+    constexpr int NT = stage_threads(LEVEL);
+    constexpr int MAXBINS = LEVEL == 0 ? kStageBins : (LEVEL == 1 ? kMaxSupers + 1 : kMaxLocal);
+    constexpr int PER = (MAXBINS + NT - 1) / NT;
+    constexpr uint32_t kNone = ~0u;
+    constexpr int MAXREC = ((int)stage_budget(LEVEL) / 20 + NT - 1) / NT;  // records per thread
+    extern __shared__ __align__(16) unsigned char stage_smem[];
+    __shared__ uint32_t warp_sums[32];
+    __shared__ uint32_t s_queued, s_extra, s_total;
+    const int nbins = A.nbins, tile = A.tile, recs = A.recs;
+    uint4 *const stage = reinterpret_cast<uint4 *>(stage_smem);
+    uint32_t *const bin = reinterpret_cast<uint32_t *>(stage + recs);  // [nbins]
+    uint32_t *const brick = bin + nbins;                               // LEVEL 2 [nbins]: the bin's brick
+    uint32_t *const limit = brick + nbins;                             // LEVEL 2 [nbins]: end of its slots
+    uint32_t *const tstart = limit + nbins;                            // LEVEL 2 [kMaxSupers + 2]
+    uint32_t *const order = LEVEL == 2 ? tstart + kMaxSupers + 2 : bin + nbins;  // [recs]
+    uint16_t *const queue = reinterpret_cast<uint16_t *>(order + recs);          // [tile], LEVEL 0 and 2
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    const uint32_t slab = SLAB ? A.slab : 0u;
+    unsigned int my_lost = 0;
+    WeightStats ws;
+    const int per = (nbins + NT - 1) / NT;  // bins per thread in step 3
+    for (int b = tid; b < nbins; b += NT) bin[b] = 0u;
     if (tid == 0) s_queued = s_extra = 0u;
     __syncthreads();
-    for (int64_t p0 = (int64_t)blockIdx.x * tile; p0 < np; p0 += (int64_t)gridDim.x * tile) {
-        const int count = (int)min((int64_t)tile, np - p0);
-        // 1. first bricks
-        for_particles(x, y, z, w, p0, count, [&](int i, float px, float py, float pz, float wt) {
-            const float pos[3] = {px, py, pz};
-            int c[3], bl[3], cl[3];
-            float t[3] = {0.f, 0.f, 0.f};
-            if (!locate<SCHEME, true>(pos, g, c, t)) {
-                if (SLAB) ++my_lost;
-                kr[i] = ~0u;
+    int64_t tiles;
+    int64_t t0, t1, tstep;
+    if (LEVEL == 2) {  // consecutive tiles: the super-brick changes rarely
+        tiles = tile_starts<NT>(A, s, tstart, warp_sums);
+        const int64_t each = (tiles + gridDim.x - 1) / gridDim.x;
+        t0 = blockIdx.x * each;
+        t1 = min(tiles, t0 + each);
+        tstep = 1;
+    } else {
+        tiles = (A.np + tile - 1) / tile;
+        t0 = blockIdx.x;
+        t1 = tiles;
+        tstep = gridDim.x;
+    }
+    int sup = -1, org[3] = {0, 0, 0};
+    for (int64_t t = t0; t < t1; t += tstep) {
+        int count;
+        int64_t p0 = 0;
+        if (LEVEL == 2) {
+            int k = sup < 0 ? super_of_tile(tstart, s.count, (int)t) : sup;
+            while (tstart[k + 1] <= (uint32_t)t) ++k;
+            uint32_t beg, cnt;
+            super_range(A, s, k, beg, cnt);
+            const uint32_t off = ((uint32_t)t - tstart[k]) * (uint32_t)tile;
+            p0 = (int64_t)beg + off;
+            count = (int)min((uint32_t)tile, cnt - off);
+            if (k == s.count) {  // outside the box, wrapped or lost: one by one
+                for_packed<NT>(A.part + p0, count, [&](int, float px, float py, float pz, float wt) {
+                    const bool in = append_one<SCHEME>(px, py, pz, wt, g, A.cursor, A.payload, A.cap,
+                                                                      A.ovf, slab);
+                    if (SLAB && !in) ++my_lost;
+                    if (SLAB && in && A.weighted) ws.add(wt);
+                });
+                sup = k;
+                continue;
+            }
+            if (k != sup) {
+                sup = k;
+                local_origin(s, k, org);
+                for (int b = tid; b < nbins; b += NT) {
+                    const int l2 = b % s.D[2], r = b / s.D[2];
+                    const int gk = (to_brick(g, 0, org[0], r / s.D[1]) * g.nb[1] + to_brick(g, 1, org[1], r % s.D[1])) *
+                                       g.nb[2] + to_brick(g, 2, org[2], l2);
+                    brick[b] = (uint32_t)gk;
+                    limit[b] = slab ? (uint32_t)(gk + 1) * slab : (uint32_t)min(A.cap, (uint64_t)0xffffffffu);
+                }
+                __syncthreads();
+            }
+        } else {
+            p0 = t * tile;
+            count = (int)min((int64_t)tile, A.np - p0);
+        }
+        // 1. first bins
+        auto first = [&](int i, float px, float py, float pz, float wt) {
+            if (LEVEL == 1) {
+                const int key = super_of(g, s, px, py, pz);
+                const uint32_t rank = atomicAdd(bin + key, 1u);
+                stage[i] = make_uint4(__float_as_uint(px), __float_as_uint(py), __float_as_uint(pz), __float_as_uint(wt));
+                order[i] = ((uint32_t)key << 14) | rank;
                 return;
             }
-            if (SLAB && weighted) weight_stats(wt, my_wmax, my_neg, my_wminc);
+            int c[3], bl[3], cl[3];
+            uint32_t off[3];
+            if (!locate<SCHEME, true>(px, py, pz, g, c, off)) {
+                if (SLAB) ++my_lost;
+                order[i] = kNone;
+                return;
+            }
+            if (SLAB && A.weighted) ws.add(wt);
             unsigned cross = 0;
 #pragma unroll
             for (int a = 0; a < 3; ++a) cross |= brick_axis<SCHEME>(g, a, c[a], bl[a], cl[a]) ? 1u << a : 0u;
-            const int key = (bl[0] * g.nb[1] + bl[1]) * g.nb[2] + bl[2];
+            int key;
+            if (LEVEL == 0) {
+                key = (bl[0] * g.nb[1] + bl[1]) * g.nb[2] + bl[2];
+            } else {
+                const int l0 = to_local(g, 0, org[0], bl[0]), l1 = to_local(g, 1, org[1], bl[1]),
+                          l2 = to_local(g, 2, org[2], bl[2]);
+                if (l0 >= s.D[0] || l1 >= s.D[1] || l2 >= s.D[2]) {
+                    order[i] = kNone;
+                    append_one<SCHEME>(px, py, pz, wt, g, A.cursor, A.payload, A.cap, A.ovf, slab);
+                    return;
+                }
+                key = (l0 * s.D[1] + l1) * s.D[2] + l2;
+            }
             const uint32_t rank = atomicAdd(bin + key, 1u);
-            stage[i] = make_uint4(pack_axis(cl[0], t[0]), pack_axis(cl[1], t[1]), pack_axis(cl[2], t[2]),
+            stage[i] = make_uint4(pack_axis(cl[0], off[0]), pack_axis(cl[1], off[1]), pack_axis(cl[2], off[2]),
                                   __float_as_uint(wt));
-            kr[i] = ((uint32_t)key << 14) | rank;
-            if (SCHEME != CAM_NGP && cross) perm[atomicAdd(&s_queued, 1u)] = (uint16_t)(i | (cross << 13));
-        });
+            order[i] = ((uint32_t)key << 14) | rank;
+            if (SCHEME != CAM_NGP && cross) queue[atomicAdd(&s_queued, 1u)] = (uint16_t)(i | (cross << 13));
+        };
+        if (LEVEL == 2) for_packed<NT>(A.part + p0, count, first);
+        else for_particles<NT>(A.x, A.y, A.z, A.w, p0, count, first);
         __syncthreads();
         // 2. the next bricks of the queued particles
-        if (SCHEME != CAM_NGP) {
+        if (LEVEL != 1 && SCHEME != CAM_NGP) {
             const int nq = (int)s_queued;
-            for (int q = tid; q < nq; q += kStageThreads) {
-                const unsigned ent = perm[q];
+            const int d1 = LEVEL == 0 ? g.nb[1] : s.D[1], d2 = LEVEL == 0 ? g.nb[2] : s.D[2];
+            for (int q = tid; q < nq; q += NT) {
+                const unsigned ent = queue[q];
                 const int i = (int)(ent & 8191u);
                 const unsigned cross = ent >> 13;
                 const uint4 rec = stage[i];
-                const int key = (int)(kr[i] >> 14);
-                int bl[3], step[3];
-                const int r = g.nb[2] == 1 ? key : (int)__umulhi((unsigned)key, g.kmagic[0]);
-                bl[2] = key - r * g.nb[2];
-                bl[0] = g.nb[1] == 1 ? r : (int)__umulhi((unsigned)r, g.kmagic[1]);
-                bl[1] = r - bl[0] * g.nb[1];
-                key_steps(g, bl, step);
+                const int key = (int)(order[i] >> 14);
+                const int r = d2 == 1 ? key : (int)__umulhi((unsigned)key, LEVEL == 0 ? g.kmagic[0] : s.dmagic[0]);
+                int l[3], bl[3], step[3];
+                l[2] = key - r * d2;
+                l[0] = d1 == 1 ? r : (int)__umulhi((unsigned)r, LEVEL == 0 ? g.kmagic[1] : s.dmagic[1]);
+                l[1] = r - l[0] * d1;
+                unsigned outside = 0u;  // LEVEL 2: axes along which the next brick is not among the bins
+                if (LEVEL == 0) {
+                    bl[0] = l[0];
+                    bl[1] = l[1];
+                    bl[2] = l[2];
+                    key_steps(g, bl, step);
+                } else {
+                    const int stride[3] = {d1 * d2, d2, 1};
+#pragma unroll
+                    for (int a = 0; a < 3; ++a) {
+                        bl[a] = to_brick(g, a, org[a], l[a]);
+                        step[a] = stride[a];
+                        if (l[a] + 1 == s.D[a]) {
+                            step[a] = -l[a] * stride[a];  // every brick of the axis is a bin: periodic
+                            if (s.ns[a] > 1) outside |= 1u << a;
+                        }
+                    }
+                }
+#pragma unroll 1
                 for (unsigned m = cross; m; m = (m - 1u) & cross) {
-                    const int k = key + (m & 1u ? step[0] : 0) + (m & 2u ? step[1] : 0) + (m & 4u ? step[2] : 0);
                     const uint4 nrec = next_brick_record(g, rec, bl, m);
-                    const int at = tile + (int)atomicAdd(&s_extra, 1u);
+                    int k = key + (m & 1u ? step[0] : 0) + (m & 2u ? step[1] : 0) + (m & 4u ? step[2] : 0);
+                    int at = recs;
+                    if (!(m & outside)) at = tile + (int)atomicAdd(&s_extra, 1u);
                     if (at < recs) {
                         const uint32_t rank = atomicAdd(bin + k, 1u);
                         stage[at] = nrec;
-                        kr[at] = ((uint32_t)k << 14) | rank;
+                        order[at] = ((uint32_t)k << 14) | rank;
                     } else {
-                        put_record(payload, nrec, k, atomicAdd(table + (int64_t)k * kCursorStride, 1u), slab_v, cap, ovf);
+                        if (LEVEL == 2) {
+                            int gs[3];
+                            key_steps(g, bl, gs);
+                            k = (bl[0] * g.nb[1] + bl[1]) * g.nb[2] + bl[2] + (m & 1u ? gs[0] : 0) +
+                                (m & 2u ? gs[1] : 0) + (m & 4u ? gs[2] : 0);
+                        }
+                        put_record(A.payload, nrec, k, atomicAdd(A.cursor + k, 1u), slab, A.cap,
+                                   A.ovf);
                     }
                 }
             }
             __syncthreads();
         }
-        // 3. cursors and the order by brick
-        const int extra = min((int)s_extra, recs - tile);
-        uint32_t base[kStagePer];
+        // 3. cursors and the bins' places
+        const int extra = LEVEL == 1 ? 0 : min((int)s_extra, recs - tile);
+        uint32_t slot0[PER], place[PER];  // of the run's first record
         {
-            uint32_t cnt[kStagePer], sum = 0;
+            uint32_t cnt[PER], sum = 0;
 #pragma unroll
-            for (int j = 0; j < kStagePer; ++j) {
+            for (int j = 0; j < PER; ++j) {
                 const int b = tid * per + j;
-                cnt[j] = j < per && b < nb ? bin[b] : 0u;
-                base[j] = cnt[j] ? atomicAdd(table + (int64_t)b * kCursorStride, cnt[j]) : 0u;
+                cnt[j] = j < per && b < nbins ? bin[b] : 0u;
+                slot0[j] = 0u;
+                if (cnt[j]) {
+                    const int at = LEVEL == 2 ? (int)brick[b] : b;
+                    slot0[j] = atomicAdd((LEVEL == 1 ? A.scursor : A.cursor) + at, cnt[j]);
+                }
                 sum += cnt[j];
             }
             uint32_t incl = sum;
@@ -280,67 +554,246 @@ staged_kernel(const float *__restrict__ x, const float *__restrict__ y, const fl
             }
             if (lane == 31) warp_sums[wid] = incl;
             __syncthreads();
-            if (wid == 0) {
-                const uint32_t ws = warp_sums[lane];
-                uint32_t wi = ws;
+            uint32_t run = __reduce_add_sync(0xffffffffu, lane < wid ? warp_sums[lane] : 0u) + incl - sum;
+            if (tid == NT - 1) s_total = run + sum;
 #pragma unroll
-                for (int off = 1; off < 32; off <<= 1) {
-                    const uint32_t v = __shfl_up_sync(0xffffffffu, wi, off);
-                    if (lane >= off) wi += v;
-                }
-                warp_sums[lane] = wi - ws;
-                if (lane == 31) s_total = wi;
-            }
-            __syncthreads();
-            uint32_t run = warp_sums[wid] + incl - sum;
-#pragma unroll
-            for (int j = 0; j < kStagePer; ++j) {
+            for (int j = 0; j < PER; ++j) {
                 const int b = tid * per + j;
-                if (j < per && b < nb) bin[b] = run;
+                if (j < per && b < nbins) bin[b] = run;
+                place[j] = run;
                 run += cnt[j];
             }
         }
         __syncthreads();
-        for (int i = tid; i < count; i += kStageThreads) {
-            const uint32_t k = kr[i];
-            if (k != ~0u) perm[bin[k >> 14] + (k & 16383u)] = (uint16_t)i;
-        }
-        for (int i = tile + tid; i < tile + extra; i += kStageThreads) {
-            const uint32_t k = kr[i];
-            perm[bin[k >> 14] + (k & 16383u)] = (uint16_t)i;
-        }
-        __syncthreads();
+        // 4. the order
+        {
+            const int end = tile + extra;
+            uint32_t to[MAXREC], what[MAXREC];
 #pragma unroll
-        for (int j = 0; j < kStagePer; ++j) {
+            for (int j = 0; j < MAXREC; ++j) {
+                const int i = tid + j * NT;
+                const uint32_t o = i < count || (i >= tile && i < end) ? order[i] : kNone;
+                to[j] = kNone;
+                if (o != kNone) to[j] = bin[o >> 14] + (o & 16383u);
+                what[j] = (o & ~16383u) | (uint32_t)i;
+            }
+            __syncthreads();
+#pragma unroll
+            for (int j = 0; j < MAXREC; ++j)
+                if (to[j] != kNone) order[to[j]] = what[j];
+        }
+#pragma unroll
+        for (int j = 0; j < PER; ++j) {
             const int b = tid * per + j;
-            if (j < per && b < nb) bin[b] = base[j];
+            if (j < per && b < nbins) {
+                uint32_t first_slot = slot0[j] - place[j];
+                if (LEVEL == 2 && SLAB) first_slot += brick[b] * slab;
+                if (LEVEL == 1) first_slot += (uint32_t)b * s.cap;
+                bin[b] = first_slot;
+            }
         }
         __syncthreads();
-        // 4. out, in brick order
+        // 5. out, in that order
         const int total = (int)s_total;
-#pragma unroll 2
-        for (int i = tid; i < total; i += kStageThreads) {
-            const int at = perm[i];
-            const uint32_t k = kr[at];
-            put_record(payload, stage[at], (int)(k >> 14), bin[k >> 14] + (k & 16383u), slab_v, cap, ovf);
+        bool over = false;
+#pragma unroll 4
+        for (int i = tid; i < total; i += NT) {
+            const uint32_t o = order[i];
+            const unsigned k = o >> 14;
+            const uint4 rec = stage[o & 16383u];
+            const uint32_t slot = bin[k] + (uint32_t)i;
+            uint64_t at = slot;
+            bool fits;
+            if (LEVEL == 0) {
+                fits = SLAB ? slot < slab : slot < A.cap;
+                if (SLAB) at = (uint64_t)k * slab + slot;
+            } else if (LEVEL == 1) {
+                // the last bin takes what is left of the buffer
+                fits = s.cap && (int)k < s.count ? slot < (k + 1u) * s.cap : slot < A.part_cap;
+            } else {
+                fits = slot < limit[k];
+            }
+            if (fits) (LEVEL == 1 ? reinterpret_cast<uint4 *>(A.part) : A.payload)[at] = rec;
+            over = over || !fits;
         }
+        if (over) atomicOr(A.ovf, 1u);
         __syncthreads();
-        for (int b = tid; b < nb; b += kStageThreads) bin[b] = 0u;
+        for (int b = tid; b < nbins; b += NT) bin[b] = 0u;
         if (tid == 0) s_queued = s_extra = 0u;
         __syncthreads();
     }
-    if (SLAB) flush_stats(my_lost, my_wmax, my_neg, my_wminc, lost, wstat);
+    if (SLAB && LEVEL != 1) flush_stats(my_lost, ws, A.lost, A.wstat);
+}
+
+// Particles per super-brick (two levels, exact ranges).
+__global__ void __launch_bounds__(kBinThreads)
+super_count_kernel(const __grid_constant__ SortArgs A, const __grid_constant__ AssignGeom g,
+                   const __grid_constant__ SuperGeom s, unsigned chunk)
+{
+    __shared__ uint32_t hist[kMaxSupers + 1];
+    for (int i = threadIdx.x; i <= s.count; i += kBinThreads) hist[i] = 0u;
+    __syncthreads();
+    const int64_t p0 = (int64_t)blockIdx.x * chunk;
+    const int count = (int)max((int64_t)0, min((int64_t)chunk, A.np - p0));
+    for_particles<kBinThreads>(A.x, A.y, A.z, (const float *)nullptr, p0, count,
+                               [&](int, float px, float py, float pz, float) {
+                                   atomicAdd(hist + super_of(g, s, px, py, pz), 1u);
+                               });
+    __syncthreads();
+    for (int i = threadIdx.x; i <= s.count; i += kBinThreads)
+        if (hist[i]) atomicAdd(A.scursor + i, hist[i]);
+}
+
+// Super-brick ranges from their counts (one CTA): beg[k], beg[count + 1] =
+// all particles, cursors at their starts, *fullest = the largest count of a
+// super-brick (the last bin left out).
+__global__ void __launch_bounds__(1024)
+super_offsets_kernel(uint32_t *__restrict__ scursor, int count, uint32_t *__restrict__ beg, unsigned int *__restrict__ fullest)
+{
+    __shared__ uint32_t sums[32];
+    const int k = threadIdx.x, lane = k & 31, wid = k >> 5;
+    const uint32_t n = k <= count ? scursor[k] : 0u;
+    uint32_t incl = n;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+        const uint32_t v = __shfl_up_sync(0xffffffffu, incl, off);
+        if (lane >= off) incl += v;
+    }
+    if (lane == 31) sums[wid] = incl;
+    __syncthreads();
+    uint32_t before = 0;
+    for (int w = 0; w < wid; ++w) before += sums[w];
+    if (k <= count) {
+        beg[k] = before + incl - n;
+        scursor[k] = before + incl - n;
+        if (k == count) beg[k + 1] = before + incl;
+    }
+    const unsigned m = __reduce_max_sync(0xffffffffu, k < count ? n : 0u);
+    if (lane == 0 && m) atomicMax(fullest, m);
+}
+
+// Records per brick from particles sorted by super-brick (the count pass of
+// two levels): a shared histogram over the super-brick's bins, flushed when
+// the super-brick changes, with the lost count and weight statistics.
+template <int SCHEME>
+__global__ void __launch_bounds__(512, 2)
+super_tally_kernel(const __grid_constant__ SortArgs A, const __grid_constant__ AssignGeom g,
+                   const __grid_constant__ SuperGeom s)
+{
+    constexpr int NT = 512;
+    extern __shared__ __align__(16) unsigned char tally_smem[];
+    __shared__ uint32_t warp_sums[32];
+    __shared__ uint32_t s_queued;
+    uint32_t *const bin = reinterpret_cast<uint32_t *>(tally_smem);  // [nbins]
+    uint32_t *const tstart = bin + A.nbins;                          // [kMaxSupers + 2]
+    uint16_t *const queue = reinterpret_cast<uint16_t *>(tstart + kMaxSupers + 2);  // [tile]: key | cross << 10
+    const int tid = threadIdx.x;
+    unsigned int my_lost = 0;
+    WeightStats ws;
+    for (int b = tid; b < A.nbins; b += NT) bin[b] = 0u;
+    if (tid == 0) s_queued = 0u;
+    __syncthreads();
+    const int64_t tiles = tile_starts<NT>(A, s, tstart, warp_sums);
+    const int64_t each = (tiles + gridDim.x - 1) / gridDim.x;
+    const int64_t t0 = blockIdx.x * each, t1 = min(tiles, t0 + each);
+    int sup = -1, org[3] = {0, 0, 0};
+    auto flush = [&]() {
+        for (int b = tid; b < A.nbins; b += NT) {
+            const uint32_t n = bin[b];
+            if (!n) continue;
+            const int l2 = b % s.D[2], r = b / s.D[2];
+            const int gk = (to_brick(g, 0, org[0], r / s.D[1]) * g.nb[1] + to_brick(g, 1, org[1], r % s.D[1])) * g.nb[2] +
+                           to_brick(g, 2, org[2], l2);
+            atomicAdd(A.cursor + gk, n);
+            bin[b] = 0u;
+        }
+    };
+    for (int64_t t = t0; t < t1; ++t) {
+        int k = sup < 0 ? super_of_tile(tstart, s.count, (int)t) : sup;
+        while (tstart[k + 1] <= (uint32_t)t) ++k;
+        uint32_t beg, cnt;
+        super_range(A, s, k, beg, cnt);
+        const uint32_t off = ((uint32_t)t - tstart[k]) * (uint32_t)A.tile;
+        const float4 *in = A.part + beg + off;
+        const int count = (int)min((uint32_t)A.tile, cnt - off);
+        if (k != sup) {
+            if (sup >= 0 && sup < s.count) flush();
+            sup = k;
+            if (k < s.count) local_origin(s, k, org);
+            __syncthreads();
+        }
+        if (k == s.count) {
+            for_packed<NT>(in, count, [&](int, float px, float py, float pz, float wt) {
+                count_one<SCHEME, false>(px, py, pz, wt, A.weighted != 0, g, nullptr, A.cursor, my_lost, ws);
+            });
+            continue;
+        }
+        for_packed<NT>(in, count, [&](int, float px, float py, float pz, float wt) {
+            int c[3], bl[3], cl;
+            uint32_t o[3];
+            if (!locate<SCHEME, false>(px, py, pz, g, c, o)) {
+                ++my_lost;
+                return;
+            }
+            unsigned cross = 0;
+#pragma unroll
+            for (int a = 0; a < 3; ++a) cross |= brick_axis<SCHEME>(g, a, c[a], bl[a], cl) ? 1u << a : 0u;
+            const int l0 = to_local(g, 0, org[0], bl[0]), l1 = to_local(g, 1, org[1], bl[1]),
+                      l2 = to_local(g, 2, org[2], bl[2]);
+            // a stencil that leaves the bins (never, but for a particle the
+            // approximate home cell put on the wrong side)
+            bool in_bins = l0 < s.D[0] && l1 < s.D[1] && l2 < s.D[2];
+            if (SCHEME != CAM_NGP)
+                in_bins = in_bins && !((cross & 1u) && s.ns[0] > 1 && l0 + 1 == s.D[0]) &&
+                          !((cross & 2u) && s.ns[1] > 1 && l1 + 1 == s.D[1]) &&
+                          !((cross & 4u) && s.ns[2] > 1 && l2 + 1 == s.D[2]);
+            if (!in_bins) {
+                count_one<SCHEME, false>(px, py, pz, wt, A.weighted != 0, g, nullptr, A.cursor, my_lost, ws);
+                return;
+            }
+            if (A.weighted) ws.add(wt);
+            const int key = (l0 * s.D[1] + l1) * s.D[2] + l2;
+            atomicAdd(bin + key, 1u);
+            if (SCHEME != CAM_NGP && cross) queue[atomicAdd(&s_queued, 1u)] = (uint16_t)(key | (cross << 10));
+        });
+        __syncthreads();
+        if (SCHEME != CAM_NGP) {
+            const int nq = (int)s_queued;
+            for (int q = tid; q < nq; q += NT) {
+                const unsigned ent = queue[q];
+                const int key = (int)(ent & 1023u);
+                const unsigned cross = ent >> 10;
+                const int r = s.D[2] == 1 ? key : (int)__umulhi((unsigned)key, s.dmagic[0]);
+                int l[3], step[3];
+                l[2] = key - r * s.D[2];
+                l[0] = s.D[1] == 1 ? r : (int)__umulhi((unsigned)r, s.dmagic[1]);
+                l[1] = r - l[0] * s.D[1];
+                const int stride[3] = {s.D[1] * s.D[2], s.D[2], 1};
+#pragma unroll
+                for (int a = 0; a < 3; ++a) step[a] = l[a] + 1 == s.D[a] ? -l[a] * stride[a] : stride[a];
+#pragma unroll 1
+                for (unsigned m = cross; m; m = (m - 1u) & cross)
+                    atomicAdd(bin + key + (m & 1u ? step[0] : 0) + (m & 2u ? step[1] : 0) + (m & 4u ? step[2] : 0), 1u);
+            }
+            __syncthreads();
+            if (tid == 0) s_queued = 0u;
+            __syncthreads();
+        }
+    }
+    __syncthreads();
+    if (sup >= 0 && sup < s.count) flush();
+    flush_stats(my_lost, ws, A.lost, A.wstat);
 }
 
 // Brick starts in one CTA (nb <= kOffThreads * kOffItems): thread t scans
 // the counts of bricks [t * kOffItems, (t + 1) * kOffItems) in order, the
 // per-thread sums are scanned across the CTA, and every brick's start goes
-// to start[b] and to its padded cursor (which held its count); start[nb] =
+// to start[b] and to its cursor (which held its count); start[nb] =
 // *total = all records.
 constexpr int kOffThreads = 1024;
 constexpr int kOffItems = 16;
 __global__ void __launch_bounds__(kOffThreads)
-brick_offsets_kernel(uint32_t *__restrict__ padded, int nb, uint32_t *__restrict__ start, uint32_t *__restrict__ total)
+brick_offsets_kernel(uint32_t *__restrict__ table, int stride, int nb, uint32_t *__restrict__ start, uint32_t *__restrict__ total)
 {
     __shared__ uint32_t warp_sums[kOffThreads / 32];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -349,7 +802,7 @@ brick_offsets_kernel(uint32_t *__restrict__ padded, int nb, uint32_t *__restrict
     uint32_t s = 0;
 #pragma unroll
     for (int i = 0; i < kOffItems; ++i) {
-        v[i] = base + i < nb ? padded[(int64_t)(base + i) * kCursorStride] : 0u;
+        v[i] = base + i < nb ? table[(int64_t)(base + i) * stride] : 0u;
         s += v[i];
     }
     uint32_t incl = s;
@@ -380,7 +833,7 @@ brick_offsets_kernel(uint32_t *__restrict__ padded, int nb, uint32_t *__restrict
     for (int i = 0; i < kOffItems; ++i) {
         if (base + i < nb) {
             start[base + i] = run;
-            padded[(int64_t)(base + i) * kCursorStride] = run;
+            table[(int64_t)(base + i) * stride] = run;
         }
         run += v[i];
     }
@@ -399,23 +852,23 @@ brick_max_kernel(const uint32_t *__restrict__ start, int nb, unsigned int *__res
     if ((threadIdx.x & 31) == 0 && m) atomicMax(out, m);
 }
 
-// counts[b] = padded[b * kCursorStride] (contiguous, for the scan).
-__global__ void compact_counts_kernel(const uint32_t *__restrict__ padded, int nb, uint32_t *__restrict__ counts)
+// counts[b] = table[b * stride] (contiguous, for the scan).
+__global__ void compact_counts_kernel(const uint32_t *__restrict__ table, int stride, int nb, uint32_t *__restrict__ counts)
 {
     for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < nb; b += gridDim.x * blockDim.x)
-        counts[b] = padded[(int64_t)b * kCursorStride];
+        counts[b] = table[(int64_t)b * stride];
 }
 
 // start[b] = scanned count of brick b (its first payload), start[nb] = total;
-// the padded cursors start there.
+// the cursors start there.
 __global__ void brick_starts_kernel(const uint32_t *__restrict__ scanned, int nb,
                                     const uint32_t *__restrict__ total, uint32_t *__restrict__ start,
-                                    uint32_t *__restrict__ cursor)
+                                    uint32_t *__restrict__ cursor, int stride)
 {
     for (int b = blockIdx.x * blockDim.x + threadIdx.x; b <= nb; b += gridDim.x * blockDim.x) {
         const uint32_t v = b < nb ? scanned[b] : *total;
         start[b] = v;
-        if (b < nb) cursor[(int64_t)b * kCursorStride] = v;
+        if (b < nb) cursor[(int64_t)b * stride] = v;
     }
 }
 
@@ -450,7 +903,7 @@ deposit_kernel(const uint4 *__restrict__ payload, const uint32_t *__restrict__ s
     // flag); with slabs, the brick's records are the first of its slab (the
     // host keeps every slab index below 2^32)
     const uint32_t beg = slab ? (uint32_t)B * slab : min(start[B], nrec);
-    const uint32_t end = slab ? beg + min(slab_count[(int64_t)B * kCursorStride], slab) : min(start[B + 1], nrec);
+    const uint32_t end = slab ? beg + min(slab_count[(int64_t)B * g.cstride], slab) : min(start[B + 1], nrec);
     const bool nonneg = !weighted || wstat[1] == 0u;
     const int s = fixed_scale(wstat, weighted, end - beg);
     // 2^s as two exact factors (s may exceed the float exponent range)
@@ -532,34 +985,96 @@ AssignGeom make_geom(const cam_grid &gr, int scheme, int64_t np)
     for (int a = 0; a < 3; ++a) {
         while (g.b[a] < g.n[a] && g.n[a] % g.b[a] != 0 && g.n[a] % g.b[a] < 2 && g.b[a] > 3) --g.b[a];
         g.nb[a] = (g.n[a] + g.b[a] - 1) / g.b[a];
-        g.bmagic[a] = (unsigned)(((1ull << 32) + (uint64_t)g.b[a] - 1) / (uint64_t)g.b[a]);
         g.inv_d[a] = 1.0f / g.d[a];
         g.e_last[a] = g.n[a] - (g.nb[a] - 1) * g.b[a];
         g.nf[a] = (float)g.n[a];
-        // home_cell divides exactly when a quotient u <= n lies within
-        // 4e-7 max(u, 1) of an integer; a little more is set aside here
-        g.safe[a] = 0.5f - (4.2e-7f * (float)(g.n[a] + 1) + 1e-6f);
+        g.half_d[a] = 0.5f * g.d[a];
+        g.off_scale[a] = g.inv_d[a] * 16777216.0f;
         g.origin |= g.mn[a] != 0.0f;
+        // an axis that one brick spans: brick 0 always, nothing crosses
+        const bool whole = g.nb[a] == 1;
+        const int reach = scheme == CAM_TSC ? 2 : 1;  // from the stencil's first to its last cell
+        g.bmagic[a] = whole ? 0u : (unsigned)(((1ull << 32) + (uint64_t)g.b[a] - 1) / (uint64_t)g.b[a]);
+        g.lo0[a] = whole ? -1 : g.n[a] - 1;
+        g.cross_b[a] = whole ? INT32_MAX : g.b[a] - reach;
+        g.cross_n[a] = whole ? INT32_MAX : g.n[a] - reach;
+        // home_cell divides exactly when a quotient u <= n lies within
+        // 4e-7 max(u, 1) of an integer; a little more is set aside here.
+        // A quotient u < n - thr means x - min <= (n - thr) d (1 + 3e-7)
+        // before rounding, which is inside the box if that is below its
+        // rounded end less min.
+        const float thr = 4.2e-7f * (float)(g.n[a] + 1) + 1e-6f;
+        const double end = (double)(g.mn[a] + g.L[a]) - (double)g.mn[a];
+        const double nd = (double)g.n[a] * (double)g.d[a];
+        const bool regular = g.n[a] >= 4 && std::isfinite(g.off_scale[a]) && std::isnormal(g.inv_d[a]) && ((double)g.n[a] - thr) * g.d[a] * (1.0 + 3e-7) < end &&
+                             std::fabs(nd - (double)g.L[a]) <= 1e-3 * g.d[a] * std::max(1.0, 1e-3 * g.n[a]);
+        g.safe[a] = regular ? 0.5f - thr : -1.0f;
     }
     for (int a = 0; a < 2; ++a)
         g.kmagic[a] = g.nb[2 - a] > 1 ? (unsigned)(((1ull << 32) + (uint64_t)g.nb[2 - a] - 1) / (uint64_t)g.nb[2 - a]) : 0u;
-    (void)scheme;
+    g.cstride = 1;
     return g;
 }
 
+// The super-bricks of a mesh: brick groups doubled along the axis where they
+// are shortest until at most `most` remain.
+static SuperGeom super_geom(const AssignGeom &g, int most)
+{
+    SuperGeom s{};
+    for (int a = 0; a < 3; ++a) s.gs[a] = 1;
+    for (;;) {
+        int64_t count = 1;
+        int grow = -1;
+        for (int a = 0; a < 3; ++a) {
+            s.ns[a] = (g.nb[a] + s.gs[a] - 1) / s.gs[a];
+            count *= s.ns[a];
+            if (s.ns[a] > 1 && (grow < 0 || s.gs[a] * g.b[a] < s.gs[grow] * g.b[grow])) grow = a;
+        }
+        if (count <= most) {
+            s.count = (int)count;
+            break;
+        }
+        s.gs[grow] *= 2;
+    }
+    for (int a = 0; a < 3; ++a) {
+        s.D[a] = s.ns[a] == 1 ? g.nb[a] : s.gs[a] + 2;
+        s.inv[a] = 1.0f / (float)(s.gs[a] * g.b[a]);
+    }
+    for (int a = 0; a < 2; ++a)
+        s.dmagic[a] = (unsigned)(((1ull << 32) + (uint64_t)s.D[2 - a] - 1) / (uint64_t)std::max(s.D[2 - a], 2));
+    return s;
+}
+static int local_bins_of(const SuperGeom &s) { return s.D[0] * s.D[1] * s.D[2]; }
+
 template <int SCHEME>
 static void assign_impl(cam_ctx *ctx, const float *x, const float *y, const float *z,
-                        const float *w, int64_t np, const AssignGeom &g, AssignOut &out)
+                        const float *w, int64_t np, const AssignGeom &geom, AssignOut &out)
 {
-    const int64_t nb = (int64_t)g.nb[0] * g.nb[1] * g.nb[2];
+    const int64_t nb = (int64_t)geom.nb[0] * geom.nb[1] * geom.nb[2];
     CAM_REQUIRE(nb < (1ll << 31), CAM_E_UNSUPPORTED, "too many mesh bricks");
     // Count pass: one CTA of 1024 threads per SM (its brick histogram in
     // shared memory), contiguous chunks of >= 4096 particles.
     const int G = (int)std::max<int64_t>(1, std::min<int64_t>(kNumSMs, (np + 4095) / 4096));
-    const int64_t chunk = std::max<int64_t>(1, (np + G - 1) / G);
+    const unsigned chunk = (unsigned)std::max<int64_t>(1, (np + G - 1) / G);
     const bool smem_hist = nb <= kSmemBricks;
-    // per-brick counters, one per 128-byte line (counts, then cursors)
-    auto *table = static_cast<uint32_t *>(scratch(ctx, "asg.cursor", (size_t)nb * kCursorStride * sizeof(uint32_t)));
+    // Two levels of sorting when the records would otherwise leave a tile in
+    // runs of a few per brick.
+    const bool plain_ctx = !ctx->sync_free && !ctx->slabs_off && !ctx->budget;
+    SuperGeom sg{};
+    if (plain_ctx && nb > kStageBins && np >= kTwoLevelParticles && geom.safe[0] > 0.f && geom.safe[1] > 0.f &&
+        geom.safe[2] > 0.f)
+        // as few super-bricks as LEVEL 2 has bins for: LEVEL 1's runs are the
+        // longer (512^3: 128 of them 0.95 ms, 512 of them 1.87, LEVEL 2 alike)
+        for (int most = 128; most <= 1024 && sg.count == 0; most *= 2) {
+            const SuperGeom s = super_geom(geom, std::min(most, kMaxSupers));
+            if (local_bins_of(s) <= kMaxLocal) sg = s;
+        }
+    const bool two = sg.count > 0;
+    const bool staged = two || nb <= kStageBins;
+    AssignGeom g = geom;
+    g.cstride = staged ? 1 : kPaddedStride;
+    // per-brick counters (counts, then cursors)
+    auto *table = static_cast<uint32_t *>(scratch(ctx, "asg.cursor", (size_t)nb * g.cstride * sizeof(uint32_t)));
     auto *start = static_cast<uint32_t *>(scratch(ctx, "asg.start", (nb + 1) * sizeof(uint32_t)));
     auto *stats = static_cast<unsigned long long *>(scratch(ctx, "asg.stats", 64));
     auto *bsum = static_cast<double *>(scratch(ctx, "asg.bsum", nb * sizeof(double)));
@@ -567,7 +1082,7 @@ static void assign_impl(cam_ctx *ctx, const float *x, const float *y, const floa
     unsigned int *d_wmax = reinterpret_cast<unsigned int *>(stats + 1);
     uint32_t *d_total = reinterpret_cast<uint32_t *>(stats + 2);
     unsigned int *d_ovf = reinterpret_cast<unsigned int *>(stats + 3);
-    CAM_CUDA_TRY(cudaMemsetAsync(table, 0, (size_t)nb * kCursorStride * sizeof(uint32_t), ctx->stream));
+    CAM_CUDA_TRY(cudaMemsetAsync(table, 0, (size_t)nb * g.cstride * sizeof(uint32_t), ctx->stream));
     CAM_CUDA_TRY(cudaMemsetAsync(stats, 0, 64, ctx->stream));
 
     // Expected records per particle of a uniform catalogue: a stencil
@@ -584,40 +1099,119 @@ static void assign_impl(cam_ctx *ctx, const float *x, const float *y, const floa
     // sized from the clumping the last exact job run of this mesh shape
     // measured (a slab that overflows makes the job rerun exactly, which
     // measures again); no count pass and no scan then, and the scatter
-    // gathers the statistics.  Only while the slabs stay within twice the
-    // expected records (or 2^20 records): the scatter slows as the slabs
-    // spread its appends over more memory (256^3: 0.37 ms per job densely
-    // packed, 0.48 in slabs of twice, 0.55 of four times the mean brick).
+    // gathers the statistics.  With two levels the super-bricks get slabs of
+    // their own the same way.  Only while the slabs stay within twice the
+    // expected records (or 2^20 records), three times with two levels: one
+    // level's short runs slow down as the slabs spread them over more memory.
     // A context with an HBM budget keeps the exact path, whose payload the
     // budget was sized for.
     const double est_brick = (double)np * f / (double)nb;
     const int64_t shape = ((int64_t)g.n[0] << 32) | ((int64_t)g.n[1] << 16) | (int64_t)g.n[2];
+    double est_super = (double)np;
+    for (int a = 0; a < 3 && two; ++a)
+        est_super *= (double)std::min(sg.gs[a] * g.b[a], g.n[a]) / (double)g.n[a];
+    const uint64_t beyond = std::max<uint64_t>(65536, (uint64_t)np / 256);  // room of the last bin, with slabs
     uint32_t slab = 0;
-    if (out.defer && !ctx->sync_free && !ctx->slabs_off && !ctx->budget && np > 0) {
+    if (out.defer && plain_ctx && np > 0) {
         const auto it = ctx->slab_clump.find(shape);
-        if (it != ctx->slab_clump.end()) {
+        const auto is = ctx->super_clump.find(shape);
+        if (it != ctx->slab_clump.end() && (!two || is != ctx->super_clump.end())) {
             const uint64_t cap = slab_capacity(it->second * est_brick);
-            const double room = std::max(2.0 * (double)np * f, (double)(1u << 20));
-            if ((double)nb * (double)cap <= room && (uint64_t)nb * cap < (1ull << 32)) slab = (uint32_t)cap;
+            const double room = std::max((two ? 3.0 : 2.0) * (double)np * f, (double)(1u << 20));
+            bool fits = (double)nb * (double)cap <= room && (uint64_t)nb * cap < (1ull << 32);
+            if (two) {
+                const uint64_t scap = slab_capacity(is->second * est_super);
+                fits = fits && (double)sg.count * (double)scap <= 2.0 * (double)np + (double)(1u << 20) &&
+                       (uint64_t)sg.count * scap + beyond < (1ull << 32);
+                if (fits) sg.cap = (uint32_t)scap;
+            }
+            if (fits) slab = (uint32_t)cap;
         }
+    }
+    // What the sort kernels share; tile and recs are set per level.
+    SortArgs A{};
+    A.x = x;
+    A.y = y;
+    A.z = z;
+    A.w = w;
+    A.np = np;
+    A.cursor = table;
+    A.lost = d_lost;
+    A.wstat = d_wmax;
+    A.ovf = d_ovf;
+    A.slab = slab;
+    A.weighted = w != nullptr;
+    // Tiles as large as the stage holds with the expected records (15% margin
+    // on the extra ones); LEVEL 0 and 1: split evenly over the resident CTAs.
+    auto tile_for = [&](int level, int nbins, double records) {
+        A.nbins = nbins;
+        const size_t bytes = stage_budget(level) - stage_fixed(level, nbins);
+        const double fr = 1.0 + 1.15 * (records - 1.0);
+        const double each = 20.0 * fr + (level == 1 ? 0.0 : 2.0);
+        const int64_t most = std::max<int64_t>(512, std::min<int64_t>(kStageTile, (int64_t)((double)bytes / each)));
+        // a batch's jobs run beside each other: fewer, larger tiles cost less
+        // in all (64 jobs of 64^3: 4.82 ms split over 148, 4.51 over 32)
+        const int64_t ctas = ctx->sync_free ? 32 : stage_ctas(level) * kNumSMs;
+        const int64_t rounds = std::max<int64_t>(1, (np + ctas * most - 1) / (ctas * most));
+        const int64_t even = (np + ctas * rounds - 1) / (ctas * rounds);
+        A.tile = (int)(level == 2 ? most & ~(int64_t)31
+                                  : std::min<int64_t>(most, std::max<int64_t>(1024, (even + 31) & ~(int64_t)31)));
+        // small jobs leave the rest of the shared memory to other streams'
+        // kernels: no more than twice the expected further records
+        const size_t want = (size_t)((double)A.tile * (1.0 + 2.0 * (records - 1.0))) + (level == 1 ? 0 : 512);
+        A.recs = (int)std::min<size_t>(std::min<size_t>(16383, want), (bytes - (level == 1 ? 0 : (size_t)A.tile * 2)) / 20);
+        const int64_t tiles = (np + A.tile - 1) / A.tile;
+        return (unsigned)std::max<int64_t>(1, std::min<int64_t>(stage_ctas(level) * kNumSMs, tiles));
+    };
+    auto sort_bytes = [&](int level) {
+        return (size_t)A.recs * 20 + (level == 1 ? 0 : (size_t)A.tile * 2) + stage_fixed(level, A.nbins);
+    };
+    const int local_bins = two ? local_bins_of(sg) : 0;
+
+    if (two) {
+        A.part_cap = slab ? (uint64_t)sg.count * sg.cap + beyond : (uint64_t)np;
+        A.part = static_cast<float4 *>(scratch(ctx, "asg.part", A.part_cap * sizeof(float4)));
+        A.scursor = static_cast<uint32_t *>(
+            scratch(ctx, "asg.scursor", (size_t)(kMaxSupers + 1) * sizeof(uint32_t)));
+        auto *sbeg = static_cast<uint32_t *>(scratch(ctx, "asg.sbeg", (kMaxSupers + 3) * sizeof(uint32_t)));
+        A.sbeg = sbeg;
+        CAM_CUDA_TRY(cudaMemsetAsync(A.scursor, 0, (size_t)(sg.count + 1) * sizeof(uint32_t), ctx->stream));
+        if (!slab) {
+            CAM_LAUNCH_NAMED(ctx, "assign_super_count", super_count_kernel, G, kBinThreads, 0, A, g, sg, chunk);
+            CAM_LAUNCH_NAMED(ctx, "assign_starts", super_offsets_kernel, 1, 1024, 0, A.scursor, sg.count, sbeg,
+                             reinterpret_cast<unsigned int *>(stats + 6));
+            out.super_est = est_super;
+        }
+        const unsigned grid = tile_for(1, sg.count + 1, 1.0);
+        const size_t smem1 = sort_bytes(1);
+        auto k = sort_kernel<CAM_NGP, false, 1>;
+        smem_at_least(k, smem1);
+        CAM_LAUNCH_NAMED(ctx, "assign_super_sort", k, grid, stage_threads(1), smem1, A, g, sg);
     }
 
     const size_t hsmem = smem_hist ? (size_t)nb * sizeof(uint32_t) : 0;
     auto count_k = smem_hist ? count_kernel<SCHEME, true> : count_kernel<SCHEME, false>;
     if (!slab) {
-        smem_at_least(count_k, hsmem);
-        CAM_LAUNCH_NAMED(ctx, "assign_bin_count", count_k, G, kBinThreads, hsmem, x, y, z, w, np, chunk, g, (int)nb,
-                         table, d_lost, d_wmax);
+        if (two) {
+            A.nbins = local_bins;
+            A.tile = kStageTile;
+            const size_t tsmem = (size_t)local_bins * 4 + (kMaxSupers + 2) * 4 + (size_t)A.tile * 2;
+            CAM_LAUNCH_NAMED(ctx, "assign_bin_count", super_tally_kernel<SCHEME>, 2 * kNumSMs, 512, tsmem, A, g, sg);
+        } else {
+            smem_at_least(count_k, hsmem);
+            CAM_LAUNCH_NAMED(ctx, "assign_bin_count", count_k, G, kBinThreads, hsmem, x, y, z, w, np, chunk, g, (int)nb,
+                             table, d_lost, d_wmax);
+        }
         if (nb <= (int64_t)kOffThreads * kOffItems) {
-            CAM_LAUNCH_NAMED(ctx, "assign_starts", brick_offsets_kernel, 1, kOffThreads, 0, table, (int)nb, start,
+            CAM_LAUNCH_NAMED(ctx, "assign_starts", brick_offsets_kernel, 1, kOffThreads, 0, table, g.cstride, (int)nb, start,
                              d_total);
         } else {
             auto *counts = static_cast<uint32_t *>(scratch(ctx, "asg.counts", (size_t)nb * sizeof(uint32_t)));
-            const unsigned sg = (unsigned)std::min<int64_t>((nb + 256) / 256, 1024);
-            CAM_LAUNCH_NAMED(ctx, "assign_starts", compact_counts_kernel, sg, 256, 0, table, (int)nb, counts);
+            const unsigned blocks = (unsigned)std::min<int64_t>((nb + 256) / 256, 1024);
+            CAM_LAUNCH_NAMED(ctx, "assign_starts", compact_counts_kernel, blocks, 256, 0, table, g.cstride, (int)nb, counts);
             exclusive_scan_u32(ctx, counts, nb, d_total);
-            CAM_LAUNCH_NAMED(ctx, "assign_starts", brick_starts_kernel, sg, 256, 0, counts, (int)nb, d_total, start,
-                             table);
+            CAM_LAUNCH_NAMED(ctx, "assign_starts", brick_starts_kernel, blocks, 256, 0, counts, (int)nb, d_total, start,
+                             table, g.cstride);
         }
         // the fullest brick, for the slabs of later deferred jobs
         if (!ctx->sync_free) {
@@ -658,12 +1252,13 @@ static void assign_impl(cam_ctx *ctx, const float *x, const float *y, const floa
     } else {
         // Payload size and diagnostics back to the host (one synchronisation),
         // with the fullest brick's record count for later slabs.
-        unsigned long long hstats[6] = {0, 0, 0, 0, 0, 0};
+        unsigned long long hstats[8] = {};
         CAM_CUDA_TRY(cudaMemcpyAsync(hstats, stats, sizeof(hstats), cudaMemcpyDeviceToHost, ctx->stream));
         CAM_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
         total = (uint32_t)(hstats[2] & 0xffffffffu);
         ctx->asg_cap = std::max<uint64_t>(ctx->asg_cap, total);  // deferred runs size from it
         out.brick_max = hstats[5] & 0xffffffffu;
+        out.super_max = hstats[6] & 0xffffffffu;
         const unsigned int wmax_bits = (unsigned int)(hstats[1] & 0xffffffffu);
         CAM_REQUIRE(!w || wmax_bits < 0x7f800000u, CAM_E_NONFINITE, "a particle weight is NaN or infinite");
         out.n_lost = (int64_t)hstats[0];
@@ -671,25 +1266,19 @@ static void assign_impl(cam_ctx *ctx, const float *x, const float *y, const floa
     }
 
     uint4 *payload = static_cast<uint4 *>(scratch(ctx, "asg.payload", std::max<size_t>(total, 1) * sizeof(uint4)));
-    if (nb <= kStageBricks) {
-        // Tiles as large as the stage holds with the expected records (15%
-        // margin on the extra ones), split evenly over the SMs.
-        const int recs = (int)std::min<size_t>(16384, (kStageSmem - 16 - (size_t)nb * 4) / 22);
-        const double room = (double)recs / (1.0 + 1.15 * (f - 1.0));
-        const int64_t most = std::max<int64_t>(1024, std::min<int64_t>(kStageTile, (int64_t)room));
-        const int64_t rounds = std::max<int64_t>(1, (np + kNumSMs * most - 1) / (kNumSMs * most));
-        const int64_t even = (np + kNumSMs * rounds - 1) / (kNumSMs * rounds);
-        const int tile = (int)std::min<int64_t>(most, std::max<int64_t>(1024, (even + 31) & ~(int64_t)31));
-        const int64_t tiles = (np + tile - 1) / tile;
-        const unsigned grid_s = (unsigned)std::max<int64_t>(1, std::min<int64_t>(kNumSMs, tiles));
-        const size_t ssmem = stage_bytes(recs, (int)nb);
-        auto k = slab ? staged_kernel<SCHEME, true> : staged_kernel<SCHEME, false>;
+    A.payload = payload;
+    A.cap = total;
+    if (staged) {
+        const int level = two ? 2 : 0;
+        const unsigned grid = tile_for(level, two ? local_bins : (int)nb, f);
+        const size_t ssmem = sort_bytes(level);
+        auto k = two ? (slab ? sort_kernel<SCHEME, true, 2> : sort_kernel<SCHEME, false, 2>)
+                     : (slab ? sort_kernel<SCHEME, true, 0> : sort_kernel<SCHEME, false, 0>);
         smem_at_least(k, ssmem);
-        CAM_LAUNCH_NAMED(ctx, "assign_bin_scatter", k, grid_s, kStageThreads, ssmem, x, y, z, w, np, tile, recs, g,
-                         (int)nb, table, payload, d_lost, d_wmax, total, d_ovf, slab);
+        CAM_LAUNCH_NAMED(ctx, "assign_bin_scatter", k, grid, stage_threads(level), ssmem, A, g, sg);
     } else {
         const int G2 = (int)std::max<int64_t>(1, std::min<int64_t>(2 * kNumSMs, (np + 4095) / 4096));
-        const int64_t chunk2 = std::max<int64_t>(1, (np + G2 - 1) / G2);
+        const unsigned chunk2 = (unsigned)std::max<int64_t>(1, (np + G2 - 1) / G2);
         auto k = slab ? append_kernel<SCHEME, true> : append_kernel<SCHEME, false>;
         CAM_LAUNCH_NAMED(ctx, "assign_bin_scatter", k, G2, kScatterThreads, 0, x, y, z, w, np, chunk2, g, table, payload,
                          d_lost, d_wmax, total, d_ovf, slab);

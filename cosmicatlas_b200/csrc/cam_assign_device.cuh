@@ -16,10 +16,12 @@
 namespace cam {
 namespace asg {
 
-// Global per-brick counters and append cursors sit one per 128-byte line:
-// atomics on one line are serialised in its L2 slice, so packed counters
-// would funnel all bricks through a few slices.
-constexpr int kCursorStride = 32;
+// Global per-brick counters and append cursors: packed where a tile's bricks
+// are advanced together (the lanes of a warp then share a request; 32 words
+// apart the staged scatter of 16.8 M CIC particles onto 256^3 takes 330 us
+// instead of 285), one per 128-byte line where every record takes its own
+// atomic (append_kernel): those on one line are serialised in its L2 slice.
+constexpr int kPaddedStride = 32;
 
 // Reference FP32 home cell (see orc_keys / ref_home in the oracle).
 // NGP: x on [min, min+L); CIC: x - d/2 wrapped once by +-L then [min, min+L);
@@ -61,12 +63,6 @@ __device__ __forceinline__ bool home_cell(const float p[3], const AssignGeom &g,
     return true;
 }
 
-// cell / b for the brick extent b (exact for cell < 2^21, b <= 2^11).
-__device__ __forceinline__ int brick_of(int cell, int b, unsigned magic)
-{
-    return b == 1 ? cell : (int)__umulhi((unsigned)cell, magic);
-}
-
 // Cell centre (in cells) nearest to the position u = (x - min) / d: c + 1/2 of
 // the home cell c or its periodic image.
 __device__ __forceinline__ float nearest_centre(float u, float ci, float nf)
@@ -77,19 +73,17 @@ __device__ __forceinline__ float nearest_centre(float u, float ci, float nf)
     return ci;
 }
 
-// Exact offset t = (x - min)/d - ci in cells, in FP32 with error-free
-// transformations: TwoSum for x - min (nothing to do for min = 0) and a
-// fused multiply-add for the subtraction of ci d (the product is exact
-// inside the FMA); the residual (|r| <= 1.5 d) is scaled by 1/d.
-// |error| <= ~2e-7 cells.
-__device__ __forceinline__ float exact_offset(float x, float mn, float d, float inv_d, float ci, bool origin)
+// Exact residual (x - min) - ci d, in FP32 with error-free transformations:
+// TwoSum for x - min (nothing to do for min = 0) and a fused multiply-add
+// for the subtraction of ci d (the product is exact inside the FMA).  The
+// offset is the residual (|r| <= 1.5 d) times 1/d: |error| <= ~2e-7 cells.
+__device__ __forceinline__ float exact_residual(float x, float mn, float d, float ci, bool origin)
 {
-    if (!origin) return __fmaf_rn(-ci, d, x) * inv_d;
+    if (!origin) return __fmaf_rn(-ci, d, x);
     const float hi = __fsub_rn(x, mn);
     const float bb = __fsub_rn(hi, x);
     const float lo = __fadd_rn(__fsub_rn(x, __fsub_rn(hi, bb)), __fsub_rn(-mn, bb));
-    const float r = __fadd_rn(__fmaf_rn(-ci, d, hi), lo);
-    return r * inv_d;
+    return __fadd_rn(__fmaf_rn(-ci, d, hi), lo);
 }
 
 template <int SCHEME>
@@ -98,47 +92,101 @@ struct Stencil {
     static constexpr int FIRST = SCHEME == CAM_TSC ? -1 : 0;
 };
 
-// Home cell c[] of a particle as home_cell gives it (false: lost) and, with
-// OFFSETS, its exact offsets t[] from the cell centre.  The common case --
-// every quotient well inside [0, n) and away from an integer -- takes the
-// floor by one addition of 2^23 rounded down (the float then holds the
-// integer in its low bits); any other particle goes through home_cell.
-template <int SCHEME, bool OFFSETS>
-__device__ __forceinline__ bool locate(const float p[3], const AssignGeom &g, int c[3], float t[3])
+// Payload word per axis: bits 26..31 = home cell relative to the brick + 8,
+// bits 0..25 = round(t * 2^24) + 2^24 (t in [-1, 3)), the fixed-point offset.
+__device__ __forceinline__ uint32_t fixed_offset(float t)
 {
-    float ci[3];
-    bool ok = true, rare = false;
+    const int tq = __float2int_rn(t * 16777216.0f) + 16777216;
+    return (uint32_t)min(max(tq, 0), (1 << 26) - 1);
+}
+__device__ __forceinline__ uint32_t pack_axis(int cl, uint32_t off) { return ((uint32_t)(cl + 8) << 26) + off; }
+__device__ __forceinline__ void unpack_axis(uint32_t v, int &cl, float &t)
+{
+    cl = (int)(v >> 26) - 8;
+    t = (float)((int)(v & 0x3FFFFFFu) - 16777216) * (1.0f / 16777216.0f);
+}
+
+// Home cell c[] and fixed-point offsets off[] of any particle (false: lost).
+// Out of line: few particles take it (see locate).
+struct Located {
+    int c[3];
+    uint32_t off[3];
+    bool ok;
+};
+template <int SCHEME>
+__device__ __noinline__ Located locate_general(const AssignGeom &g, float px, float py, float pz)
+{
+    const float p[3] = {px, py, pz};
+    Located r;
+    r.ok = home_cell<SCHEME>(p, g, r.c);
+    for (int a = 0; a < 3; ++a) {
+        float t = 0.0f;
+        if (SCHEME != CAM_NGP && r.ok) {
+            const float ci = nearest_centre(__fsub_rn(p[a], g.mn[a]) * g.inv_d[a], (float)r.c[a] + 0.5f, g.nf[a]);
+            t = exact_residual(p[a], g.mn[a], g.d[a], ci, true) * g.inv_d[a];
+        }
+        r.off[a] = fixed_offset(t);
+    }
+    return r;
+}
+
+// Home cell c[] of a particle as home_cell gives it (false: lost) and, with
+// OFFSETS, its fixed-point offsets off[] from the cell centre.  The common
+// case (see AssignGeom::safe) takes the floor by one addition of 3 2^22
+// rounded down -- the float then holds the integer in its low bits -- and
+// needs no test against the box: a particle outside it has a quotient outside
+// [0, n).  A CIC particle in the first half cell has its home cell at -1, the
+// periodic image of n - 1; with an origin the reference wraps positions below
+// zero instead, whatever the origin, and so does this.  |offset| < 1.1, so it
+// needs no clamp.
+template <int SCHEME, bool OFFSETS>
+__device__ __forceinline__ bool locate(float px, float py, float pz, const AssignGeom &g, int c[3], uint32_t off[3])
+{
+    constexpr int LOW = SCHEME == CAM_CIC ? 1 : 0;
+    const float p[3] = {px, py, pz};
+    float ci[3], image[3];
+    bool rare = false;
+    const bool origin = g.origin != 0;
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
-        float v = p[a];
-        if (SCHEME == CAM_CIC) {
-            v = __fsub_rn(v, __fmul_rn(0.5f, g.d[a]));
-            if (v < 0.0f) v = __fadd_rn(v, g.L[a]);
-            if (v >= g.L[a]) v = __fsub_rn(v, g.L[a]);
+        float v = SCHEME == CAM_CIC ? __fsub_rn(p[a], g.half_d[a]) : p[a];
+        image[a] = 0.0f;
+        if (SCHEME == CAM_CIC && origin) {
+            if (v < 0.0f) {
+                v = __fadd_rn(v, g.L[a]);
+                image[a] = -g.nf[a];
+            }
+            if (v >= g.L[a]) {
+                v = __fsub_rn(v, g.L[a]);
+                image[a] += g.nf[a];
+            }
         }
-        const float hi = __fadd_rn(g.mn[a], g.L[a]);
-        ok = ok && (SCHEME == CAM_TSC ? (v >= g.mn[a] && v <= hi) : (v >= g.mn[a] && v < hi));
         const float u = __fmul_rn(__fsub_rn(v, g.mn[a]), g.inv_d[a]);
-        const float f = __fadd_rd(u, 8388608.0f);
-        const float fl = f - 8388608.0f;
-        c[a] = __float_as_int(f) - 0x4b000000;
-        ci[a] = fl + 0.5f;
-        rare = rare || !(fabsf(u - ci[a]) < g.safe[a]) || !(u < g.nf[a]);
+        const float f = __fadd_rd(u, 12582912.0f);
+        const int k = __float_as_int(f) - (0x4b400000 - LOW);  // home cell, + 1 for CIC
+        ci[a] = (f - 12582912.0f) + 0.5f;
+        rare = rare || !(fabsf(u - ci[a]) < g.safe[a]) || (unsigned)k >= (unsigned)(g.n[a] + LOW);
+        if (SCHEME == CAM_CIC && origin) rare = rare || k == 0;
+        c[a] = SCHEME == CAM_CIC ? (k == 0 ? g.n[a] - 1 : k - 1) : k;
     }
-    if (!ok) return false;
     if (rare) {
-        home_cell<SCHEME>(p, g, c);
-#pragma unroll
-        for (int a = 0; a < 3; ++a) ci[a] = (float)c[a] + 0.5f;
-    }
-    if (OFFSETS && SCHEME != CAM_NGP) {
+        const Located r = locate_general<SCHEME>(g, px, py, pz);
 #pragma unroll
         for (int a = 0; a < 3; ++a) {
-            // TSC: only a quotient that rounded up to n has its home cell
-            // wrapped; CIC: the half-cell shift can wrap any particle
-            if (SCHEME == CAM_CIC || rare)
-                ci[a] = nearest_centre(__fsub_rn(p[a], g.mn[a]) * g.inv_d[a], ci[a], g.nf[a]);
-            t[a] = exact_offset(p[a], g.mn[a], g.d[a], g.inv_d[a], ci[a], g.origin != 0);
+            c[a] = r.c[a];
+            off[a] = r.off[a];
+        }
+        return r.ok;
+    }
+    if (OFFSETS) {
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            if (SCHEME == CAM_NGP) {
+                off[a] = 1u << 24;
+                continue;
+            }
+            const float r = exact_residual(p[a], g.mn[a], g.d[a], ci[a] + image[a], origin);
+            off[a] = (uint32_t)(__float2int_rn(r * g.off_scale[a]) + 16777216);
         }
     }
     return true;
@@ -146,23 +194,16 @@ __device__ __forceinline__ bool locate(const float p[3], const AssignGeom &g, in
 
 // The brick of a particle's first stencil cell along axis a: its coordinate
 // bl, the home cell relative to it (cl in [0, e], e its extent), and whether
-// the stencil reaches into the next brick (periodic; never along an axis
-// that one brick spans).
+// the stencil reaches into the next brick (periodic).
 template <int SCHEME>
 __device__ __forceinline__ bool brick_axis(const AssignGeom &g, int a, int c, int &bl, int &cl)
 {
-    if (g.nb[a] == 1) {
-        bl = 0;
-        cl = c;
-        return false;
-    }
-    int lo = c;
-    if (SCHEME == CAM_TSC) lo = c == 0 ? g.n[a] - 1 : c - 1;
-    bl = brick_of(lo, g.b[a], g.bmagic[a]);
-    cl = lo - bl * g.b[a] + (SCHEME == CAM_TSC ? 1 : 0);
+    const int lo = SCHEME == CAM_TSC ? (c == 0 ? g.lo0[a] : c - 1) : c;
+    bl = (int)__umulhi((unsigned)lo, g.bmagic[a]);
+    const int in = lo - bl * g.b[a];
+    cl = SCHEME == CAM_TSC ? in + 1 : in;
     if (SCHEME == CAM_NGP) return false;
-    const int e = bl == g.nb[a] - 1 ? g.e_last[a] : g.b[a];
-    return cl + 1 >= e;
+    return in >= g.cross_b[a] || lo >= g.cross_n[a];
 }
 
 // Step of the brick number to the next brick along each axis (periodic).
@@ -172,20 +213,6 @@ __device__ __forceinline__ void key_steps(const AssignGeom &g, const int bl[3], 
     step[0] = (bl[0] + 1 == g.nb[0] ? -bl[0] : 1) * s0;
     step[1] = (bl[1] + 1 == g.nb[1] ? -bl[1] : 1) * s1;
     step[2] = bl[2] + 1 == g.nb[2] ? -bl[2] : 1;
-}
-
-// Payload word per axis: bits 26..31 = home cell relative to the brick + 8,
-// bits 0..25 = round(t * 2^24) + 2^24 (t in [-1, 3)).
-__device__ __forceinline__ uint32_t pack_axis(int cl, float t)
-{
-    int tq = __float2int_rn(t * 16777216.0f) + 16777216;
-    tq = min(max(tq, 0), (1 << 26) - 1);
-    return ((uint32_t)(cl + 8) << 26) | (uint32_t)tq;
-}
-__device__ __forceinline__ void unpack_axis(uint32_t v, int &cl, float &t)
-{
-    cl = (int)(v >> 26) - 8;
-    t = (float)((int)(v & 0x3FFFFFFu) - 16777216) * (1.0f / 16777216.0f);
 }
 
 // A record as the next brick along the axes of mask m sees it: the home
@@ -199,43 +226,55 @@ __device__ __forceinline__ uint4 next_brick_record(const AssignGeom &g, uint4 r,
     return r;
 }
 
-// The weight statistics of one particle (wstat of fixed_scale).
-__device__ __forceinline__ void weight_stats(float wt, unsigned int &wmax, unsigned int &neg, unsigned int &wminc)
-{
-    wmax = max(wmax, __float_as_uint(fabsf(wt)));
-    neg |= wt < 0.0f;
-    if (wt != 0.0f) wminc = max(wminc, 0x7fffffffu - __float_as_uint(fabsf(wt)));
-}
+// Weight statistics of a thread's particles: largest |w| (bits), smallest
+// w, and smallest nonzero |w| as bits - 1 (a zero weight wraps to the
+// largest value).
+struct WeightStats {
+    unsigned wmax = 0u, wmin1 = 0xffffffffu;
+    float low = 0.0f;
+    __device__ __forceinline__ void add(float w)
+    {
+        const unsigned b = __float_as_uint(w) & 0x7fffffffu;
+        wmax = max(wmax, b);
+        wmin1 = min(wmin1, b - 1u);
+        low = fminf(low, w);
+    }
+    // the words of wstat (fixed_scale): some weight is negative; 0x7fffffff
+    // minus the bits of the smallest nonzero |w| (0: every weight is zero)
+    __device__ __forceinline__ unsigned neg() const { return low < 0.0f ? 1u : 0u; }
+    __device__ __forceinline__ unsigned wminc() const { return wmin1 == 0xffffffffu ? 0u : 0x7fffffffu - (wmin1 + 1u); }
+};
 
 // One particle of the count pass: the bricks its stencil touches (the brick
 // of its first stencil cell and, along each axis whose stencil crosses a
 // brick face, the next brick, periodically) each get one count.
 template <int SCHEME, bool SMEM>
 __device__ __forceinline__ void count_one(float px, float py, float pz, float wt, bool weighted, const AssignGeom &g,
-                                          uint32_t *hist, uint32_t *__restrict__ table, unsigned long long &my_lost,
-                                          unsigned int &my_wmax, unsigned int &my_neg, unsigned int &my_wminc)
+                                          uint32_t *hist, uint32_t *__restrict__ table, unsigned int &my_lost,
+                                          WeightStats &ws)
 {
-    const float pos[3] = {px, py, pz};
     int c[3], bl[3], cl, step[3];
-    float t[3];
-    if (!locate<SCHEME, false>(pos, g, c, t)) {
+    uint32_t off[3];
+    if (!locate<SCHEME, false>(px, py, pz, g, c, off)) {
         ++my_lost;
         return;
     }
-    if (weighted) weight_stats(wt, my_wmax, my_neg, my_wminc);
+    if (weighted) ws.add(wt);
     unsigned cross = 0;
 #pragma unroll
     for (int a = 0; a < 3; ++a) cross |= brick_axis<SCHEME>(g, a, c[a], bl[a], cl) ? 1u << a : 0u;
     const int key = (bl[0] * g.nb[1] + bl[1]) * g.nb[2] + bl[2];
     auto add = [&](int k) {
         if (SMEM) atomicAdd(hist + k, 1u);
-        else atomicAdd(table + (int64_t)k * kCursorStride, 1u);
+        else atomicAdd(table + (int64_t)k * g.cstride, 1u);
     };
     add(key);
     if (SCHEME == CAM_NGP || cross == 0u) return;
     key_steps(g, bl, step);
-    for (unsigned m = cross; m; m = (m - 1u) & cross)
-        add(key + (m & 1u ? step[0] : 0) + (m & 2u ? step[1] : 0) + (m & 4u ? step[2] : 0));
+    // unrolled: some lane of nearly every warp takes most of the seven
+#pragma unroll
+    for (unsigned m = 1; m < 8; ++m)
+        if ((cross & m) == m) add(key + (m & 1u ? step[0] : 0) + (m & 2u ? step[1] : 0) + (m & 4u ? step[2] : 0));
 }
 
 // Writes one record at `slot` of brick `key`: slab > 0, its own slab of
@@ -252,34 +291,33 @@ __device__ __forceinline__ void put_record(uint4 *__restrict__ payload, uint4 re
 }
 
 // One particle appended record by record: every touched brick's cursor
-// (cursor[key * CSTRIDE]) gives the next slot.
-template <int SCHEME, int CSTRIDE>
-__device__ __forceinline__ void append_one(float px, float py, float pz, float wt, const AssignGeom &g,
+// (cursor[key * g.cstride]) gives the next slot.  Returns false if it is lost.
+template <int SCHEME>
+__device__ __forceinline__ bool append_one(float px, float py, float pz, float wt, const AssignGeom &g,
                                            uint32_t *__restrict__ cursor, uint4 *__restrict__ payload, uint64_t cap,
-                                           unsigned int *ovf, unsigned long long &my_lost, uint32_t slab)
+                                           unsigned int *ovf, uint32_t slab)
 {
-    const float pos[3] = {px, py, pz};
     int c[3], bl[3], cl[3], step[3];
-    float t[3] = {0.f, 0.f, 0.f};
-    if (!locate<SCHEME, true>(pos, g, c, t)) {
-        ++my_lost;
-        return;
-    }
+    uint32_t off[3];
+    if (!locate<SCHEME, true>(px, py, pz, g, c, off)) return false;
     unsigned cross = 0;
 #pragma unroll
     for (int a = 0; a < 3; ++a) cross |= brick_axis<SCHEME>(g, a, c[a], bl[a], cl[a]) ? 1u << a : 0u;
     const int key = (bl[0] * g.nb[1] + bl[1]) * g.nb[2] + bl[2];
-    const uint32_t slot = atomicAdd(cursor + (int64_t)key * CSTRIDE, 1u);
-    const uint4 rec = make_uint4(pack_axis(cl[0], t[0]), pack_axis(cl[1], t[1]), pack_axis(cl[2], t[2]),
+    const uint32_t slot = atomicAdd(cursor + (int64_t)key * g.cstride, 1u);
+    const uint4 rec = make_uint4(pack_axis(cl[0], off[0]), pack_axis(cl[1], off[1]), pack_axis(cl[2], off[2]),
                                  __float_as_uint(wt));
     put_record(payload, rec, key, slot, slab, cap, ovf);
-    if (SCHEME == CAM_NGP || cross == 0u) return;
+    if (SCHEME == CAM_NGP || cross == 0u) return true;
     key_steps(g, bl, step);
-    for (unsigned m = cross; m; m = (m - 1u) & cross) {
+#pragma unroll
+    for (unsigned m = 1; m < 8; ++m) {
+        if ((cross & m) != m) continue;
         const int k = key + (m & 1u ? step[0] : 0) + (m & 2u ? step[1] : 0) + (m & 4u ? step[2] : 0);
-        const uint32_t sl = atomicAdd(cursor + (int64_t)k * CSTRIDE, 1u);
+        const uint32_t sl = atomicAdd(cursor + (int64_t)k * g.cstride, 1u);
         put_record(payload, next_brick_record(g, rec, bl, m), k, sl, slab, cap, ovf);
     }
+    return true;
 }
 
 // Cell sum q (units of 2^-s) as the output type; sc = 2^-s, so q * sc is

@@ -178,11 +178,12 @@ __device__ void dl_assign(const DlJob &J, const DlScratch &S, uint4 *payload, fl
     }
     __syncthreads();
     const bool weighted = J.w != nullptr;
-    unsigned long long my_lost = 0;
-    unsigned my_wmax = 0, my_neg = 0, my_wminc = 0;
+    unsigned my_lost = 0;
+    WeightStats ws;
     for (int64_t p = tid; p < J.np; p += kDlThreads)
         count_one<SCHEME, true>(J.x[p], J.y[p], J.z[p], weighted ? J.w[p] : 1.0f, weighted, g, sh.hist, nullptr,
-                                my_lost, my_wmax, my_neg, my_wminc);
+                                my_lost, ws);
+    unsigned my_wmax = ws.wmax, my_neg = ws.neg(), my_wminc = ws.wminc();
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) {
         my_lost += __shfl_down_sync(0xffffffffu, my_lost, off);
@@ -191,7 +192,7 @@ __device__ void dl_assign(const DlJob &J, const DlScratch &S, uint4 *payload, fl
         my_wminc = max(my_wminc, __shfl_down_sync(0xffffffffu, my_wminc, off));
     }
     if ((tid & 31) == 0) {
-        if (my_lost) atomicAdd(sh.lost, my_lost);
+        if (my_lost) atomicAdd(sh.lost, (unsigned long long)my_lost);
         if (my_wmax) atomicMax(sh.wstat, my_wmax);
         if (my_neg) atomicOr(sh.wstat + 1, 1u);
         if (my_wminc) atomicMax(sh.wstat + 6, my_wminc);
@@ -204,10 +205,9 @@ __device__ void dl_assign(const DlJob &J, const DlScratch &S, uint4 *payload, fl
     // append cursors (the counts are not needed any more)
     for (int b = tid; b < nb; b += kDlThreads) sh.hist[b] = sh.start[b];
     __syncthreads();
-    unsigned long long dummy_lost = 0;
     for (int64_t p = tid; p < J.np; p += kDlThreads)
-        append_one<SCHEME, 1>(J.x[p], J.y[p], J.z[p], weighted ? J.w[p] : 1.0f, g, sh.hist, payload, S.pcap, sh.ovf,
-                              dummy_lost, 0u);
+        append_one<SCHEME>(J.x[p], J.y[p], J.z[p], weighted ? J.w[p] : 1.0f, g, sh.hist, payload, S.pcap, sh.ovf,
+                              0u);
     __syncthreads();
     // deposit, brick by brick (the tile of deposit_kernel)
     uint32_t *tile = reinterpret_cast<uint32_t *>(sh.big);

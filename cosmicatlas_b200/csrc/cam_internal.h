@@ -100,7 +100,8 @@ struct cam_ctx {
     // slabs_off: always the exact path (the server's contexts, whose
     // admission budgets the exact payload); so does a context with an HBM
     // budget.
-    std::map<int64_t, double> slab_clump;
+    // super_clump: the same for the super-bricks of two-level sorts.
+    std::map<int64_t, double> slab_clump, super_clump;
     bool slabs_off = false;
     unsigned char *job_pin = nullptr;  // pinned readback buffer of cam_job_run
     size_t job_pin_bytes = 0;
@@ -183,13 +184,22 @@ struct AssignGeom {
     float inv_d[3];      // 1/d rounded (offsets only; keys divide exactly)
     int b[3];            // brick extent (cells)
     int nb[3];           // bricks per axis
-    unsigned bmagic[3];  // ceil(2^32 / b): cell / b = umulhi(cell, bmagic)
+    unsigned bmagic[3];  // ceil(2^32 / b): cell / b = umulhi(cell, bmagic); 0 along an axis one brick spans
     int e_last[3];       // extent of the last brick
-    unsigned kmagic[2];  // ceil(2^32 / nb[2]), ceil(2^32 / nb[1]) (0 for 1): brick number -> coordinates
+    int lo0[3];          // first cell of the TSC stencil of home cell 0: n - 1, or -1 along an axis one brick spans
+    int cross_b[3];      // a stencil whose first cell is cross_b (or more) cells into its brick, or is cross_n or
+    int cross_n[3];      // a later cell, reaches into the next brick (never along an axis one brick spans)
+    unsigned kmagic[2];  // ceil(2^32 / nb[2]), ceil(2^32 / nb[1]): brick number -> coordinates
+    // The common case of locate(): a quotient u = (x - min) * inv_d in [0, n)
+    // at less than `safe` from the middle of its cell has the floor of the
+    // IEEE quotient and is inside the box.  Negative: no such case (a mesh
+    // whose n * d is not L, or with fewer than 4 cells along an axis).
+    float safe[3];
     float nf[3];         // (float)n
-    float safe[3];       // a quotient (x - min) * inv_d in [0, n) whose fraction lies within `safe` of 1/2
-                         // has the floor of the IEEE quotient
+    float half_d[3];     // d / 2 rounded
+    float off_scale[3];  // inv_d * 2^24
     int origin;          // some min is not zero
+    int cstride;         // words between the cursors of consecutive bricks
 };
 
 struct AssignOut {
@@ -208,6 +218,9 @@ struct AssignOut {
     double brick_est = 0.0;
     uint64_t brick_max = 0;
     int64_t brick_shape = 0;  // slab_clump key of the mesh
+    // The same for super-bricks (two-level sorts; word [6] with defer).
+    double super_est = 0.0;
+    uint64_t super_max = 0;
 };
 
 // Records per brick (noise included) that hold the fullest brick of a
@@ -230,7 +243,8 @@ inline double slab_clump_of(uint64_t m, double est)
 // Device statistics of the last assignment of a context (asg.stats):
 // [0] lost particles, [1] low word: bits of max |w|, [2] low word: payload
 // records, [3] low word: nonzero if the deferred payload overflowed,
-// [5] low word: records of the fullest brick (exact runs; 0 with slabs).
+// [5] low word: records of the fullest brick (exact runs; 0 with slabs),
+// [6] low word: particles of the fullest super-brick (exact two-level runs).
 unsigned long long *assign_stats(cam_ctx *ctx);
 
 // Runs the assignment pipeline on device particle arrays.  Writes the mesh

@@ -301,3 +301,57 @@ def test_deposit_tile_edges(ctx, scheme, signed, n):
     assert r.n_lost == lost
     unit = 1.0 if w is None else float(np.mean(np.abs(w)))
     assert rel_err_cells(r.mesh, ref, unit) <= 1e-5
+
+
+@pytest.mark.parametrize("n,box,mn", [(33, 777.7, 0.0), (400, 1000.0, 0.0), (100, 313.1, -40.0), (96, 250.0, 17.5)])
+def test_cells_next_to_every_face(ctx, n, box, mn):
+    # positions within three float steps of every cell face: the common-case
+    # floor, the exact quotient beside faces and the periodic images must give
+    # the oracle's keys (NGP counts) and meshes
+    f = np.float32
+    d = f(f(box) / f(n))
+    face = (np.arange(n + 1, dtype=np.float64) * float(d) + mn).astype(f)
+    steps = [face]
+    for toward in (f(-np.inf), f(np.inf)):
+        v = face
+        for _ in range(3):
+            v = np.nextafter(v, toward)
+            steps.append(v)
+    x = np.concatenate(steps + [(face + f(0.5) * d).astype(f), (face + f(0.25) * d).astype(f)])
+    rng = np.random.default_rng(n)
+    y, z = (rng.permutation(x) for _ in range(2))
+    g = make_grid(n, box, None, mn)
+    og = orc.Grid((n,) * 3, (box,) * 3, tuple(g.d), (mn,) * 3)
+    r = ctx.count_ngp(x, y, z, g)
+    k = orc.keys(NGP, x, y, z, og)
+    assert np.array_equal(r.mesh.reshape(-1), np.bincount(k[k < n ** 3], minlength=n ** 3).astype(np.uint32))
+    for s in (CIC, TSC):
+        a = ctx.assign(x, y, z, None, g, s, F64)
+        ref, lost = orc.assign_f64(s, x, y, z, None, og)
+        assert a.n_lost == lost
+        assert rel_err_cells(a.mesh, ref, 1.0) <= 1e-5
+
+
+@pytest.mark.parametrize("scheme", SCHEMES)
+@pytest.mark.parametrize("weighted", [False, True])
+def test_two_level_sort_vs_oracle(ctx, scheme, weighted):
+    # 384 x 320 x 400 cells are more bricks than one tile counts, and 1.2 M
+    # particles enough for the two-level sort: clumps, cell and box faces,
+    # particles outside the box (their own bin) and NaN positions
+    n, L = (384, 320, 400), (960.0, 800.0, 1000.0)
+    npart = 1_200_007
+    rng = np.random.default_rng(50 + scheme)
+    xs = [rng.uniform(-0.02 * s, 1.02 * s, npart).astype(np.float32) for s in L]
+    xs[0][: npart // 2] = (xs[0][: npart // 2] * 0.1).astype(np.float32)  # a dense slab
+    for a in range(3):
+        e = edge_positions(L[a], n[a])
+        xs[a][a * 20:a * 20 + len(e)] = e
+    w = synth.halo_masses(npart, seed=51) if weighted else None
+    g = make_grid(n, L)
+    r = ctx.assign(*xs, w, g, scheme, F32)
+    ref, lost = orc.assign_f64_mt(scheme, *xs, w, orc.Grid(n, L, tuple(g.d), (0.0, 0.0, 0.0)))
+    assert r.n_lost == lost and lost > 0
+    assert rel_err_cells(r.mesh, ref, 1.0 if w is None else float(np.mean(w, dtype=np.float64))) <= 1e-5
+    p = rng.permutation(npart)
+    again = ctx.assign(*(v[p] for v in xs), None if w is None else w[p], g, scheme, F32)
+    assert np.array_equal(r.mesh.view(np.uint32), again.mesh.view(np.uint32))

@@ -192,3 +192,35 @@ def test_job_slabs_measured_overflow_reruns():
     _, lost, opk, _ = oracle_job(cx, uy, uz, w, n, box, TSC, nbins, None, 0.0, F32)
     floor = opk.shot_noise * opk.sum_sn / np.maximum(opk.modes, 1)
     assert pk_rel_err(res[3]["pk"].pk, opk.pk, floor) <= 1e-5
+
+
+@pytest.mark.parametrize("scheme", [NGP, CIC, TSC])
+def test_two_level_slabs_overflow_reruns(scheme):
+    # The slabs of a two-level sort (super-bricks and bricks) at 384^3: exact,
+    # slabs, a catalogue past the slabs (rerun), slabs again; each result
+    # equals a fresh context's exact run bit for bit.
+    n, box, nbins, npart = 384, 1000.0, 96, 1_100_000
+    rng = np.random.default_rng(15)
+    ux, uy, uz = (rng.uniform(0.0, box, npart).astype(np.float32) for _ in range(3))
+    cx = (box * (ux.astype(np.float64) / box) ** 2.0).astype(np.float32)
+    w = synth.halo_masses(npart, seed=16)
+    g = make_grid(n, box)
+    opts = Context.pk_opts(scheme, nbins=nbins)
+    c, f = Context(0), Context(0)
+    try:
+        launches, res = [], []
+        for xs in (ux, ux, cx, cx):
+            l0 = c.kernel_launches
+            res.append(c.job(xs, uy, uz, w, g, scheme, F32, pk=opts))
+            launches.append(c.kernel_launches - l0)
+        fresh = f.job(cx, uy, uz, w, g, scheme, F32, pk=opts)
+    finally:
+        c.close()
+        f.close()
+    assert launches[1] < launches[0] < launches[2]  # slabs; the slab run, then the exact one
+    assert np.array_equal(res[0]["pk"].pk, res[1]["pk"].pk)
+    for r in res[2:]:
+        assert np.array_equal(r["pk"].pk, fresh["pk"].pk)
+        # NGP loses the positions that round to the box side
+        assert r["assign"].n_lost == fresh["assign"].n_lost
+        assert r["assign"].sum_mesh == fresh["assign"].sum_mesh
