@@ -896,19 +896,20 @@ deposit_kernel(const uint4 *__restrict__ payload, const uint32_t *__restrict__ s
                       min(g.b[2], g.n[2] - o[2])};
     const unsigned fold = (g.nb[0] == 1 ? 1u : 0u) | (g.nb[1] == 1 ? 2u : 0u) | (g.nb[2] == 1 ? 4u : 0u);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    zero_tile(tile32, e, threadIdx.x, kDepositThreads);
-    __syncthreads();
-
     // records beyond the payload's capacity nrec were not written (overflow
     // flag); with slabs, the brick's records are the first of its slab (the
     // host keeps every slab index below 2^32)
     const uint32_t beg = slab ? (uint32_t)B * slab : min(start[B], nrec);
     const uint32_t end = slab ? beg + min(slab_count[(int64_t)B * g.cstride], slab) : min(start[B + 1], nrec);
+    RecordStream rec;
+    rec.open(payload, beg, end, warp, kDepositThreads / 32, lane);
     const bool nonneg = !weighted || wstat[1] == 0u;
     const int s = fixed_scale(wstat, weighted, end - beg);
     // 2^s as two exact factors (s may exceed the float exponent range)
     const float f1 = scalbnf(1.0f, s / 2), f2 = scalbnf(1.0f, s - s / 2);
-    deposit_records<SCHEME>(payload, beg, end, e, f1, f2, nonneg, tile32, warp, kDepositThreads / 32, lane);
+    zero_tile(tile32, e, threadIdx.x, kDepositThreads);
+    __syncthreads();
+    deposit_records<SCHEME>(rec, e, f1, f2, nonneg, tile32);
     __syncthreads();
 
     const double sc = ldexp(1.0, -s);

@@ -514,27 +514,48 @@ __device__ __noinline__ void deposit_general(RecordWeights r, float ws, uint32_t
         }
 }
 
-// The payload records [beg, end) of one brick into its tile; whole warps
-// take 32 consecutive records (warp `warp` of nwarp), the next 32 already
-// on their way.  Lanes past the end deposit zeros.  ws = weight * 2^s; the
-// stencil weights are <= 1 and, up to a rounding next to a cell face (CIC),
+// A thread's share of the payload records [beg, end) of one brick: whole
+// warps take 32 consecutive records (warp `warp` of nwarp), two such groups
+// ahead of the one in work; open() starts the first loads, so that they run
+// while the tile is zeroed.  Lanes past the end get a record of weight zero.
+struct RecordStream {
+    const uint4 *payload;
+    uint32_t p, first, end, step;
+    uint4 a, b;
+    __device__ __forceinline__ uint4 load(uint32_t i) const
+    {
+        const uint32_t zero_word = (8u << 26) | (1u << 24);  // home cell 0, offset 0
+        return i < end ? __ldcs(payload + i) : make_uint4(zero_word, zero_word, zero_word, 0u);
+    }
+    __device__ __forceinline__ void open(const uint4 *__restrict__ pay, uint32_t beg, uint32_t end_, int warp, int nwarp,
+                                         int lane)
+    {
+        payload = pay;
+        end = end_;
+        step = 32u * (uint32_t)nwarp;
+        first = beg + 32u * (uint32_t)warp;
+        p = first + (uint32_t)lane;
+        a = load(p);
+        b = load(p + step);
+    }
+};
+
+// Deposits a brick's records into its tile.  ws = weight * 2^s; the stencil
+// weights are <= 1 and, up to a rounding next to a cell face (CIC),
 // non-negative, so |ws| < 2^32 bounds every contribution; a warp with any
 // record that this does not hold for takes the general form (the same
 // integers).
 template <int SCHEME>
-__device__ __forceinline__ void deposit_records(const uint4 *__restrict__ payload, uint32_t beg, uint32_t end,
-                                                const int e[3], float f1, float f2, bool nonneg, uint32_t *tile,
-                                                int warp, int nwarp, int lane)
+__device__ __forceinline__ void deposit_records(RecordStream &r, const int e[3], float f1, float f2, bool nonneg,
+                                                uint32_t *tile)
 {
     const uint32_t tile_addr = (uint32_t)__cvta_generic_to_shared(tile);
-    const uint32_t zero_word = (8u << 26) | (1u << 24);  // home cell 0, offset 0
-    const uint4 none = make_uint4(zero_word, zero_word, zero_word, 0u);
-    const uint32_t step = 32u * (uint32_t)nwarp;
-    uint32_t p = beg + 32u * (uint32_t)warp + (uint32_t)lane;
-    uint4 v = p < end ? payload[p] : none;
-    for (uint32_t left = beg + 32u * (uint32_t)warp; left < end; left += step) {
-        p += step;
-        const uint4 vn = p < end ? payload[p] : none;
+#pragma unroll 1
+    for (uint32_t left = r.first; left < r.end; left += r.step) {
+        const uint4 v = r.a;
+        r.a = r.b;
+        r.b = r.load(r.p + 2u * r.step);
+        r.p += r.step;
         float w0[3] = {1.f, 1.f, 1.f}, w1[3] = {1.f, 1.f, 1.f}, w2[3] = {1.f, 1.f, 1.f};
         const int i0 = axis_base<SCHEME>(v.x, e[0], w0);
         const int i1 = axis_base<SCHEME>(v.y, e[1], w1);
@@ -547,10 +568,9 @@ __device__ __forceinline__ void deposit_records(const uint4 *__restrict__ payloa
         if (__all_sync(0xffffffffu, fast)) {
             add_rows<SCHEME, 0, 0>(tile_addr + 4u * (uint32_t)slot, ws, ws, w0, w1, w2);
         } else {
-            const RecordWeights r = {{{w0[0], w0[1], w0[2]}, {w1[0], w1[1], w1[2]}, {w2[0], w2[1], w2[2]}}};
-            deposit_general<SCHEME>(r, ws, tile + slot);
+            const RecordWeights rw = {{{w0[0], w0[1], w0[2]}, {w1[0], w1[1], w1[2]}, {w2[0], w2[1], w2[2]}}};
+            deposit_general<SCHEME>(rw, ws, tile + slot);
         }
-        v = vn;
     }
 }
 

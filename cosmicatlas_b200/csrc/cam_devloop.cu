@@ -220,12 +220,14 @@ __device__ void dl_assign(const DlJob &J, const DlScratch &S, uint4 *payload, fl
         const int B0 = B / (g.nb[2] * g.nb[1]);
         const int o[3] = {B0 * g.b[0], B1 * g.b[1], B2 * g.b[2]};
         const int e[3] = {min(g.b[0], g.n[0] - o[0]), min(g.b[1], g.n[1] - o[1]), min(g.b[2], g.n[2] - o[2])};
+        const uint32_t beg = sh.start[B], end = sh.start[B + 1];
+        RecordStream rec;
+        rec.open(payload, beg, end, tid >> 5, kDlWarps, tid & 31);
         zero_tile(tile, e, tid, kDlThreads);
         __syncthreads();
-        const uint32_t beg = sh.start[B], end = sh.start[B + 1];
         const int s = fixed_scale(sh.wstat, weighted ? 1 : 0, end - beg);
         const float f1 = scalbnf(1.0f, s / 2), f2 = scalbnf(1.0f, s - s / 2);
-        deposit_records<SCHEME>(payload, beg, end, e, f1, f2, nonneg, tile, tid >> 5, kDlWarps, tid & 31);
+        deposit_records<SCHEME>(rec, e, f1, f2, nonneg, tile);
         __syncthreads();
         const double sc = ldexp(1.0, -s);
         long long acc = store_tile<float>(tile, o, e, g.n, fold, s, sc, mesh, tid >> 5, kDlWarps, tid & 31);

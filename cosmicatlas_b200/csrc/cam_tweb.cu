@@ -887,6 +887,9 @@ void tweb_impl(cam_ctx *ctx, FftPlan *plan, const Spectrum &dk, float L, const d
                          (int)n);
         sf = t;
     }
+    // The Nyquist planes' x and y passes (a few CTAs each: 13 + 21 us at 64^3,
+    // 19 + 33 at 256^3) run on the side stream beside the main planes' ones.
+    const cudaStream_t side_stream = aux_fork(ctx);
     auto passes = [&](auto fdc) {
     constexpr bool FD = decltype(fdc)::value;
     // 1. x: k_x^p phi + inverse FFT along x, p = 0, 1, 2 (slots 0..2).
@@ -906,6 +909,7 @@ void tweb_impl(cam_ctx *ctx, FftPlan *plan, const Spectrum &dk, float L, const d
                              (int)M, n * M, (int64_t)M, ccomp, rn, tw, gcoef, d_mean, density, scale, sf, pot);
         }
         dim3 g1(3, (unsigned)((n + W - 1) / W), 1);
+        StreamScope side(ctx, side_stream);
         CAM_LAUNCH_NAMED(ctx, "tweb_tidal_x_nyq", k1, g1, nthr, smem, static_cast<const C *>(dk.nyq), cn, (int)n, (int)n, n,
                    (int64_t)0, nn, rn, tw, gcoef, d_mean, density, scale, sf, pot);
         });
@@ -927,6 +931,7 @@ void tweb_impl(cam_ctx *ctx, FftPlan *plan, const Spectrum &dk, float L, const d
         }
         // Nyquist plane: columns i (stride N), FFT index j (stride 1)
         dim3 g1(3, (unsigned)((n + W - 1) / W), 1);
+        StreamScope side(ctx, side_stream);
         CAM_LAUNCH_NAMED(ctx, "tweb_tidal_y_nyq", ky, g1, nthr, smem, cn, (int)n, (int)n, (int64_t)1, n, (int64_t)0,
                          nn, rn, tw, (int)M, sf);
         });
@@ -934,6 +939,7 @@ void tweb_impl(cam_ctx *ctx, FftPlan *plan, const Spectrum &dk, float L, const d
     };
     if (sf) passes(std::true_type{});
     else passes(std::false_type{});
+    aux_join(ctx);
     // 3. z: c2r + eigenvalues + labels.
     {
         // Small tiles (<= 4096 complex, 256 threads) so that several CTAs
