@@ -380,11 +380,15 @@ tidal_pipe_kernel(const typename CTw<T>::t *src, typename CTw<T>::t *dst, int n,
 // step on the FP64 characteristic polynomial; returned in descending
 // order.  FP64 throughout because acos is ill-conditioned next to r = +-1
 // (two equal eigenvalues): an error e in r moves phi by ~sqrt(2e), which
-// for FP32 (e ~ 6e-8) is ~3e-4 of the spread; in FP64 it is ~2e-8.  Only
-// the eigenvalue planes take this path; labels alone use the sign count.
-__device__ __forceinline__ void eig3(float a00f, float a11f, float a22f, float a01f, float a02f, float a12f,
-                                     double lam[3])
+// for FP32 (e ~ 6e-8) is ~3e-4 of the spread; in FP64 it is ~2e-8.  Out of
+// line: only the cells that eig3 leaves take it.
+struct Eigen3 {
+    double l[3];
+};
+__device__ __noinline__ Eigen3 eig3_general(float a00f, float a11f, float a22f, float a01f, float a02f, float a12f)
 {
+    Eigen3 out;
+    double *lam = out.l;
     const double a00 = a00f, a11 = a11f, a22 = a22f, a01 = a01f, a02 = a02f, a12 = a12f;
     const double p1 = a01 * a01 + a02 * a02 + a12 * a12;
     const double q = (a00 + a11 + a22) * (1.0 / 3.0);
@@ -426,6 +430,56 @@ __device__ __forceinline__ void eig3(float a00f, float a11f, float a22f, float a
     if (lam[0] < lam[1]) { const double t = lam[0]; lam[0] = lam[1]; lam[1] = t; }
     if (lam[1] < lam[2]) { const double t = lam[1]; lam[1] = lam[2]; lam[2] = t; }
     if (lam[0] < lam[1]) { const double t = lam[0]; lam[0] = lam[1]; lam[1] = t; }
+    return out;
+}
+
+// Eigenvalues of a symmetric 3x3 matrix in FP64 from the FP32 entries, in
+// descending order.  With q the mean of the diagonal, the eigenvalues are
+// q + x for the roots x of x^3 - c x - d (c = tr(B^2) / 2, d = det B, B the
+// traceless part).  The root furthest from the other two has the sign of d;
+// as a multiple y of p = sqrt(c / 3) it solves y^3 - 3 y - 2 r = 0 with
+// r = |d| / (2 p^3) in [0, 1], y in [sqrt 3, 2].  Two Newton steps in FP32
+// from the chord sqrt 3 + (2 - sqrt 3) r (error 0.014, then < 2e-4, then the
+// FP32 rounding) start two in FP64 with an FP32 reciprocal of the slope (each
+// gains a factor 1e-7); the other roots are -x/2 +- sqrt(c - 3 x^2 / 4), the
+// root from an FP32 reciprocal root and one FP64 step.  Error ~1e-13 of the
+// spread while r <= 1 - 1e-5; nearer to a double root, or where FP32 would
+// under- or overflow, eig3_general.  About 45 FP64 operations a cell in place
+// of some 350: the eigenvalue z pass at 256^3 was bound by them.
+__device__ __forceinline__ void eig3(float a00f, float a11f, float a22f, float a01f, float a02f, float a12f,
+                                     double lam[3])
+{
+    const double a00 = a00f, a11 = a11f, a22 = a22f, a01 = a01f, a02 = a02f, a12 = a12f;
+    const double q = (a00 + a11 + a22) * (1.0 / 3.0);
+    const double b00 = a00 - q, b11 = a11 - q, b22 = a22 - q;
+    const double c = 0.5 * (b00 * b00 + b11 * b11 + b22 * b22) + (a01 * a01 + a02 * a02 + a12 * a12);
+    const double d = b00 * (b11 * b22 - a12 * a12) - a01 * (a01 * b22 - a12 * a02) + a02 * (a01 * a12 - b11 * a02);
+    const float cf = (float)c;
+    const float p = sqrtf(cf * (1.0f / 3.0f));
+    const float r = fabsf((float)d) / (2.0f * p * p * p);
+    if (!(cf > 1e-22f && cf < 1e22f && r <= 0.99999f)) {
+        const Eigen3 e = eig3_general(a00f, a11f, a22f, a01f, a02f, a12f);
+        lam[0] = e.l[0];
+        lam[1] = e.l[1];
+        lam[2] = e.l[2];
+        return;
+    }
+    float y = 1.7320508f + 0.2679492f * r;
+#pragma unroll
+    for (int k = 0; k < 2; ++k) y -= ((y * y - 3.0f) * y - 2.0f * r) * __frcp_rn(3.0f * y * y - 3.0f);
+    const bool neg = d < 0.0;
+    double x = (double)(neg ? -p * y : p * y);
+    const float slope = __frcp_rn(p * p * (3.0f * y * y - 3.0f));  // 1 / (3 x^2 - c)
+#pragma unroll
+    for (int k = 0; k < 2; ++k) x -= ((x * x - c) * x - d) * (double)slope;
+    const double disc = c - 0.75 * x * x;
+    const float h = rsqrtf((float)disc);
+    double s = disc * (double)h;
+    s += (0.5 * (double)h) * (disc - s * s);
+    const double m = q - 0.5 * x;
+    lam[0] = neg ? m + s : q + x;
+    lam[1] = neg ? m - s : m + s;
+    lam[2] = neg ? q + x : m - s;
 }
 
 // Coefficients of det(x I - A) = x^3 - c2 x^2 + c1 x - c0 in FP64 from the
