@@ -302,7 +302,20 @@ final_sum_kernel(const double *__restrict__ part, int np, double *__restrict__ o
     }
 }
 
+__global__ void __launch_bounds__(256) publish_kernel(const __grid_constant__ Publish p, uint32_t *__restrict__ dst)
+{
+    for (int k = 0; k < p.n; ++k) {
+        const uint32_t *src = static_cast<const uint32_t *>(p.seg[k].src);
+        for (uint32_t i = threadIdx.x; i < p.seg[k].words; i += 256) dst[p.seg[k].at + i] = src[i];
+    }
+}
+
 }  // namespace
+
+void publish(cam_ctx *ctx, const Publish &p, void *pinned_dst)
+{
+    CAM_LAUNCH(ctx, publish_kernel, 1, 256, 0, p, static_cast<uint32_t *>(pinned_dst));
+}
 
 // out[0] = sum, out[1] = sum / divisor (FP64, fixed order).  Up to 2^16
 // values are summed by one CTA directly.
@@ -385,6 +398,65 @@ DevParticles stage_particles(cam_ctx *ctx, const cam_particles *p)
     d.z = stage_in(ctx, "in.z", p->z, p->n, p->mem);
     d.w = p->w ? stage_in(ctx, "in.w", p->w, p->n, p->mem) : nullptr;
     return d;
+}
+
+// The context's pinned readback buffer, at least `bytes`.
+unsigned char *pinned(cam_ctx *ctx, size_t bytes)
+{
+    if (ctx->job_pin_bytes < bytes) {
+        std::lock_guard<std::mutex> lk(alloc_mutex());
+        if (ctx->job_pin) CAM_CUDA_TRY(cudaFreeHost(ctx->job_pin));
+        ctx->job_pin = nullptr;
+        ctx->job_pin_bytes = 0;
+        CAM_CUDA_TRY(cudaHostAlloc(reinterpret_cast<void **>(&ctx->job_pin), bytes, cudaHostAllocDefault));
+        ctx->job_pin_bytes = bytes;
+    }
+    return ctx->job_pin;
+}
+
+// An exact run measured its fullest brick (and super-brick): later deferred
+// runs of this context and mesh shape size their slabs from it.
+void keep_clumps(cam_ctx *ctx, const AssignOut &out, const unsigned long long *hstats)
+{
+    const uint64_t bmax = out.defer ? (hstats[5] & 0xffffffffu) : out.brick_max;
+    const uint64_t smax = out.defer ? (hstats[6] & 0xffffffffu) : out.super_max;
+    if (bmax && out.brick_est > 0.0) ctx->slab_clump[out.brick_shape] = slab_clump_of(bmax, out.brick_est);
+    if (smax && out.super_est > 0.0) ctx->super_clump[out.brick_shape] = slab_clump_of(smax, out.super_est);
+}
+
+// One assignment call: a deferred run (see AssignOut) and, if its slabs or
+// its payload estimate fell short, an exact one; the host waits once in the
+// common case.
+void assign_call(cam_ctx *ctx, const DevParticles &d, const cam_grid &g, int scheme, AssignOut &out, size_t out_bytes,
+                 void *host_out, cam_assign_stats *stats)
+{
+    unsigned char *pin = pinned(ctx, 64 + 16);
+    const auto *hstats = reinterpret_cast<const unsigned long long *>(pin);
+    // a context with a budget, and a catalogue whose records would fill a
+    // quarter of the device, sizes its payload exactly
+    const bool exact = ctx->budget || (uint64_t)d.n * 8 * sizeof(uint4) > ctx->device_bytes / 4;
+    for (int pass = exact ? 1 : 0; pass < 2; ++pass) {
+        out.defer = pass == 0;
+        assign_device(ctx, d.x, d.y, d.z, d.w, d.n, g, scheme, out);
+        Publish p;
+        p.add(assign_stats(ctx), 64, 0);
+        p.add(out.d_sum, 16, 64);
+        publish(ctx, p, pin);
+        CAM_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+        keep_clumps(ctx, out, hstats);
+        if (!(out.defer && (hstats[3] & 0xffffffffu))) break;
+    }
+    CAM_REQUIRE(!d.w || (unsigned)(hstats[1] & 0xffffffffu) < 0x7f800000u, CAM_E_NONFINITE,
+                "a particle weight is NaN or infinite");
+    if (host_out) {
+        CAM_CUDA_TRY(cudaMemcpyAsync(host_out, out.mesh, out_bytes, cudaMemcpyDeviceToHost, ctx->stream));
+        CAM_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+    }
+    if (stats) {
+        stats->n_lost = (int64_t)hstats[0];
+        stats->n_in = d.n - stats->n_lost;
+        stats->sum_mesh = reinterpret_cast<const double *>(pin + 64)[0];
+    }
 }
 
 }  // namespace
@@ -495,7 +567,8 @@ int cam_ctx_create(int device, size_t hbm_budget, cam_ctx **out)
     if (!c) return CAM_E_NOMEM;
     c->device = device;
     c->budget = hbm_budget;
-    if (cudaSetDevice(device) != cudaSuccess ||
+    size_t idle = 0;
+    if (cudaSetDevice(device) != cudaSuccess || cudaMemGetInfo(&idle, &c->device_bytes) != cudaSuccess ||
         cudaStreamCreateWithFlags(&c->own_stream, cudaStreamNonBlocking) != cudaSuccess ||
         cudaStreamCreateWithFlags(&c->aux_stream, cudaStreamNonBlocking) != cudaSuccess ||
         cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming) != cudaSuccess ||
@@ -643,17 +716,7 @@ int cam_assign(cam_ctx *ctx, const cam_particles *parts, const cam_grid *grid, i
         out.precision = precision;
         out.mesh = out_mem == CAM_MEM_DEVICE ? mesh_out : scratch(ctx, "asg.mesh", ncell * esize(precision));
         out.d_sum = static_cast<double *>(scratch(ctx, "asg.sum", 2 * sizeof(double)));
-        assign_device(ctx, d.x, d.y, d.z, d.w, d.n, g, scheme, out);
-        if (out_mem == CAM_MEM_HOST)
-            CAM_CUDA_TRY(cudaMemcpyAsync(mesh_out, out.mesh, ncell * esize(precision), cudaMemcpyDeviceToHost, ctx->stream));
-        double sum = 0.0;
-        CAM_CUDA_TRY(cudaMemcpyAsync(&sum, out.d_sum, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
-        CAM_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
-        if (stats) {
-            stats->n_in = out.n_in;
-            stats->n_lost = out.n_lost;
-            stats->sum_mesh = sum;
-        }
+        assign_call(ctx, d, g, scheme, out, ncell * esize(precision), out_mem == CAM_MEM_HOST ? mesh_out : nullptr, stats);
     });
 }
 
@@ -671,17 +734,7 @@ int cam_count_ngp(cam_ctx *ctx, const cam_particles *parts, const cam_grid *grid
         out.precision = -1;
         out.mesh = out_mem == CAM_MEM_DEVICE ? (void *)counts_out : scratch(ctx, "asg.mesh", ncell * 4);
         out.d_sum = static_cast<double *>(scratch(ctx, "asg.sum", 2 * sizeof(double)));
-        assign_device(ctx, d.x, d.y, d.z, nullptr, d.n, g, CAM_NGP, out);
-        if (out_mem == CAM_MEM_HOST)
-            CAM_CUDA_TRY(cudaMemcpyAsync(counts_out, out.mesh, ncell * 4, cudaMemcpyDeviceToHost, ctx->stream));
-        double sum = 0.0;
-        CAM_CUDA_TRY(cudaMemcpyAsync(&sum, out.d_sum, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
-        CAM_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
-        if (stats) {
-            stats->n_in = out.n_in;
-            stats->n_lost = out.n_lost;
-            stats->sum_mesh = sum;
-        }
+        assign_call(ctx, d, g, CAM_NGP, out, ncell * 4, out_mem == CAM_MEM_HOST ? counts_out : nullptr, stats);
     });
 }
 
@@ -1122,22 +1175,16 @@ int cam_job_run(cam_ctx *ctx, const cam_job_desc *job, cam_job_result *res)
         const DevParticles d = stage_particles(ctx, &job->parts);
         FftPlan *plan = get_plan(ctx, n, job->precision);
         const int nb = want_pk ? nbins_for(job->pk, n) : 0;
-        // Readback of one run: assignment statistics [8], mesh sum and mean
-        // [2], P(k) sums [nb][2] and modes [nb], into a pinned buffer.
-        const size_t pin_bytes = 8 * 8 + 2 * 8 + (size_t)nb * 24 + 8;
-        if (ctx->job_pin_bytes < pin_bytes) {
-            std::lock_guard<std::mutex> lk(alloc_mutex());
-            if (ctx->job_pin) CAM_CUDA_TRY(cudaFreeHost(ctx->job_pin));
-            ctx->job_pin = nullptr;
-            ctx->job_pin_bytes = 0;
-            CAM_CUDA_TRY(cudaHostAlloc(reinterpret_cast<void **>(&ctx->job_pin), pin_bytes, cudaHostAllocDefault));
-            ctx->job_pin_bytes = pin_bytes;
-        }
-        auto *hstats = reinterpret_cast<unsigned long long *>(ctx->job_pin);
-        auto *hsum = reinterpret_cast<double *>(ctx->job_pin + 64);
-        auto *hpk = reinterpret_cast<double *>(ctx->job_pin + 80);
-        auto *hmd = reinterpret_cast<unsigned long long *>(ctx->job_pin + 80 + (size_t)nb * 16);
-        auto *herr = reinterpret_cast<unsigned *>(ctx->job_pin + 80 + (size_t)nb * 24);
+        // Readback of one run into pinned memory: assignment statistics [8],
+        // T-web counters [8], mesh sum and mean [2], the error word, P(k)
+        // sums [nb][2] and modes [nb].
+        constexpr size_t kTw = 64, kSum = 128, kErr = 144, kPk = 160;
+        unsigned char *pin = pinned(ctx, kPk + (size_t)nb * 24);
+        const auto *hstats = reinterpret_cast<const unsigned long long *>(pin);
+        const auto *htw = reinterpret_cast<const unsigned long long *>(pin + kTw);
+        const auto *hsum = reinterpret_cast<const double *>(pin + kSum);
+        const auto *hpk = reinterpret_cast<const double *>(pin + kPk);
+        const auto *hmd = reinterpret_cast<const unsigned long long *>(pin + kPk + (size_t)nb * 16);
         const unsigned *derr = device_error_word(ctx);
         // One run of the whole job.  defer: the assignment sizes its payload
         // from an estimate and nothing waits for the host until the single
@@ -1155,21 +1202,25 @@ int cam_job_run(cam_ctx *ctx, const cam_job_desc *job, cam_job_result *res)
             Spectrum s = alloc_spectrum(ctx, n, job->precision, "job.spec");
             const PkDevice pkd = job_fft_pk(ctx, plan, out.mesh, dsum + 1, s, want_pk ? &job->pk : nullptr, nb,
                                             job->want_tweb != 0);
-            CAM_CUDA_TRY(cudaMemcpyAsync(hstats, assign_stats(ctx), 64, cudaMemcpyDeviceToHost, ctx->stream));
-            CAM_CUDA_TRY(cudaMemcpyAsync(hsum, dsum, 16, cudaMemcpyDeviceToHost, ctx->stream));
-            if (want_pk) {
-                CAM_CUDA_TRY(cudaMemcpyAsync(hpk, pkd.sums, (size_t)nb * 16, cudaMemcpyDeviceToHost, ctx->stream));
-                CAM_CUDA_TRY(cudaMemcpyAsync(hmd, pkd.modes, (size_t)nb * 8, cudaMemcpyDeviceToHost, ctx->stream));
+            uint8_t *dl = nullptr;
+            if (job->want_tweb) {
+                if (res->labels) dl = static_cast<uint8_t *>(scratch(ctx, "tw.labels", ncell));
+                tweb_device(ctx, plan, s, g.L[0], dsum + 1, job->tweb.input_type, job->tweb, dl, nullptr, nullptr, nullptr,
+                            job_tweb_counts(ctx));
             }
-            CAM_CUDA_TRY(cudaMemcpyAsync(herr, derr, sizeof(unsigned), cudaMemcpyDeviceToHost, ctx->stream));
+            Publish p;
+            p.add(assign_stats(ctx), kAssignHead, 0);  // with the T-web's counters
+            p.add(dsum, 16, kSum);
+            p.add(derr, sizeof(unsigned), kErr);
+            if (want_pk) {
+                p.add(pkd.sums, (size_t)nb * 16, kPk);
+                p.add(pkd.modes, (size_t)nb * 8, kPk + (size_t)nb * 16);
+            }
+            publish(ctx, p, pin);
             CAM_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
-            CAM_REQUIRE(*herr == 0u, CAM_E_CUDA, "a kernel's bulk copy did not complete within its wait limit");
-            // An exact run measured its fullest brick: later deferred jobs
-            // of this context and mesh shape size their slabs from it.
-            const uint64_t bmax = defer ? (hstats[5] & 0xffffffffu) : out.brick_max;
-            const uint64_t smax = defer ? (hstats[6] & 0xffffffffu) : out.super_max;
-            if (bmax && out.brick_est > 0.0) ctx->slab_clump[out.brick_shape] = slab_clump_of(bmax, out.brick_est);
-            if (smax && out.super_est > 0.0) ctx->super_clump[out.brick_shape] = slab_clump_of(smax, out.super_est);
+            CAM_REQUIRE(*reinterpret_cast<const unsigned *>(pin + kErr) == 0u, CAM_E_CUDA,
+                        "a kernel's bulk copy did not complete within its wait limit");
+            keep_clumps(ctx, out, hstats);
             // a slab (or the payload estimate) was too small: an exact run,
             // which also measures the bricks again
             if (defer && (hstats[3] & 0xffffffffu)) return true;
@@ -1192,9 +1243,9 @@ int cam_job_run(cam_ctx *ctx, const cam_job_desc *job, cam_job_result *res)
                             res->kvector, &res->pk_info);
             }
             if (job->want_tweb) {
-                uint8_t *dl = res->labels ? static_cast<uint8_t *>(scratch(ctx, "tw.labels", ncell)) : nullptr;
-                cam_tweb_opts to = job->tweb;
-                tweb_device(ctx, plan, s, g.L[0], dsum + 1, to.input_type, to, dl, nullptr, &res->tweb);
+                for (int a = 0; a < 4; ++a) res->tweb.counts[a] = (int64_t)htw[a];
+                res->tweb.ties = (int64_t)htw[4];
+                res->tweb.mean = hsum[1];
                 if (dl) {
                     CAM_CUDA_TRY(cudaMemcpyAsync(res->labels, dl, ncell, cudaMemcpyDeviceToHost, ctx->stream));
                     CAM_CUDA_TRY(cudaStreamSynchronize(ctx->stream));

@@ -1062,7 +1062,8 @@ static void assign_impl(cam_ctx *ctx, const float *x, const float *y, const floa
     // runs of a few per brick.
     const bool plain_ctx = !ctx->sync_free && !ctx->slabs_off && !ctx->budget;
     SuperGeom sg{};
-    if (plain_ctx && nb > kStageBins && np >= kTwoLevelParticles && geom.safe[0] > 0.f && geom.safe[1] > 0.f &&
+    if (plain_ctx && nb > kStageBins && np >= kTwoLevelParticles &&
+        (uint64_t)np * sizeof(float4) <= ctx->device_bytes / 16 && geom.safe[0] > 0.f && geom.safe[1] > 0.f &&
         geom.safe[2] > 0.f)
         // as few super-bricks as LEVEL 2 has bins for: LEVEL 1's runs are the
         // longer (512^3: 128 of them 0.95 ms, 512 of them 1.87, LEVEL 2 alike)
@@ -1074,17 +1075,18 @@ static void assign_impl(cam_ctx *ctx, const float *x, const float *y, const floa
     const bool staged = two || nb <= kStageBins;
     AssignGeom g = geom;
     g.cstride = staged ? 1 : kPaddedStride;
-    // per-brick counters (counts, then cursors)
-    auto *table = static_cast<uint32_t *>(scratch(ctx, "asg.cursor", (size_t)nb * g.cstride * sizeof(uint32_t)));
+    // statistics and per-brick counters (counts, then cursors): one buffer,
+    // zeroed at once
+    const size_t head_bytes = kAssignHead + (size_t)nb * g.cstride * sizeof(uint32_t);
+    auto *stats = static_cast<unsigned long long *>(scratch(ctx, "asg.head", head_bytes));
+    auto *table = reinterpret_cast<uint32_t *>(reinterpret_cast<unsigned char *>(stats) + kAssignHead);
     auto *start = static_cast<uint32_t *>(scratch(ctx, "asg.start", (nb + 1) * sizeof(uint32_t)));
-    auto *stats = static_cast<unsigned long long *>(scratch(ctx, "asg.stats", 64));
     auto *bsum = static_cast<double *>(scratch(ctx, "asg.bsum", nb * sizeof(double)));
     unsigned long long *d_lost = stats;
     unsigned int *d_wmax = reinterpret_cast<unsigned int *>(stats + 1);
     uint32_t *d_total = reinterpret_cast<uint32_t *>(stats + 2);
     unsigned int *d_ovf = reinterpret_cast<unsigned int *>(stats + 3);
-    CAM_CUDA_TRY(cudaMemsetAsync(table, 0, (size_t)nb * g.cstride * sizeof(uint32_t), ctx->stream));
-    CAM_CUDA_TRY(cudaMemsetAsync(stats, 0, 64, ctx->stream));
+    CAM_CUDA_TRY(cudaMemsetAsync(stats, 0, head_bytes, ctx->stream));
 
     // Expected records per particle of a uniform catalogue: a stencil
     // crosses a face of a brick of extent b with probability (W-1)/b per
@@ -1105,7 +1107,8 @@ static void assign_impl(cam_ctx *ctx, const float *x, const float *y, const floa
     // expected records (or 2^20 records), three times with two levels: one
     // level's short runs slow down as the slabs spread them over more memory.
     // A context with an HBM budget keeps the exact path, whose payload the
-    // budget was sized for.
+    // budget was sized for; nor do slabs take more than a quarter of the
+    // device's memory, or sorted particles a sixteenth.
     const double est_brick = (double)np * f / (double)nb;
     const int64_t shape = ((int64_t)g.n[0] << 32) | ((int64_t)g.n[1] << 16) | (int64_t)g.n[2];
     double est_super = (double)np;
@@ -1119,7 +1122,8 @@ static void assign_impl(cam_ctx *ctx, const float *x, const float *y, const floa
         if (it != ctx->slab_clump.end() && (!two || is != ctx->super_clump.end())) {
             const uint64_t cap = slab_capacity(it->second * est_brick);
             const double room = std::max((two ? 3.0 : 2.0) * (double)np * f, (double)(1u << 20));
-            bool fits = (double)nb * (double)cap <= room && (uint64_t)nb * cap < (1ull << 32);
+            bool fits = (double)nb * (double)cap <= room && (uint64_t)nb * cap < (1ull << 32) &&
+                        (uint64_t)nb * cap * sizeof(uint4) <= ctx->device_bytes / 4;
             if (two) {
                 const uint64_t scap = slab_capacity(is->second * est_super);
                 fits = fits && (double)sg.count * (double)scap <= 2.0 * (double)np + (double)(1u << 20) &&
@@ -1232,7 +1236,7 @@ static void assign_impl(cam_ctx *ctx, const float *x, const float *y, const floa
         // No host round trip (stream capture): size the payload for the
         // provable bound, one record per touched brick and at most two
         // bricks per axis.  Lost count and max |w| stay on the device
-        // (asg.stats) for the caller to read back with the results.
+        // for the caller to read back with the results.
         total = (uint64_t)np * per;
         CAM_REQUIRE(total < (1ull << 32), CAM_E_UNSUPPORTED, "payload bound exceeds 2^32 records");
         out.n_lost = -1;
@@ -1305,7 +1309,7 @@ static void assign_impl(cam_ctx *ctx, const float *x, const float *y, const floa
 
 unsigned long long *assign_stats(cam_ctx *ctx)
 {
-    return static_cast<unsigned long long *>(scratch(ctx, "asg.stats", 64));
+    return static_cast<unsigned long long *>(scratch(ctx, "asg.head", kAssignHead));
 }
 
 void assign_device(cam_ctx *ctx, const float *x, const float *y, const float *z,

@@ -75,6 +75,7 @@ struct cam_ctx {
     int device = 0;
     size_t budget = 0;  // 0 = unlimited
     size_t used = 0;
+    size_t device_bytes = 0;  // the device's memory (bounds what assignments spend on speed)
     cudaStream_t own_stream = nullptr;
     cudaStream_t stream = nullptr;
     // Side stream for independent work inside one call (the Nyquist plane
@@ -240,12 +241,34 @@ inline double slab_clump_of(uint64_t m, double est)
     return std::max(1.0, (md - 4.0 * std::sqrt(md)) / est);
 }
 
-// Device statistics of the last assignment of a context (asg.stats):
+// Device statistics of the last assignment of a context:
 // [0] lost particles, [1] low word: bits of max |w|, [2] low word: payload
 // records, [3] low word: nonzero if the deferred payload overflowed,
 // [5] low word: records of the fullest brick (exact runs; 0 with slabs),
 // [6] low word: particles of the fullest super-brick (exact two-level runs).
 unsigned long long *assign_stats(cam_ctx *ctx);
+// Bytes at the start of that buffer that an assignment zeroes besides its
+// cursors: the statistics [8] and eight words for the T-web that follows in a
+// job (its label counters, tweb_device's d_counts).
+constexpr size_t kAssignHead = 128;
+inline unsigned long long *job_tweb_counts(cam_ctx *ctx) { return assign_stats(ctx) + 8; }
+
+// Copies small device results to one place in pinned host memory with one
+// launch (in place of a copy each); the host sees them once the stream has
+// passed it.  bytes are multiples of 4; dst advances by each segment.
+struct Publish {
+    static constexpr int kMax = 6;
+    struct Segment {
+        const void *src;
+        uint32_t words, at;  // 4-byte words; offset in words from dst
+    } seg[kMax];
+    int n = 0;
+    void add(const void *src, size_t bytes, size_t at_bytes)
+    {
+        seg[n++] = Segment{src, (uint32_t)(bytes / 4), (uint32_t)(at_bytes / 4)};
+    }
+};
+void publish(cam_ctx *ctx, const Publish &p, void *pinned_dst);
 
 // Runs the assignment pipeline on device particle arrays.  Writes the mesh
 // and, on the device, the FP64 mesh sum.  Synchronises once (payload size)
@@ -344,10 +367,11 @@ PkDevice job_fft_pk(cam_ctx *ctx, FftPlan *plan, const void *mesh, const double 
 
 // ------------------------------------------------------ T-web
 // d_inv (may be null): 4 planes of N^3 floats, the tidal invariants I, II,
-// III and the anisotropy per cell.
+// III and the anisotropy per cell.  d_counts (may be null): eight zeroed
+// device words for the label and tie counters, in place of its own.
 void tweb_device(cam_ctx *ctx, FftPlan *plan, const Spectrum &dk, float L, const double *d_mean,
                  int input_type, const cam_tweb_opts &o, uint8_t *d_labels, float *d_lambdas,
-                 cam_tweb_stats *stats, float *d_inv = nullptr);
+                 cam_tweb_stats *stats, float *d_inv = nullptr, unsigned long long *d_counts = nullptr);
 
 // PoissonSolver's multiplier -1/k^2 (times exp(-k^2 R^2 / 2) if R > 0) on a
 // split spectrum, in place (cam_fd.cu).

@@ -443,7 +443,7 @@ __device__ __noinline__ Eigen3 eig3_general(float a00f, float a11f, float a22f, 
 // FP32 rounding) start two in FP64 with an FP32 reciprocal of the slope (each
 // gains a factor 1e-7); the other roots are -x/2 +- sqrt(c - 3 x^2 / 4), the
 // root from an FP32 reciprocal root and one FP64 step.  Error ~1e-13 of the
-// spread while r <= 1 - 1e-5; nearer to a double root, or where FP32 would
+// spread up to r = 1 - 2e-7 (the cancellation in the root there); nearer to a double root, or where FP32 would
 // under- or overflow, eig3_general.  About 45 FP64 operations a cell in place
 // of some 350: the eigenvalue z pass at 256^3 was bound by them.
 __device__ __forceinline__ void eig3(float a00f, float a11f, float a22f, float a01f, float a02f, float a12f,
@@ -457,7 +457,7 @@ __device__ __forceinline__ void eig3(float a00f, float a11f, float a22f, float a
     const float cf = (float)c;
     const float p = sqrtf(cf * (1.0f / 3.0f));
     const float r = fabsf((float)d) / (2.0f * p * p * p);
-    if (!(cf > 1e-22f && cf < 1e22f && r <= 0.99999f)) {
+    if (!(cf > 1e-22f && cf < 1e22f && r <= 0.9999998f)) {
         const Eigen3 e = eig3_general(a00f, a11f, a22f, a01f, a02f, a12f);
         lam[0] = e.l[0];
         lam[1] = e.l[1];
@@ -913,7 +913,7 @@ bool pipe_launch(cam_ctx *ctx, const char *name, const typename CTw<T>::t *src, 
 template <typename T>
 void tweb_impl(cam_ctx *ctx, FftPlan *plan, const Spectrum &dk, float L, const double *d_mean,
                int input_type, const cam_tweb_opts &o, uint8_t *d_labels, float *d_lambdas,
-               cam_tweb_stats *stats, float *d_inv)
+               cam_tweb_stats *stats, float *d_inv, unsigned long long *d_counts)
 {
     using C = typename CTw<T>::t;
     constexpr int W = CTw<T>::kCols;
@@ -924,8 +924,11 @@ void tweb_impl(cam_ctx *ctx, FftPlan *plan, const Spectrum &dk, float L, const d
     const int64_t ccomp = nn * M;
     C *cm = static_cast<C *>(scratch(ctx, "tw.main", (size_t)6 * ccomp * sizeof(C)));
     C *cn = static_cast<C *>(scratch(ctx, "tw.nyq", (size_t)6 * nn * sizeof(C)));
-    auto *cnt = static_cast<unsigned long long *>(scratch(ctx, "tw.cnt", 8 * sizeof(unsigned long long)));
-    CAM_CUDA_TRY(cudaMemsetAsync(cnt, 0, 8 * sizeof(unsigned long long), ctx->stream));
+    unsigned long long *cnt = d_counts;
+    if (!cnt) {
+        cnt = static_cast<unsigned long long *>(scratch(ctx, "tw.cnt", 8 * sizeof(unsigned long long)));
+        CAM_CUDA_TRY(cudaMemsetAsync(cnt, 0, 8 * sizeof(unsigned long long), ctx->stream));
+    }
 
     const double kf = 2.0 * M_PI / (double)L;
     const double R = o.smoothing_R;
@@ -1043,7 +1046,7 @@ void tweb_impl(cam_ctx *ctx, FftPlan *plan, const Spectrum &dk, float L, const d
 
 void tweb_device(cam_ctx *ctx, FftPlan *plan, const Spectrum &dk, float L, const double *d_mean,
                  int input_type, const cam_tweb_opts &o, uint8_t *d_labels, float *d_lambdas,
-                 cam_tweb_stats *stats, float *d_inv)
+                 cam_tweb_stats *stats, float *d_inv, unsigned long long *d_counts)
 {
     CAM_REQUIRE(std::isfinite(o.lambda_th) && o.tie_band >= 0.0, CAM_E_INVAL, "invalid T-web threshold");
     CAM_REQUIRE(o.smoothing_R >= 0.f && std::isfinite(o.smoothing_R), CAM_E_INVAL, "invalid smoothing radius");
@@ -1058,9 +1061,9 @@ void tweb_device(cam_ctx *ctx, FftPlan *plan, const Spectrum &dk, float L, const
         d_lambdas = static_cast<float *>(scratch(ctx, "tw.lam", (size_t)3 * ncell * sizeof(float)));
     }
     if (dk.precision == CAM_F32)
-        tweb_impl<float>(ctx, plan, dk, L, d_mean, input_type, o, d_labels, d_lambdas, stats, d_inv);
+        tweb_impl<float>(ctx, plan, dk, L, d_mean, input_type, o, d_labels, d_lambdas, stats, d_inv, d_counts);
     else
-        tweb_impl<double>(ctx, plan, dk, L, d_mean, input_type, o, d_labels, d_lambdas, stats, d_inv);
+        tweb_impl<double>(ctx, plan, dk, L, d_mean, input_type, o, d_labels, d_lambdas, stats, d_inv, d_counts);
 }
 
 }  // namespace cam
