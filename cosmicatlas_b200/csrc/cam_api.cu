@@ -312,6 +312,19 @@ __global__ void __launch_bounds__(256) publish_kernel(const __grid_constant__ Pu
 
 }  // namespace
 
+unsigned char *pinned(cam_ctx *ctx, size_t bytes)
+{
+    if (ctx->job_pin_bytes < bytes) {
+        std::lock_guard<std::mutex> lk(alloc_mutex());
+        if (ctx->job_pin) CAM_CUDA_TRY(cudaFreeHost(ctx->job_pin));
+        ctx->job_pin = nullptr;
+        ctx->job_pin_bytes = 0;
+        CAM_CUDA_TRY(cudaHostAlloc(reinterpret_cast<void **>(&ctx->job_pin), bytes, cudaHostAllocDefault));
+        ctx->job_pin_bytes = bytes;
+    }
+    return ctx->job_pin;
+}
+
 void publish(cam_ctx *ctx, const Publish &p, void *pinned_dst)
 {
     CAM_LAUNCH(ctx, publish_kernel, 1, 256, 0, p, static_cast<uint32_t *>(pinned_dst));
@@ -398,20 +411,6 @@ DevParticles stage_particles(cam_ctx *ctx, const cam_particles *p)
     d.z = stage_in(ctx, "in.z", p->z, p->n, p->mem);
     d.w = p->w ? stage_in(ctx, "in.w", p->w, p->n, p->mem) : nullptr;
     return d;
-}
-
-// The context's pinned readback buffer, at least `bytes`.
-unsigned char *pinned(cam_ctx *ctx, size_t bytes)
-{
-    if (ctx->job_pin_bytes < bytes) {
-        std::lock_guard<std::mutex> lk(alloc_mutex());
-        if (ctx->job_pin) CAM_CUDA_TRY(cudaFreeHost(ctx->job_pin));
-        ctx->job_pin = nullptr;
-        ctx->job_pin_bytes = 0;
-        CAM_CUDA_TRY(cudaHostAlloc(reinterpret_cast<void **>(&ctx->job_pin), bytes, cudaHostAllocDefault));
-        ctx->job_pin_bytes = bytes;
-    }
-    return ctx->job_pin;
 }
 
 // An exact run measured its fullest brick (and super-brick): later deferred
@@ -528,14 +527,30 @@ Spectrum alloc_spectrum(cam_ctx *ctx, int64_t n, int precision, const char *tag)
 
 namespace {
 
-// Power spectrum of a spectrum already on the device (split layout).
-void power_from_spectrum(cam_ctx *ctx, const Spectrum &s, float L, double n_obj, const cam_pk_opts &o,
+// Power spectrum of a spectrum already on the device (split layout); d_sum
+// (may be null): the sum of the density mesh.  One readback.
+void power_from_spectrum(cam_ctx *ctx, const Spectrum &s, float L, const double *d_sum, const cam_pk_opts &o,
                          double *pk, int64_t *modes, double *kvec, cam_pk_info *info)
 {
     const int nbins = nbins_for(o, s.n);
+    const PkDevice d = power_bin_device(ctx, s, o, nbins);
+    unsigned char *pin = pinned(ctx, 8 + (size_t)nbins * 24);
+    const auto *hs = reinterpret_cast<const double *>(pin + 8);
+    const auto *hm = reinterpret_cast<const unsigned long long *>(pin + 8 + (size_t)nbins * 16);
+    Publish p;
+    if (d_sum) p.add(d_sum, 8, 0);
+    p.add(d.sums, (size_t)nbins * 16, 8);
+    p.add(d.modes, (size_t)nbins * 8, 8 + (size_t)nbins * 16);
+    publish(ctx, p, pin);
+    CAM_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
     std::vector<double> sr(nbins), ss(nbins);
     std::vector<int64_t> md(nbins);
-    power_bin(ctx, s, o, nbins, sr.data(), ss.data(), md.data());
+    for (int b = 0; b < nbins; ++b) {
+        sr[b] = hs[2 * b];
+        ss[b] = hs[2 * b + 1];
+        md[b] = (int64_t)hm[b];
+    }
+    const double n_obj = d_sum ? *reinterpret_cast<const double *>(pin) : 0.0;
     finalize_pk(s.n, L, n_obj, o, nbins, sr.data(), ss.data(), md.data(), pk, modes, kvec, info);
 }
 
@@ -769,9 +784,8 @@ int cam_fft_r2c(cam_ctx *ctx, int64_t n, int precision, const void *in, void *ou
         const void *din = mem == CAM_MEM_DEVICE ? in : scratch(ctx, "fft.in", in_bytes);
         if (mem == CAM_MEM_HOST) CAM_CUDA_TRY(cudaMemcpyAsync((void *)din, in, in_bytes, cudaMemcpyHostToDevice, ctx->stream));
         Spectrum s = alloc_spectrum(ctx, n, precision, "fft.spec");
-        fft_r2c_split(ctx, plan, din, nullptr, s);
         void *dout = mem == CAM_MEM_DEVICE ? out : scratch(ctx, "fft.out", out_bytes);
-        split_to_fftw(ctx, s, dout);
+        fft_r2c_fftw(ctx, plan, din, s, dout);
         if (mem == CAM_MEM_HOST) CAM_CUDA_TRY(cudaMemcpyAsync(out, dout, out_bytes, cudaMemcpyDeviceToHost, ctx->stream));
         CAM_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
     });
@@ -790,9 +804,8 @@ int cam_fft_c2r(cam_ctx *ctx, int64_t n, int precision, const void *in, void *ou
         const void *din = mem == CAM_MEM_DEVICE ? in : scratch(ctx, "fft.out", in_bytes);
         if (mem == CAM_MEM_HOST) CAM_CUDA_TRY(cudaMemcpyAsync((void *)din, in, in_bytes, cudaMemcpyHostToDevice, ctx->stream));
         Spectrum s = alloc_spectrum(ctx, n, precision, "fft.spec");
-        fftw_to_split(ctx, din, s);
         void *dout = mem == CAM_MEM_DEVICE ? out : scratch(ctx, "fft.in", out_bytes);
-        fft_c2r_split(ctx, plan, s, dout, 1.0 / ((double)n * n * n));
+        fft_c2r_fftw(ctx, plan, din, s, dout, 1.0 / ((double)n * n * n));
         if (mem == CAM_MEM_HOST) CAM_CUDA_TRY(cudaMemcpyAsync(out, dout, out_bytes, cudaMemcpyDeviceToHost, ctx->stream));
         CAM_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
     });
@@ -822,7 +835,6 @@ int cam_power_multipoles(cam_ctx *ctx, const cam_grid *grid, const void *mesh, i
         const void *dm = mem == CAM_MEM_DEVICE ? mesh : scratch(ctx, "pk.mesh", bytes);
         if (mem == CAM_MEM_HOST) CAM_CUDA_TRY(cudaMemcpyAsync((void *)dm, mesh, bytes, cudaMemcpyHostToDevice, ctx->stream));
         auto *dsum = static_cast<double *>(scratch(ctx, "pk.sum", 2 * sizeof(double)));
-        double hs[2] = {0.0, 0.0};
         const double *sub = nullptr;
         if (opts->input_type == CAM_INPUT_DENSITY) {
             mesh_mean(ctx, dm, precision, n * n * n, dsum);
@@ -830,12 +842,8 @@ int cam_power_multipoles(cam_ctx *ctx, const cam_grid *grid, const void *mesh, i
         }
         Spectrum s = alloc_spectrum(ctx, n, precision, "job.spec");
         fft_r2c_split(ctx, plan, dm, sub, s);
-        if (sub) {
-            CAM_CUDA_TRY(cudaMemcpyAsync(hs, dsum, sizeof(hs), cudaMemcpyDeviceToHost, ctx->stream));
-            CAM_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
-        }
         cam_pk_info inf{};
-        power_from_spectrum(ctx, s, grid->L[0], hs[0], *opts, pk, modes, kvector, &inf);
+        power_from_spectrum(ctx, s, grid->L[0], sub ? dsum : nullptr, *opts, pk, modes, kvector, &inf);
         if (info) *info = inf;
         if (los >= 0 && (p2 || p4)) {
             // P_l = (2l + 1) sum L_l(mu) |F|^2 / W^2 / (modes normal), no shot
@@ -1081,10 +1089,13 @@ int cam_bam_kernel_update(cam_ctx *ctx, const cam_grid *grid, int precision, dou
         CAM_CUDA_TRY(cudaMemcpyAsync(dw, weight, (size_t)nbins * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
         bam_kernel_update_device(ctx, dk, precision, n, grid->L[0], DeltaKmin, ndel, nbins, dw, mode, dsum, dmod);
         if (mem == CAM_MEM_HOST) CAM_CUDA_TRY(cudaMemcpyAsync(kernel, dk, kbytes, cudaMemcpyDeviceToHost, ctx->stream));
-        std::vector<double> hs(nbins);
-        std::vector<unsigned long long> hm(nbins);
-        CAM_CUDA_TRY(cudaMemcpyAsync(hs.data(), dsum, (size_t)nbins * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
-        CAM_CUDA_TRY(cudaMemcpyAsync(hm.data(), dmod, (size_t)nbins * 8, cudaMemcpyDeviceToHost, ctx->stream));
+        unsigned char *pin = pinned(ctx, (size_t)nbins * 16);
+        const auto *hs = reinterpret_cast<const double *>(pin);
+        const auto *hm = reinterpret_cast<const unsigned long long *>(pin + (size_t)nbins * 8);
+        Publish p;
+        p.add(dsum, (size_t)nbins * 8, 0);
+        p.add(dmod, (size_t)nbins * 8, (size_t)nbins * 8);
+        publish(ctx, p, pin);
         CAM_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
         if (kernel_binned) {
             // kernel_updated[b] /= nmodes[b]; then bin 0 = mean of bins 1..4
@@ -1123,10 +1134,12 @@ int cam_konvolve(cam_ctx *ctx, const cam_grid *grid, const void *in, int precisi
         void *dout = out_mem == CAM_MEM_DEVICE ? out : scratch(ctx, "fd.out", bytes);
         fft_c2r_split(ctx, plan, s, dout, 1.0 / ((double)n * n * n));
         if (out_mem == CAM_MEM_HOST) CAM_CUDA_TRY(cudaMemcpyAsync(out, dout, bytes, cudaMemcpyDeviceToHost, ctx->stream));
-        double hsum = 0.0;
-        CAM_CUDA_TRY(cudaMemcpyAsync(&hsum, dsum, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
+        unsigned char *pin = pinned(ctx, sizeof(double));
+        Publish p;
+        p.add(dsum, sizeof(double), 0);
+        publish(ctx, p, pin);
         CAM_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
-        CAM_REQUIRE(std::isfinite(hsum), CAM_E_NONFINITE, "Konvolve: the input mesh holds a non-finite value");
+        CAM_REQUIRE(std::isfinite(*reinterpret_cast<const double *>(pin)), CAM_E_NONFINITE, "Konvolve: the input mesh holds a non-finite value");
     });
 }
 

@@ -269,6 +269,8 @@ struct Publish {
     }
 };
 void publish(cam_ctx *ctx, const Publish &p, void *pinned_dst);
+// The context's pinned readback buffer, at least `bytes`; one use at a time.
+unsigned char *pinned(cam_ctx *ctx, size_t bytes);
 
 // Runs the assignment pipeline on device particle arrays.  Writes the mesh
 // and, on the device, the FP64 mesh sum.  Synchronises once (payload size)
@@ -298,6 +300,10 @@ void fft_r2c_split(cam_ctx *ctx, FftPlan *plan, const void *real_in, const doubl
                    Spectrum &out);
 // Inverse c2r (in place on the spectrum), result scaled by `scale`.
 void fft_c2r_split(cam_ctx *ctx, FftPlan *plan, Spectrum &spec, void *real_out, double scale);
+// The same transforms to and from FFTW's layout; `work` is a spectrum to work
+// in, and the input of the c2r is not changed.
+void fft_r2c_fftw(cam_ctx *ctx, FftPlan *plan, const void *real_in, Spectrum &work, void *out);
+void fft_c2r_fftw(cam_ctx *ctx, FftPlan *plan, const void *in, Spectrum &work, void *real_out, double scale);
 void split_to_fftw(cam_ctx *ctx, const Spectrum &s, void *dst);
 void fftw_to_split(cam_ctx *ctx, const void *src, Spectrum &s);
 
@@ -323,8 +329,6 @@ PkDevice power_cross_device(cam_ctx *ctx, const Spectrum &s1, const Spectrum &s2
 // Multipole sums about axis los (0 x, 1 y, 2 z): sums [nbins][2] FP64
 // (sum L_2(mu) |F|^2/W^2, sum L_4(mu) |F|^2/W^2), modes [nbins]; own buffers.
 PkDevice power_multipole_device(cam_ctx *ctx, const Spectrum &s, const cam_pk_opts &o, int nbins, int los);
-void power_bin(cam_ctx *ctx, const Spectrum &s, const cam_pk_opts &o, int nbins,
-               double *h_sum_raw, double *h_sum_sn, int64_t *h_modes);
 
 // Binning tables of a P(k) (cam_power.cu): on the device [h+1] 1/W^2 per
 // axis, [h+1] C/W^2 per axis, [nbins+1] squared bin edges (units of k_f),

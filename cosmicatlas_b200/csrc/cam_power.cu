@@ -586,23 +586,4 @@ PkDevice power_multipole_device(cam_ctx *ctx, const Spectrum &s, const cam_pk_op
     return power_bin_impl(ctx, s, nullptr, ox, nbins, "pkm", 2, los);
 }
 
-void power_bin(cam_ctx *ctx, const Spectrum &s, const cam_pk_opts &o, int nbins, double *h_sum_raw,
-               double *h_sum_sn, int64_t *h_modes)
-{
-    const PkDevice d = power_bin_device(ctx, s, o, nbins);
-    if (ctx->sync_free) return;  // sums stay in pk.res / pk.resm for the caller
-    double *res = d.sums;
-    unsigned long long *resm = d.modes;
-    std::vector<double> hres(2 * nbins);
-    std::vector<unsigned long long> hm(nbins);
-    CAM_CUDA_TRY(cudaMemcpyAsync(hres.data(), res, 2 * nbins * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
-    CAM_CUDA_TRY(cudaMemcpyAsync(hm.data(), resm, nbins * sizeof(unsigned long long), cudaMemcpyDeviceToHost, ctx->stream));
-    CAM_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
-    for (int b = 0; b < nbins; ++b) {
-        if (h_sum_raw) h_sum_raw[b] = hres[2 * b];
-        if (h_sum_sn) h_sum_sn[b] = hres[2 * b + 1];
-        if (h_modes) h_modes[b] = (int64_t)hm[b];
-    }
-}
-
 }  // namespace cam

@@ -1031,11 +1031,14 @@ void tweb_impl(cam_ctx *ctx, FftPlan *plan, const Spectrum &dk, float L, const d
         });
     }
     if (stats) {
-        unsigned long long h[5];
-        double mean = 0.0;
-        CAM_CUDA_TRY(cudaMemcpyAsync(h, cnt, sizeof(h), cudaMemcpyDeviceToHost, ctx->stream));
-        if (d_mean) CAM_CUDA_TRY(cudaMemcpyAsync(&mean, d_mean, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
+        unsigned char *pin = pinned(ctx, 6 * 8);
+        const auto *h = reinterpret_cast<const unsigned long long *>(pin);
+        Publish p;
+        p.add(cnt, 5 * 8, 0);
+        if (d_mean) p.add(d_mean, 8, 5 * 8);
+        publish(ctx, p, pin);
         CAM_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+        const double mean = d_mean ? *reinterpret_cast<const double *>(pin + 5 * 8) : 0.0;
         for (int a = 0; a < 4; ++a) stats->counts[a] = (int64_t)h[a];
         stats->ties = (int64_t)h[4];
         stats->mean = mean;
