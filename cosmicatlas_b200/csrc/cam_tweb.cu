@@ -647,13 +647,41 @@ __device__ __forceinline__ void flush_counts(unsigned lc0, unsigned lc1, unsigne
     if (threadIdx.x < 5 && cnt_s[threadIdx.x]) atomicAdd(&counts[threadIdx.x], (unsigned long long)cnt_s[threadIdx.x]);
 }
 
+// Threads of tidal_z_kernel for a compile-time row length (one per kPPT
+// points) and the CTAs per SM it is built for: the pass waits on its loads
+// and barriers, so the float label pass takes as many as 64 registers a
+// thread allow (384-point rows: six CTAs of 160; at five, 768^3 takes 11.2 ms
+// instead of 9.7), the eigenvalue pass as many as 80 (384^3 2.21 -> 1.87 ms).
+template <typename T, int LEN>
+constexpr int zthreads()
+{
+    if (LEN == 0) return 256;
+    const int t = fftdev::ct_threads(LEN, 6 * tweb_rpc<T>(LEN), CTw<T>::kPPT);
+    return t < 256 ? t : 256;
+}
+template <typename T, int LEN, bool LAMBDAS>
+constexpr int zmin_blocks()
+{
+    if (LAMBDAS) return LEN > 0 && LEN <= 384 ? 65536 / (80 * zthreads<T, LEN>()) : 2;
+    return sizeof(T) == 4 && LEN > 0 && LEN <= 384 ? 65536 / (64 * zthreads<T, LEN>()) : 2;
+}
+// Label two cells (one complex element) per thread and round, unless that
+// takes more rounds than one cell at a time.
+template <typename T, int LEN>
+constexpr bool zpairs()
+{
+    if (LEN == 0) return true;
+    const int t = zthreads<T, LEN>(), m = LEN * tweb_rpc<T>(LEN);
+    return 2 * ((m + t - 1) / t) <= (2 * m + t - 1) / t;
+}
+
 // c2r along z of the six components for `rpc` rows, then eigenvalues and
 // labels.  Without LAMBDAS the eigenvalues are not formed: the label needs
 // only the number of them above lambda_th, and the tie flag whether that
 // number differs between lambda_th - band and lambda_th + band.  Component c of row r: main at src + c*ccomp + r*M, Nyquist at
 // nyq + c*N*N + r.
 template <typename T, int LEN, bool LAMBDAS>
-__global__ void __launch_bounds__(256, 2)
+__global__ void __launch_bounds__(zthreads<T, LEN>(), zmin_blocks<T, LEN, LAMBDAS>())
 tidal_z_kernel(const typename CTw<T>::t *__restrict__ src, const typename CTw<T>::t *__restrict__ nyq,
                int n, int64_t nrows, int rpc, int64_t ccomp, Radices rd,
                const typename CTw<T>::t *__restrict__ tw, double lth, double band,
@@ -675,31 +703,48 @@ tidal_z_kernel(const typename CTw<T>::t *__restrict__ src, const typename CTw<T>
     const int nr = (int)min((int64_t)rpcv, nrows - row0);
     const int64_t nn = (int64_t)n * n;
     if (threadIdx.x < 5) cnt_s[threadIdx.x] = 0;
-    // Load + c2r untangling (see fft_rows_kernel, mode c2r).
+    // Load and c2r untangling: elements k and M - k of a row from one pair of
+    // loads (see tidal_z_pipe_kernel); item 0 makes Z[0], with the Nyquist
+    // element, and Z[M/2].  An odd M has no middle element and (M - 1)/2 pairs.
     const int per = rpcv * M;
-    for (int e = threadIdx.x; e < 6 * per; e += blockDim.x) {
-        const int c = e / per, rem = e % per;
-        const int r = rem / M, k = rem % M;
+    const int items = (M + 1) / 2;
+    const int nthr = LEN > 0 ? zthreads<T, LEN>() : (int)blockDim.x;
+#pragma unroll 4
+    for (int e = threadIdx.x; e < 6 * rpcv * items; e += nthr) {
+        const int row = e / items, k = e % items;  // row = field * rpcv + r
+        const int c = row / rpcv, r = row % rpcv;
         if (r >= nr) continue;
         const C *sm = src + (int64_t)c * ccomp + (row0 + r) * M;
-        C xk = sm[k];
-        C xm = k == 0 ? nyq[(int64_t)c * nn + row0 + r] : sm[M - k];
+        const int base = c * per + r * M;
+        auto pair = [&](int kk, C xk, C xm, C &zk, C &zm) {
+            const C a = C{xk.x + xm.x, xk.y - xm.y};
+            const C b = C{xk.x - xm.x, xk.y + xm.y};
+            C wv = __ldg(tw + kk);
+            wv.y = -wv.y;
+            const C u = fftdev::cmul(wv, b);
+            zk = C{a.x - u.y, a.y + u.x};
+            zm = C{a.x + u.y, u.x - a.y};
+        };
+        C zk, zm;
         if (k == 0) {
-            xk.y = 0;
-            xm.y = 0;
+            const T x0 = sm[0].x, xn = nyq[(int64_t)c * nn + row0 + r].x;
+            tile[fftdev::sidx<PAD>(base)] = C{x0 + xn, x0 - xn};
+            if ((M & 1) == 0) {
+                const C x = sm[M / 2];
+                pair(M / 2, x, x, zk, zm);
+                tile[fftdev::sidx<PAD>(base + M / 2)] = zk;
+            }
+        } else {
+            pair(k, sm[k], sm[M - k], zk, zm);
+            tile[fftdev::sidx<PAD>(base + k)] = zk;
+            tile[fftdev::sidx<PAD>(base + M - k)] = zm;
         }
-        const C a = C{xk.x + xm.x, xk.y - xm.y};
-        const C b = C{xk.x - xm.x, xk.y + xm.y};
-        C wv = __ldg(tw + k);
-        wv.y = -wv.y;
-        const C ib = fftdev::rot<C, true>(fftdev::cmul(wv, b));
-        tile[fftdev::sidx<PAD>(e)] = fftdev::cadd(a, ib);
     }
     __syncthreads();
     if constexpr (LEN > 0) {
         constexpr int RPCZ = tweb_rpc<T>(LEN);
-        fftdev::block_fft_fixed<C, true, true, 6 * RPCZ, LEN, fftdev::ct_threads(LEN, 6 * RPCZ, CTw<T>::kPPT), 1, LEN, 2,
-                                true, CTw<T>::kMaxR>(tile, tw);
+        fftdev::block_fft_fixed<C, true, true, 6 * RPCZ, LEN, zthreads<T, LEN>(), 1, LEN, 2, true, CTw<T>::kMaxR>(tile,
+                                                                                                              tw);
     } else {
         fftdev::block_fft<C, CTw<T>::kPPT, true, true, 0>(tile, M, 6 * rpc, 1, M, rd, tw, 2);
     }
@@ -709,17 +754,34 @@ tidal_z_kernel(const typename CTw<T>::t *__restrict__ src, const typename CTw<T>
     // that rounding (and by its own)
     const float thf = (float)lth;
     const float bandp = (float)((band + fabs(lth - (double)thf)) * (1.0 + 1e-3));
-    // real value z of row r of comp c: half z & 1 of complex element (c*rpc + r)*M + z/2
-    const T *re = reinterpret_cast<const T *>(tile);
+    // complex element m of a row holds the real values at z = 2m, 2m + 1
     const int64_t ncell = nn * n;
-    for (int e = threadIdx.x; e < nr * nz; e += blockDim.x) {
-        const int r = e / nz, z = e % nz;
-        float t6[6];
+    if constexpr (zpairs<T, LEN>()) {
+        for (int e = threadIdx.x; e < nr * M; e += nthr) {
+            const int r = e / M, m = e % M;
+            float ta[6], tb[6];
 #pragma unroll
-        for (int c = 0; c < 6; ++c)
-            t6[c] = (float)re[2 * fftdev::sidx<PAD>((c * rpcv + r) * M + (z >> 1)) + (z & 1)];
-        label_cell<LAMBDAS>(t6, lth, band, thf, bandp, (row0 + r) * nz + z, ncell, labels, lambdas, inv, lc0, lc1, lc2, lc3,
-                            lties);
+            for (int c = 0; c < 6; ++c) {
+                const C v = tile[fftdev::sidx<PAD>((c * rpcv + r) * M + m)];
+                ta[c] = (float)v.x;
+                tb[c] = (float)v.y;
+            }
+            const int64_t cell = (row0 + r) * nz + 2 * m;
+            label_cell<LAMBDAS>(ta, lth, band, thf, bandp, cell, ncell, labels, lambdas, inv, lc0, lc1, lc2, lc3, lties);
+            label_cell<LAMBDAS>(tb, lth, band, thf, bandp, cell + 1, ncell, labels, lambdas, inv, lc0, lc1, lc2, lc3,
+                                lties);
+        }
+    } else {
+        const T *re = reinterpret_cast<const T *>(tile);
+        for (int e = threadIdx.x; e < nr * nz; e += nthr) {
+            const int r = e / nz, z = e % nz;
+            float t6[6];
+#pragma unroll
+            for (int c = 0; c < 6; ++c)
+                t6[c] = (float)re[2 * fftdev::sidx<PAD>((c * rpcv + r) * M + (z >> 1)) + (z & 1)];
+            label_cell<LAMBDAS>(t6, lth, band, thf, bandp, (row0 + r) * nz + z, ncell, labels, lambdas, inv, lc0, lc1, lc2,
+                                lc3, lties);
+        }
     }
     flush_counts(lc0, lc1, lc2, lc3, lties, cnt_s, counts);
 }
@@ -1026,7 +1088,8 @@ void tweb_impl(cam_ctx *ctx, FftPlan *plan, const Spectrum &dk, float L, const d
         auto kz = d_lambdas ? tidal_z_kernel<T, LEN, true> : tidal_z_kernel<T, LEN, false>;
         smem_at_least(kz, smem);
         const unsigned grid = (unsigned)((nn + rpc - 1) / rpc);
-        CAM_LAUNCH_NAMED(ctx, "tweb_tidal_z_eigen", kz, grid, nthr, smem, cm, cn, (int)n, nn, rpc, ccomp, rm, tw, o.lambda_th,
+        const int zthr = LEN > 0 ? zthreads<T, LEN>() : nthr;
+        CAM_LAUNCH_NAMED(ctx, "tweb_tidal_z_eigen", kz, grid, zthr, smem, cm, cn, (int)n, nn, rpc, ccomp, rm, tw, o.lambda_th,
                    o.tie_band, d_labels, d_lambdas, d_inv, cnt);
         });
     }
