@@ -334,6 +334,8 @@ __device__ __forceinline__ int to_brick(const AssignGeom &g, int a, int o, int l
     return b;
 }
 
+__device__ __forceinline__ void prefetch_l2(const void *p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+
 // As for_particles, for particles stored as (x, y, z, w).
 template <int NT, typename F>
 __device__ __forceinline__ void for_packed(const float4 *__restrict__ in, int count, F &&one)
@@ -529,6 +531,22 @@ sort_kernel(const __grid_constant__ SortArgs A, const __grid_constant__ AssignGe
                 }
             }
             __syncthreads();
+        }
+        // the next tile's particles start on their way to L2: step 1 then
+        // waits for L2 and not for memory
+        if (LEVEL == 2) {
+            if (t + 1 < t1) {
+                const float4 *next = A.part + p0 + count;  // mostly the same super-brick's
+                for (int i = tid * 8; i < tile && p0 + count + i < (int64_t)A.part_cap; i += NT * 8) prefetch_l2(next + i);
+            }
+        } else {
+            const int64_t q0 = p0 + (int64_t)gridDim.x * tile;
+            for (int i = tid * 32; i < tile && q0 + i < A.np; i += NT * 32) {
+                prefetch_l2(A.x + q0 + i);
+                prefetch_l2(A.y + q0 + i);
+                prefetch_l2(A.z + q0 + i);
+                if (A.w) prefetch_l2(A.w + q0 + i);
+            }
         }
         // 3. cursors and the bins' places
         const int extra = LEVEL == 1 ? 0 : min((int)s_extra, recs - tile);
