@@ -502,6 +502,49 @@ fft_cols_tma_pk_kernel(const __grid_constant__ CUtensorMap map, TileDims td, int
     }
 }
 
+// r2c untangling of one row: with Z the half-length transform of the row's
+// even/odd pairs,
+//   X[k] = (Z[k] + conj Z[M-k])/2 - i/2 w^k (Z[k] - conj Z[M-k]),  w = e^{-2 pi i/n},
+// and, with w^(M-k) = -conj w^k, X[M-k] from the same sums.
+template <typename C>
+__device__ __forceinline__ void r2c_pair(C zk, C zm, C w, C &xk, C &xm)
+{
+    using T = decltype(zk.x);
+    const C zc = C{zm.x, -zm.y};
+    const C s = fftdev::cadd(zk, zc), d = fftdev::csub(zk, zc);
+    const C wd = fftdev::cmul(w, d);
+    xk = C{(T)0.5 * (s.x + wd.y), (T)0.5 * (s.y - wd.x)};
+    xm = C{(T)0.5 * (s.x - wd.y), (T)-0.5 * (s.y + wd.x)};
+}
+// Item e of a group of rows (items(M) per row): item 0 of a row writes X[0],
+// the Nyquist element X[M] and, for even M, X[M/2]; item k writes X[k] and
+// X[M-k].  at(i): element i of the group's tile.
+__host__ __device__ constexpr int row_items(int M) { return (M + 1) / 2; }
+template <typename C, typename At>
+__device__ __forceinline__ void r2c_item(int e, int M, At &&at, const C *__restrict__ tw, C *__restrict__ dm,
+                                         C *__restrict__ dn)
+{
+    const int r = e / row_items(M), k = e % row_items(M);
+    C *row = dm + (int64_t)r * M;
+    C xk, xm;
+    if (k > 0) {
+        r2c_pair(at(r * M + k), at(r * M + M - k), __ldg(tw + k), xk, xm);
+        row[k] = xk;
+        row[M - k] = xm;
+        return;
+    }
+    const C z0 = at(r * M);
+    r2c_pair(z0, z0, __ldg(tw), xk, xm);
+    row[0] = xk;
+    r2c_pair(z0, z0, __ldg(tw + M), xk, xm);
+    dn[r] = xk;
+    if ((M & 1) == 0) {
+        const C zh = at(r * M + M / 2);
+        r2c_pair(zh, zh, __ldg(tw + M / 2), xk, xm);
+        row[M / 2] = xk;
+    }
+}
+
 // Row transforms along the contiguous axis.
 //   MODE 0 (r2c): real rows of n -> main rows of n/2 + nyq element
 //   MODE 1 (c2r): main rows + nyq -> real rows of n (times `scale`)
@@ -542,21 +585,38 @@ fft_rows_kernel(const void *in, void *out_main, typename fftdev::CT<T>::t *nyq, 
     } else if (MODE == 1) {
         const C *srcm = static_cast<const C *>(in) + comp * ccomp_in + row0 * M;
         const C *srcn = nyq + comp * (ccomp_in / M) + row0;  // nyq plane is N*N per component
-        for (int e = threadIdx.x; e < tot; e += blockDim.x) {
-            const int r = e / M, k = e % M;
-            C xk = srcm[(int64_t)r * M + k];
-            C xm = (k == 0) ? srcn[r] : srcm[(int64_t)r * M + (M - k)];
-            if (k == 0) {  // imaginary parts of DC and Nyquist are ignored
-                xk.y = 0;
-                xm.y = 0;
-            }
-            // Z'[k] = X[k] + conj(X[M-k]) + i e^{+2 pi i k/n} (X[k] - conj(X[M-k]))
+        // Z'[k] = X[k] + conj(X[M-k]) + i e^{+2 pi i k/n} (X[k] - conj(X[M-k])); with
+        // a the sum and u = conj(w^k) times the difference, Z'[k] = a + i u and
+        // Z'[M-k] = conj(a) + i conj(u): one pair of loads for both.  Item 0 of
+        // a row makes Z'[0] (imaginary parts of DC and Nyquist are ignored) and
+        // Z'[M/2].
+        auto pair = [&](int kk, C xk, C xm, C &zk, C &zm) {
             const C a = C{xk.x + xm.x, xk.y - xm.y};
             const C b = C{xk.x - xm.x, xk.y + xm.y};
-            C wv = __ldg(tw + k);
+            C wv = __ldg(tw + kk);
             wv.y = -wv.y;
-            const C ib = fftdev::rot<C, true>(fftdev::cmul(wv, b));
-            at(e) = fftdev::cadd(a, ib);
+            const C u = fftdev::cmul(wv, b);
+            zk = C{a.x - u.y, a.y + u.x};
+            zm = C{a.x + u.y, u.x - a.y};
+        };
+#pragma unroll 4
+        for (int e = threadIdx.x; e < nr * row_items(M); e += blockDim.x) {
+            const int r = e / row_items(M), k = e % row_items(M);
+            const C *row = srcm + (int64_t)r * M;
+            C zk, zm;
+            if (k > 0) {
+                pair(k, row[k], row[M - k], zk, zm);
+                at(r * M + k) = zk;
+                at(r * M + M - k) = zm;
+            } else {
+                const T x0 = row[0].x, xn = srcn[r].x;
+                at(r * M) = C{x0 + xn, x0 - xn};
+                if ((M & 1) == 0) {
+                    const C x = row[M / 2];
+                    pair(M / 2, x, x, zk, zm);
+                    at(r * M + M / 2) = zk;
+                }
+            }
         }
     } else {
         const C *src = static_cast<const C *>(in) + comp * ccomp_in + row0 * n;
@@ -575,19 +635,7 @@ fft_rows_kernel(const void *in, void *out_main, typename fftdev::CT<T>::t *nyq, 
     if (MODE == 0) {
         C *dm = static_cast<C *>(out_main) + comp * ccomp_out + row0 * M;
         C *dn = nyq + comp * (ccomp_out / M) + row0;
-        const int tot2 = nr * (M + 1);
-        for (int e = threadIdx.x; e < tot2; e += blockDim.x) {
-            const int r = e / (M + 1), k = e % (M + 1);
-            const C zk = at(r * M + (k % M));
-            const C zc0 = at(r * M + ((M - k) % M));
-            const C zc = C{zc0.x, -zc0.y};
-            // X[k] = (Z[k] + conj Z[M-k])/2 - i/2 e^{-2 pi i k/n} (Z[k] - conj Z[M-k])
-            const C s = fftdev::cadd(zk, zc), d = fftdev::csub(zk, zc);
-            const C wd = fftdev::cmul(__ldg(tw + k), d);
-            const C xk = C{(T)0.5 * (s.x + wd.y), (T)0.5 * (s.y - wd.x)};
-            if (k < M) dm[(int64_t)r * M + k] = xk;
-            else dn[r] = xk;
-        }
+        for (int e = threadIdx.x; e < nr * row_items(M); e += blockDim.x) r2c_item(e, M, at, tw, dm, dn);
     } else if (MODE == 1) {
         T *dst = static_cast<T *>(out_main) + comp * ccomp_out + row0 * n;
         const T sc = (T)scale;
@@ -652,18 +700,8 @@ fft_rows_r2c_pipe_kernel(const T *__restrict__ in, typename fftdev::CT<T>::t *__
         fftdev::block_fft_fixed<C, false, true, RPC, LEN, NTHR, 1, LEN, 2, true, fftdev::CT<T>::kMaxR>(tile, tw);
         C *dm = out_main + row0 * M;
         C *dn = nyq + row0;
-        for (int e = threadIdx.x; e < nr * (M + 1); e += NTHR) {
-            const int r = e / (M + 1), k = e % (M + 1);
-            const C zk = tile[fftdev::sidx<true>(r * M + (k % M))];
-            const C zc0 = tile[fftdev::sidx<true>(r * M + ((M - k) % M))];
-            const C zc = C{zc0.x, -zc0.y};
-            // X[k] = (Z[k] + conj Z[M-k])/2 - i/2 e^{-2 pi i k/n} (Z[k] - conj Z[M-k])
-            const C s = fftdev::cadd(zk, zc), d = fftdev::csub(zk, zc);
-            const C wd = fftdev::cmul(__ldg(tw + k), d);
-            const C xk = C{(T)0.5 * (s.x + wd.y), (T)0.5 * (s.y - wd.x)};
-            if (k < M) dm[(int64_t)r * M + k] = xk;
-            else dn[r] = xk;
-        }
+        auto at = [&](int i) -> C { return tile[fftdev::sidx<true>(i)]; };
+        for (int e = threadIdx.x; e < nr * row_items(M); e += NTHR) r2c_item(e, M, at, tw, dm, dn);
         __syncthreads();  // tile is refilled next
     }
     fftdev::cp_async_wait<0>();
@@ -823,10 +861,12 @@ void rows_impl(cam_ctx *ctx, FftPlan *p, const void *in, void *out, void *nyq, i
     dispatch_fft_len(len, [&](auto lc) {
     constexpr int LEN = decltype(lc)::value;
     const size_t smem = (size_t)fftdev::padded_len((int64_t)rpc * len, LEN > 0) * sizeof(C);
-    if constexpr (MODE == 0 && LEN >= 16 && LEN <= 512 && (LEN & (LEN - 1)) == 0) {
-        // pipelined r2c rows for the power-of-two half lengths (their
-        // transforms fit the register bound without spilling): one
-        // component, 16-byte aligned input, raw + padded tile within 200 KB
+    if constexpr (MODE == 0 && LEN >= 16 && LEN <= 512 &&
+                  ((LEN & (LEN - 1)) == 0 || (sizeof(T) == 4 && LEN >= 192))) {
+        // pipelined r2c rows for the half lengths whose transforms fit the
+        // register bound (192 and 384 spill a few words and still gain: 768^3
+        // 1454 -> 1398 us): one component, 16-byte aligned input, raw + padded
+        // tile within 200 KB
         const size_t psmem = (size_t)rpc * len * sizeof(C) + smem;
         if (ncomp == 1 && ((uintptr_t)in % 16) == 0 && (len * sizeof(C)) % 16 == 0 && psmem <= 200 * 1024) {
             auto kp = fft_rows_r2c_pipe_kernel<T, LEN>;
