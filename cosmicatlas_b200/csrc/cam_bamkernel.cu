@@ -86,6 +86,9 @@ bamk_update_kernel(T *__restrict__ K, int n, const double *__restrict__ weight, 
     double *mysum = wsum + (size_t)warp * nbins;
     unsigned long long *mycnt = wcnt + (size_t)warp * nbins;
     const int h = n / 2, L1 = h + 1;
+    // mode 0 in float: a run's elements all equal its weight, and sums of up
+    // to 2^29 equal floats are exact in FP64, so the count gives the sum
+    constexpr bool kExact = sizeof(T) == 4;
     const int64_t nrows = (int64_t)n * n;
     const int64_t r_beg = (int64_t)blockIdx.x * rows_per_cta;
     const int64_t r_end = min(nrows, r_beg + rows_per_cta);
@@ -116,17 +119,19 @@ bamk_update_kernel(T *__restrict__ K, int n, const double *__restrict__ weight, 
             const unsigned heads = __ballot_sync(0xffffffffu, head);
             const unsigned later = heads & ~((2u << lane) - 1u);
             const int end = later ? __ffs((int)later) - 1 : 32;
+            if (!kExact || mode != 0) {
 #pragma unroll
-            for (int off = 1; off < 32; off <<= 1) {
-                const double o = __shfl_down_sync(0xffffffffu, v, off);
-                if (lane + off < end) v += o;
+                for (int off = 1; off < 32; off <<= 1) {
+                    const double o = __shfl_down_sync(0xffffffffu, v, off);
+                    if (lane + off < end) v += o;
+                }
             }
             const bool valid = c < L1 && bin >= 0 && bin < nbins;
             const unsigned vmask = __ballot_sync(0xffffffffu, valid);
             const unsigned run = (end == 32 ? 0xffffffffu : ((1u << end) - 1u)) & ~((1u << lane) - 1u);
             const int cnt = __popc(vmask & run);
             if (head && bin >= 0 && bin < nbins && cnt) {
-                mysum[bin] += v;
+                mysum[bin] += kExact && mode == 0 ? v * (double)cnt : v;
                 mycnt[bin] += (unsigned long long)cnt;
             }
             __syncwarp();
@@ -177,23 +182,31 @@ bamk_final_kernel(const double *__restrict__ part, const unsigned long long *__r
 
 // F(i, j, k) *= K[(i N + j)(N/2 + 1) + k] * 2 w * s2, w = *d_w: the kernel
 // product of Konvolve with the factor 2 w / N^3 of its normalisation folded
-// in (s2 = 1 / N^3; the c2r applies the other 1 / N^3).  Loops over the
-// kernel's half-complex order, so K is read contiguously.
+// in (s2 = 1 / N^3; the c2r applies the other 1 / N^3).
 template <typename T>
 __global__ void konvolve_mult_kernel(typename fftdev::CT<T>::t *__restrict__ main_, typename fftdev::CT<T>::t *__restrict__ nyq,
                                      const T *__restrict__ K, int n, const double *__restrict__ d_w, double s2)
 {
     using C = typename fftdev::CT<T>::t;
     const int M = n / 2, L1 = M + 1;
-    const int64_t tot = (int64_t)n * n * L1;
     const T f = (T)(2.0 * (*d_w) * s2);
-    for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < tot; e += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t r = e / L1;
-        const int k = (int)(e - r * L1);
-        C *p = k < M ? main_ + r * M + k : nyq + r;
-        const T m = K[e] * f;
-        const C v = *p;
-        *p = C{v.x * m, v.y * m};
+    // a warp takes a row at a time (no division per element)
+    const int lane = threadIdx.x & 31;
+    const int64_t nrows = (int64_t)n * n, warps = (int64_t)gridDim.x * (blockDim.x >> 5);
+    for (int64_t r = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); r < nrows; r += warps) {
+        const T *k_row = K + r * L1;
+        C *row = main_ + r * M;
+#pragma unroll 4
+        for (int k = lane; k < M; k += 32) {
+            const T m = k_row[k] * f;
+            const C v = row[k];
+            row[k] = C{v.x * m, v.y * m};
+        }
+        if (lane == 0) {
+            const T m = k_row[M] * f;
+            const C v = nyq[r];
+            nyq[r] = C{v.x * m, v.y * m};
+        }
     }
 }
 

@@ -30,6 +30,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <string>
 #include <type_traits>
 
 #include "cam_fft_device.cuh"
@@ -1001,9 +1002,14 @@ void tweb_impl(cam_ctx *ctx, FftPlan *plan, const Spectrum &dk, float L, const d
     const double scale = (pot ? kf * kf : 1.0) / ((double)n * (double)n * (double)n);
     const C *sf = nullptr;
     if (o.method == CAM_TWEB_FD) {
-        auto *t = static_cast<C *>(scratch(ctx, "tw.sfac", (size_t)(n + 1) * sizeof(C)));
-        CAM_LAUNCH_NAMED(ctx, "fd_table_kernel", fd_table_kernel<T>, (unsigned)((n + 1 + 127) / 128), 128, 0, t,
-                         (int)n);
+        // depends on N and the precision only: made once per context
+        const std::string key = "tw.sfac." + std::to_string(n) + (sizeof(T) == 4 ? "f" : "d");
+        const auto found = ctx->bufs.find(key);
+        const bool fresh = found == ctx->bufs.end() || found->second.ptr == nullptr;
+        auto *t = static_cast<C *>(scratch(ctx, key.c_str(), (size_t)(n + 1) * sizeof(C)));
+        if (fresh)
+            CAM_LAUNCH_NAMED(ctx, "fd_table_kernel", fd_table_kernel<T>, (unsigned)((n + 1 + 127) / 128), 128, 0, t,
+                             (int)n);
         sf = t;
     }
     // The Nyquist planes' x and y passes (a few CTAs each: 13 + 21 us at 64^3,
