@@ -4,25 +4,23 @@
 // Source/massFunctions.cpp:35-98, :678-790, :1050-1165.
 //
 // Pipeline (no float atomics, bitwise deterministic):
-//   1. bin_count   : each CTA takes a contiguous chunk of particles and
-//                    computes, per particle, the reference's FP32 home cell
-//                    (bit-exact key) and the mesh bricks its stencil
-//                    touches; a shared-memory histogram per CTA is added to
-//                    per-brick counters.  Also lost particles, max |w|.
-//   2. scan        : exclusive scan of the brick counts: every brick owns a
-//                    contiguous payload range, its counter becomes its
-//                    append cursor.
-//   3. bin_scatter : the particles again; one 16-byte payload per touched
-//                    brick (home cell relative to the brick, exact
-//                    fractional offset in fixed point, weight) at the next
-//                    slot of the brick's cursor (one global atomic each).
-//   4. deposit     : one CTA per brick accumulates its payloads into a
-//                    shared-memory tile of 64-bit fixed-point cell sums kept
-//                    as two 32-bit words (32-bit shared atomics, the carry
-//                    detected from the returned old value).  Integer sums do
-//                    not depend on arrival order, so the result is
-//                    deterministic; the tile is written once, coalesced, as
-//                    FP32/FP64 (or uint32 counts for NGP).
+//   1. count   : per particle, the reference's FP32 home cell (bit-exact key)
+//                and the mesh bricks its stencil touches, counted per brick;
+//                lost particles, weight statistics.  An exclusive scan gives
+//                every brick its range of the payload.  Deferred runs skip
+//                this and give every brick a slab (see assign_impl).
+//   2. scatter : the particles again; one 16-byte record per touched brick
+//                (home cell relative to the brick, exact fractional offset
+//                in fixed point, weight), sorted by brick within a tile in
+//                shared memory and appended in runs; meshes with more bricks
+//                than a tile counts sort by super-brick first (sort_kernel).
+//   3. deposit : one CTA per brick accumulates its records into a
+//                shared-memory tile of 64-bit fixed-point cell sums kept
+//                as two 32-bit words (32-bit shared atomics, the carry
+//                detected from the returned old value).  Integer sums do
+//                not depend on arrival order, so the result is
+//                deterministic; the tile is written once, coalesced, as
+//                FP32/FP64 (or uint32 counts for NGP).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -36,7 +34,7 @@ namespace cam {
 namespace {
 
 constexpr int kBinThreads = 1024;
-constexpr int kDepositThreads = 512;
+constexpr int kDepositThreads = 640;  // two CTAs per SM in 48 registers (512: TSC 333 -> 342 us at 256^3, NGP 101 -> 105)
 constexpr int kScatterThreads = 512;  // scatter pass: two CTAs per SM
 constexpr int kSmemBricks = 16384;  // per-CTA brick histogram in shared memory (64 KB)
 using namespace asg;
@@ -890,12 +888,13 @@ __global__ void brick_starts_kernel(const uint32_t *__restrict__ scanned, int nb
     }
 }
 
-// Pass 4: one CTA per brick, two CTAs of 512 threads per SM.  Bound by the
+// Pass 4: one CTA per brick, two CTAs per SM.  Bound by the
 // shared-memory atomics (one per stencil cell, 3.7 wavefronts each: 32 random
 // cells on 32 banks) and, for NGP and CIC, by the latency of the record
-// loads.  256^3, 16.8 M weighted particles: TSC 417 -> 341 us, CIC 200 ->
-// 156, NGP 136 -> 122 with the stencil on constant offsets from one address
-// (508 warp instructions per 32 TSC records before; 78% issue).
+// loads.  256^3, 16.8 M weighted particles: TSC 417 -> 333 us, CIC 200 ->
+// 148, NGP 136 -> 101 with the stencil on constant offsets from one address
+// (508 warp instructions per 32 TSC records before; 78% issue) and the record
+// loads two groups ahead.
 template <int SCHEME, typename OutT>
 __global__ void __launch_bounds__(kDepositThreads, 2)
 deposit_kernel(const uint4 *__restrict__ payload, const uint32_t *__restrict__ start, uint32_t nrec,
