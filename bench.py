@@ -441,7 +441,7 @@ def run_ours(args):
             "power": 8 * nh,
         }
         stage_kernels = {
-            "assign": ["assign_bin_count", "assign_starts", "assign_partition", "tile_sum_kernel", "tile_offsets_kernel",
+            "assign": ["assign_bin_count", "assign_starts", "assign_super_count", "assign_super_sort", "tile_sum_kernel", "tile_offsets_kernel",
                        "tile_scan_kernel", "assign_bin_scatter", "assign_deposit", "partial_sum_kernel<double>",
                        "final_sum_kernel"],
             # fft_cols_pk: the x pass that also bins P(k) (the binning adds no traffic)
@@ -697,7 +697,7 @@ def run_single(args):
     stage_bytes = {"assign": npart * 12 + 4 * n ** 3, "fft_r2c": 4 * n ** 3 + 8 * nh, "power": 8 * nh,
                    "tweb": 8 * nh + n ** 3}
     stage_kernels = {
-        "assign": ["assign_bin_count", "assign_scan", "assign_partition", "assign_bin_scatter", "assign_deposit",
+        "assign": ["assign_bin_count", "assign_super_count", "assign_super_sort", "assign_bin_scatter", "assign_deposit",
                    "partial_sum_kernel<double>", "final_sum_kernel", "assign_starts", "tile_sum_kernel",
                    "tile_offsets_kernel", "tile_scan_kernel"],
         "fft_r2c": ["fft_rows_r2c", "fft_cols", "fft_rows_c2c", "fft_cols_pk"],
