@@ -22,8 +22,8 @@
 //                inverse FFT along y; (p, 0) overwrites its input in place,
 //                as the last output of the same CTA;
 //   tidal_z    : c2r along z of the six fields of a few rows,
-//                then the eigenvalues (FP32 trigonometric solution plus one
-//                FP64 Newton step) and the label of every cell (uint8).
+//                then the label of every cell (uint8) from sign counts and,
+//                when asked for, its eigenvalues (eig3).
 // Field slots: 0 = (0,0) -> T_zz, 1 = (1,0) -> T_xz, 2 = (2,0) -> T_xx,
 // 3 = (0,1) -> T_yz, 4 = (0,2) -> T_yy, 5 = (1,1) -> T_xy.
 #include <cuda_runtime.h>
@@ -443,10 +443,12 @@ __device__ __noinline__ Eigen3 eig3_general(float a00f, float a11f, float a22f, 
 // from the chord sqrt 3 + (2 - sqrt 3) r (error 0.014, then < 2e-4, then the
 // FP32 rounding) start two in FP64 with an FP32 reciprocal of the slope (each
 // gains a factor 1e-7); the other roots are -x/2 +- sqrt(c - 3 x^2 / 4), the
-// root from an FP32 reciprocal root and one FP64 step.  Error ~1e-13 of the
-// spread up to r = 1 - 2e-7 (the cancellation in the root there); nearer to a double root, or where FP32 would
-// under- or overflow, eig3_general.  About 45 FP64 operations a cell in place
-// of some 350: the eigenvalue z pass at 256^3 was bound by them.
+// root from an FP32 reciprocal root and one FP64 step.  Error
+// ~1e-12 of the spread down to disc = 5e-8 c (r = 1 - 2e-7: its cancellation);
+// nearer to a double root, or where FP32 would under- or overflow,
+// eig3_general.  disc is tested and not r, whose FP32 rounding can hide that
+// the other two are equal.  About 45 FP64 operations a cell in place of some
+// 350: the eigenvalue z pass at 256^3 was bound by them.
 __device__ __forceinline__ void eig3(float a00f, float a11f, float a22f, float a01f, float a02f, float a12f,
                                      double lam[3])
 {
@@ -458,13 +460,6 @@ __device__ __forceinline__ void eig3(float a00f, float a11f, float a22f, float a
     const float cf = (float)c;
     const float p = sqrtf(cf * (1.0f / 3.0f));
     const float r = fabsf((float)d) / (2.0f * p * p * p);
-    if (!(cf > 1e-22f && cf < 1e22f && r <= 0.9999998f)) {
-        const Eigen3 e = eig3_general(a00f, a11f, a22f, a01f, a02f, a12f);
-        lam[0] = e.l[0];
-        lam[1] = e.l[1];
-        lam[2] = e.l[2];
-        return;
-    }
     float y = 1.7320508f + 0.2679492f * r;
 #pragma unroll
     for (int k = 0; k < 2; ++k) y -= ((y * y - 3.0f) * y - 2.0f * r) * __frcp_rn(3.0f * y * y - 3.0f);
@@ -474,6 +469,13 @@ __device__ __forceinline__ void eig3(float a00f, float a11f, float a22f, float a
 #pragma unroll
     for (int k = 0; k < 2; ++k) x -= ((x * x - c) * x - d) * (double)slope;
     const double disc = c - 0.75 * x * x;
+    if (!(cf > 1e-22f && cf < 1e22f && disc > 5e-8 * c)) {
+        const Eigen3 e = eig3_general(a00f, a11f, a22f, a01f, a02f, a12f);
+        lam[0] = e.l[0];
+        lam[1] = e.l[1];
+        lam[2] = e.l[2];
+        return;
+    }
     const float h = rsqrtf((float)disc);
     double s = disc * (double)h;
     s += (0.5 * (double)h) * (disc - s * s);

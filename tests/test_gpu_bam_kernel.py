@@ -36,6 +36,26 @@ def test_kernel_update_bit_exact(ctx, n, box, kmin_u, ndel, nb, prec, mode):
     np.testing.assert_allclose(binned, wbinned, rtol=1e-12)
 
 
+@pytest.mark.parametrize("n,nb", [(12, 5), (72, 30), (96, 40)])
+def test_kernel_set_and_konvolve_ragged_rows(ctx, n, nb):
+    # rows that are no multiple of a warp: the set sums come from the counts
+    # and the kernel product goes row by row
+    rng = np.random.default_rng(n)
+    box = 400.0
+    k0 = rng.uniform(0.5, 1.5, size=(n, n, n // 2 + 1)).astype(np.float32)
+    w = rng.uniform(0.8, 1.25, size=nb)
+    got = k0.copy()
+    binned, modes = ctx.bam_kernel_update(got, box, w, L.KERNEL_SET)
+    want, wbinned, wmodes = orc.bam_kernel_update_ref(k0, box, w, False)
+    assert np.array_equal(got, want)
+    assert np.array_equal(modes, wmodes)
+    np.testing.assert_allclose(binned, wbinned, rtol=1e-12)
+    delta = rng.normal(size=(n, n, n)).astype(np.float32)
+    out = ctx.konvolve(delta, box, got)
+    ref = orc.konvolve_f64(delta, got, n)
+    assert np.max(np.abs(out - ref)) <= 1e-5 * np.abs(ref).max()
+
+
 def test_kernel_update_on_device(ctx):
     import torch
     n, box, nb = 64, 500.0, 32

@@ -57,6 +57,38 @@ def test_tweb_delta_input(ctx):
     assert bad == 0
 
 
+@pytest.mark.parametrize("n,prec", [(8, F32), (12, F32), (24, F32), (96, F32), (12, F64), (96, F64)])
+def test_tweb_row_lengths(ctx, n, prec):
+    # rows of the z pass outside the pipelined kernel (half lengths with a
+    # factor 3, and the shortest): eigenvalues and labels
+    rng = np.random.default_rng(n)
+    delta = rng.normal(size=(n, n, n)).astype(np.float64 if prec == F64 else np.float32)
+    box = 10.0 * n
+    opts = Context.tweb_opts(15.0, 0.0, BAND, input_type=1)
+    got = ctx.tweb(delta, box, opts, want_lambdas=True)
+    ref = orc.tweb_from_spectrum(orc.rfft3_f64(delta.astype(np.float64)), n, box, 15.0, 0.0, BAND)
+    lam = np.moveaxis(got.lambdas, 0, -1).astype(np.float64)
+    assert np.max(np.abs(lam - ref.lam)) <= 1e-5 * np.abs(ref.lam).max()
+    assert label_check(got.labels, ref.lam, ref.labels, 0.0)[0] == 0
+    assert np.array_equal(ctx.tweb(delta, box, opts).labels, got.labels)
+
+
+@pytest.mark.parametrize("axes", [(1, 0, 0), (1, 1, 0), (1, 1, 1)])
+def test_tweb_eigenvalues_next_to_double_roots(ctx, axes):
+    # a plane wave's tensor has one eigenvalue and a double root 0, up to the
+    # rounding of the transforms; a symmetric tensor's eigenvalues move by at
+    # most the norm of its error, so the bar is the same as everywhere
+    n, box = 32, 100.0
+    i = np.arange(n) * (2 * np.pi / n)
+    phase = axes[0] * i[:, None, None] + axes[1] * i[None, :, None] + axes[2] * i[None, None, :]
+    delta = np.cos(phase).astype(np.float32)
+    got = ctx.tweb(delta, box, Context.tweb_opts(0.0, 0.0, BAND, input_type=1), want_lambdas=True)
+    ref = orc.tweb_from_spectrum(orc.rfft3_f64(delta.astype(np.float64)), n, box, 0.0, 0.0, BAND)
+    lam = np.moveaxis(got.lambdas, 0, -1).astype(np.float64)
+    assert np.max(np.abs(lam - ref.lam)) <= 1e-5 * np.abs(ref.lam).max()
+    assert np.all(lam[..., 0] >= lam[..., 1]) and np.all(lam[..., 1] >= lam[..., 2])
+
+
 def oracle_job(x, y, z, w, n, box, scheme, nbins, R, lth, precision):
     mesh, lost = orc.assign_f64(scheme, x, y, z, w, orc.Grid.cubic(n, box))
     if precision == F32:
