@@ -307,10 +307,11 @@ int cam_konvolve(cam_ctx *ctx, const cam_grid *grid, const void *in, int precisi
  * spectrum stay resident on the device between the stages, and the host
  * waits once, for the statistics and P(k) at the end.  A context's first
  * job of a mesh shape sorts the particles into mesh bricks exactly (count,
- * scan, scatter) and measures its fullest brick; later jobs of that shape
- * write every brick's records into a fixed slab sized from it and skip the
- * count.  A job whose records do not fit (its slabs or the payload
- * estimate) runs again exactly, so results never depend on the path. */
+ * scan, scatter) and measures its fullest brick (and, on meshes of more than
+ * 4096 bricks, its fullest group of bricks); later jobs and cam_assign calls
+ * of that shape write every brick's records into a fixed slab sized from it
+ * and skip the count.  A job whose records do not fit (its slabs or the
+ * payload estimate) runs again exactly, so results never depend on the path. */
 typedef struct {
     cam_particles parts;
     cam_grid grid;
