@@ -1088,23 +1088,7 @@ static void assign_impl(cam_ctx *ctx, const float *x, const float *y, const floa
             const SuperGeom s = super_geom(geom, std::min(most, kMaxSupers));
             if (local_bins_of(s) <= kMaxLocal) sg = s;
         }
-    const bool two = sg.count > 0;
-    const bool staged = two || nb <= kStageBins;
     AssignGeom g = geom;
-    g.cstride = staged ? 1 : kPaddedStride;
-    // statistics and per-brick counters (counts, then cursors): one buffer,
-    // zeroed at once
-    const size_t head_bytes = kAssignHead + (size_t)nb * g.cstride * sizeof(uint32_t);
-    auto *stats = static_cast<unsigned long long *>(scratch(ctx, "asg.head", head_bytes));
-    auto *table = reinterpret_cast<uint32_t *>(reinterpret_cast<unsigned char *>(stats) + kAssignHead);
-    auto *start = static_cast<uint32_t *>(scratch(ctx, "asg.start", (nb + 1) * sizeof(uint32_t)));
-    auto *bsum = static_cast<double *>(scratch(ctx, "asg.bsum", nb * sizeof(double)));
-    unsigned long long *d_lost = stats;
-    unsigned int *d_wmax = reinterpret_cast<unsigned int *>(stats + 1);
-    uint32_t *d_total = reinterpret_cast<uint32_t *>(stats + 2);
-    unsigned int *d_ovf = reinterpret_cast<unsigned int *>(stats + 3);
-    CAM_CUDA_TRY(cudaMemsetAsync(stats, 0, head_bytes, ctx->stream));
-
     // Expected records per particle of a uniform catalogue: a stencil
     // crosses a face of a brick of extent b with probability (W-1)/b per
     // axis; at most two bricks per axis.
@@ -1129,13 +1113,14 @@ static void assign_impl(cam_ctx *ctx, const float *x, const float *y, const floa
     const double est_brick = (double)np * f / (double)nb;
     const int64_t shape = ((int64_t)g.n[0] << 32) | ((int64_t)g.n[1] << 16) | (int64_t)g.n[2];
     double est_super = (double)np;
-    for (int a = 0; a < 3 && two; ++a)
+    for (int a = 0; a < 3 && sg.count > 0; ++a)
         est_super *= (double)std::min(sg.gs[a] * g.b[a], g.n[a]) / (double)g.n[a];
     const uint64_t beyond = std::max<uint64_t>(65536, (uint64_t)np / 256);  // room of the last bin, with slabs
     uint32_t slab = 0;
     if (out.defer && plain_ctx && np > 0) {
         const auto it = ctx->slab_clump.find(shape);
         const auto is = ctx->super_clump.find(shape);
+        const bool two = sg.count > 0;
         if (it != ctx->slab_clump.end() && (!two || is != ctx->super_clump.end())) {
             const uint64_t cap = slab_capacity(it->second * est_brick);
             const double room = std::max((two ? 3.0 : 2.0) * (double)np * f, (double)(1u << 20));
@@ -1147,9 +1132,31 @@ static void assign_impl(cam_ctx *ctx, const float *x, const float *y, const floa
                        (uint64_t)sg.count * scap + beyond < (1ull << 32);
                 if (fits) sg.cap = (uint32_t)scap;
             }
+            // With more than 128 super-bricks the exact counts of two levels
+            // cost more than their longer runs save (768^3, 453 M TSC
+            // particles, 216 of them: counts 5.0 ms, sort 3.4, records 8.0;
+            // one level 4.45 and 8.8), and a shape that has its clumping
+            // measured and is too clumped for slabs has no more use for them.
             if (fits) slab = (uint32_t)cap;
+            else if (sg.count > 128) sg = SuperGeom{};
         }
     }
+    const bool two = sg.count > 0;
+    const bool staged = two || nb <= kStageBins;
+    g.cstride = staged ? 1 : kPaddedStride;
+    // statistics and per-brick counters (counts, then cursors): one buffer,
+    // zeroed at once
+    const size_t head_bytes = kAssignHead + (size_t)nb * g.cstride * sizeof(uint32_t);
+    auto *stats = static_cast<unsigned long long *>(scratch(ctx, "asg.head", head_bytes));
+    auto *table = reinterpret_cast<uint32_t *>(reinterpret_cast<unsigned char *>(stats) + kAssignHead);
+    auto *start = static_cast<uint32_t *>(scratch(ctx, "asg.start", (nb + 1) * sizeof(uint32_t)));
+    auto *bsum = static_cast<double *>(scratch(ctx, "asg.bsum", nb * sizeof(double)));
+    unsigned long long *d_lost = stats;
+    unsigned int *d_wmax = reinterpret_cast<unsigned int *>(stats + 1);
+    uint32_t *d_total = reinterpret_cast<uint32_t *>(stats + 2);
+    unsigned int *d_ovf = reinterpret_cast<unsigned int *>(stats + 3);
+    CAM_CUDA_TRY(cudaMemsetAsync(stats, 0, head_bytes, ctx->stream));
+
     // What the sort kernels share; tile and recs are set per level.
     SortArgs A{};
     A.x = x;

@@ -355,3 +355,28 @@ def test_two_level_sort_vs_oracle(ctx, scheme, weighted):
     p = rng.permutation(npart)
     again = ctx.assign(*(v[p] for v in xs), None if w is None else w[p], g, scheme, F32)
     assert np.array_equal(r.mesh.view(np.uint32), again.mesh.view(np.uint32))
+
+
+@pytest.mark.parametrize("scheme", [NGP, TSC])
+def test_many_super_bricks_too_clumped_for_slabs(scheme):
+    # 768^3 sorts by more than 128 super-bricks; a catalogue whose fullest
+    # brick no slab holds is sorted in two levels once and counted in one
+    # after that: the same mesh, bit for bit
+    import torch
+    n, L, npart = 768, 1000.0, 1_100_003
+    gen = torch.Generator(device="cuda").manual_seed(scheme + 1)
+    xs = [torch.rand(npart, device="cuda", generator=gen) * (40.0 if a else 1000.0) for a in range(3)]
+    c = Context()
+    try:
+        g = make_grid(n, L)
+        c.profile(True)
+        c.profile_read(True)
+        first = c.assign(*xs, None, g, scheme, F32)
+        assert "assign_super_sort" in c.profile_read(True)
+        again = c.assign(*xs, None, g, scheme, F32)
+        names = c.profile_read(True)
+        assert "assign_super_sort" not in names and "assign_bin_count" in names
+        assert first.n_lost == again.n_lost and first.sum_mesh == again.sum_mesh == npart - first.n_lost
+        assert np.array_equal(np.asarray(first.mesh.cpu()), np.asarray(again.mesh.cpu()))
+    finally:
+        c.close()
