@@ -236,6 +236,7 @@ constexpr int kRedBlocks = 8 * kNumSMs;
 template <typename T>
 __global__ void __launch_bounds__(256) partial_sum_kernel(const T *__restrict__ in, int64_t n, double *__restrict__ part)
 {
+    chain_begin();
     __shared__ double red[8];
     // Static contiguous chunk per CTA, a multiple of 4 elements: the
     // summation order is fixed.  16-byte loads when the array is 16-byte
@@ -287,6 +288,7 @@ constexpr int kFinalThreads = 1024;
 __global__ void __launch_bounds__(kFinalThreads)
 final_sum_kernel(const double *__restrict__ part, int np, double *__restrict__ out, double divisor)
 {
+    chain_begin();
     __shared__ double red[kFinalThreads / 32];
     double acc = 0.0;
     for (int i = threadIdx.x; i < np; i += kFinalThreads) acc += part[i];
@@ -304,6 +306,7 @@ final_sum_kernel(const double *__restrict__ part, int np, double *__restrict__ o
 
 __global__ void __launch_bounds__(256) publish_kernel(const __grid_constant__ Publish p, uint32_t *__restrict__ dst)
 {
+    chain_begin();
     for (int k = 0; k < p.n; ++k) {
         const uint32_t *src = static_cast<const uint32_t *>(p.seg[k].src);
         for (uint32_t i = threadIdx.x; i < p.seg[k].words; i += 256) dst[p.seg[k].at + i] = src[i];

@@ -96,6 +96,7 @@ count_kernel(const float *__restrict__ x, const float *__restrict__ y, const flo
              const float *__restrict__ w, int64_t np, unsigned chunk, const __grid_constant__ AssignGeom g, int nb,
              uint32_t *__restrict__ table, unsigned long long *__restrict__ lost, unsigned int *__restrict__ wstat)
 {
+    chain_begin();
     extern __shared__ uint32_t hist[];
     if (SMEM) {
         for (int i = threadIdx.x; i < nb; i += kBinThreads) hist[i] = 0u;
@@ -132,6 +133,7 @@ append_kernel(const float *__restrict__ x, const float *__restrict__ y, const fl
               uint32_t *__restrict__ table, uint4 *__restrict__ payload, unsigned long long *__restrict__ lost,
               unsigned int *__restrict__ wstat, uint64_t cap, unsigned int *__restrict__ ovf, uint32_t slab)
 {
+    chain_begin();
     unsigned int my_lost = 0;
     WeightStats ws;
     const bool weighted = w != nullptr;
@@ -355,6 +357,7 @@ template <int SCHEME, bool SLAB, int LEVEL>
 __global__ void __launch_bounds__(stage_threads(LEVEL), stage_ctas(LEVEL))
 sort_kernel(const __grid_constant__ SortArgs A, const __grid_constant__ AssignGeom g, const __grid_constant__ SuperGeom s)
 {
+    chain_begin();
     constexpr int NT = stage_threads(LEVEL);
     constexpr int MAXBINS = LEVEL == 0 ? kStageBins : (LEVEL == 1 ? kMaxSupers + 1 : kMaxLocal);
     constexpr int PER = (MAXBINS + NT - 1) / NT;
@@ -646,6 +649,7 @@ __global__ void __launch_bounds__(kBinThreads)
 super_count_kernel(const __grid_constant__ SortArgs A, const __grid_constant__ AssignGeom g,
                    const __grid_constant__ SuperGeom s, unsigned chunk)
 {
+    chain_begin();
     __shared__ uint32_t hist[kMaxSupers + 1];
     for (int i = threadIdx.x; i <= s.count; i += kBinThreads) hist[i] = 0u;
     __syncthreads();
@@ -666,6 +670,7 @@ super_count_kernel(const __grid_constant__ SortArgs A, const __grid_constant__ A
 __global__ void __launch_bounds__(1024)
 super_offsets_kernel(uint32_t *__restrict__ scursor, int count, uint32_t *__restrict__ beg, unsigned int *__restrict__ fullest)
 {
+    chain_begin();
     __shared__ uint32_t sums[32];
     const int k = threadIdx.x, lane = k & 31, wid = k >> 5;
     const uint32_t n = k <= count ? scursor[k] : 0u;
@@ -696,6 +701,7 @@ __global__ void __launch_bounds__(512, 2)
 super_tally_kernel(const __grid_constant__ SortArgs A, const __grid_constant__ AssignGeom g,
                    const __grid_constant__ SuperGeom s)
 {
+    chain_begin();
     constexpr int NT = 512;
     extern __shared__ __align__(16) unsigned char tally_smem[];
     __shared__ uint32_t warp_sums[32];
@@ -811,6 +817,7 @@ constexpr int kOffItems = 16;
 __global__ void __launch_bounds__(kOffThreads)
 brick_offsets_kernel(uint32_t *__restrict__ table, int stride, int nb, uint32_t *__restrict__ start, uint32_t *__restrict__ total)
 {
+    chain_begin();
     __shared__ uint32_t warp_sums[kOffThreads / 32];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int base = threadIdx.x * kOffItems;
@@ -860,6 +867,7 @@ brick_offsets_kernel(uint32_t *__restrict__ table, int stride, int nb, uint32_t 
 __global__ void __launch_bounds__(256)
 brick_max_kernel(const uint32_t *__restrict__ start, int nb, unsigned int *__restrict__ out)
 {
+    chain_begin();
     unsigned m = 0u;
     for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < nb; b += gridDim.x * blockDim.x)
         m = max(m, start[b + 1] - start[b]);
@@ -871,6 +879,7 @@ brick_max_kernel(const uint32_t *__restrict__ start, int nb, unsigned int *__res
 // counts[b] = table[b * stride] (contiguous, for the scan).
 __global__ void compact_counts_kernel(const uint32_t *__restrict__ table, int stride, int nb, uint32_t *__restrict__ counts)
 {
+    chain_begin();
     for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < nb; b += gridDim.x * blockDim.x)
         counts[b] = table[(int64_t)b * stride];
 }
@@ -881,6 +890,7 @@ __global__ void brick_starts_kernel(const uint32_t *__restrict__ scanned, int nb
                                     const uint32_t *__restrict__ total, uint32_t *__restrict__ start,
                                     uint32_t *__restrict__ cursor, int stride)
 {
+    chain_begin();
     for (int b = blockIdx.x * blockDim.x + threadIdx.x; b <= nb; b += gridDim.x * blockDim.x) {
         const uint32_t v = b < nb ? scanned[b] : *total;
         start[b] = v;
@@ -902,6 +912,7 @@ deposit_kernel(const uint4 *__restrict__ payload, const uint32_t *__restrict__ s
                OutT *__restrict__ mesh, double *__restrict__ brick_sum, uint32_t slab,
                const uint32_t *__restrict__ slab_count)
 {
+    chain_begin();
     extern __shared__ __align__(16) uint32_t tile32[];
     __shared__ long long red[kDepositThreads / 32];
     const int B = blockIdx.x;
@@ -949,6 +960,7 @@ __global__ void keys_kernel(const float *__restrict__ x, const float *__restrict
                             const float *__restrict__ z, int64_t np, AssignGeom g,
                             int64_t *__restrict__ keys)
 {
+    chain_begin();
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     const int64_t ncell = (int64_t)g.n[0] * g.n[1] * g.n[2];
     for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < np; p += stride) {

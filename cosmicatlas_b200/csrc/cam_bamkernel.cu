@@ -74,6 +74,7 @@ __global__ void __launch_bounds__(kBkThreads)
 bamk_update_kernel(T *__restrict__ K, int n, const double *__restrict__ weight, int nbins, int mode, T dk, T kmin,
                    T dK, int64_t rows_per_cta, double *__restrict__ part, unsigned long long *__restrict__ part_modes)
 {
+    chain_begin();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     double *wsum = reinterpret_cast<double *>(smem_raw);  // [warps][nbins]
     unsigned long long *wcnt = reinterpret_cast<unsigned long long *>(wsum + (size_t)kBkWarps * nbins);
@@ -155,6 +156,7 @@ __global__ void __launch_bounds__(256)
 bamk_final_kernel(const double *__restrict__ part, const unsigned long long *__restrict__ pm, int nparts, int nbins,
                   double *__restrict__ out, unsigned long long *__restrict__ modes)
 {
+    chain_begin();
     __shared__ double r0[256];
     __shared__ unsigned long long rc[256];
     const int bn = blockIdx.x;
@@ -187,6 +189,7 @@ template <typename T>
 __global__ void konvolve_mult_kernel(typename fftdev::CT<T>::t *__restrict__ main_, typename fftdev::CT<T>::t *__restrict__ nyq,
                                      const T *__restrict__ K, int n, const double *__restrict__ d_w, double s2)
 {
+    chain_begin();
     using C = typename fftdev::CT<T>::t;
     const int M = n / 2, L1 = M + 1;
     const T f = (T)(2.0 * (*d_w) * s2);

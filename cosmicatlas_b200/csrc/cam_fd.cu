@@ -33,6 +33,7 @@ template <typename T>
 __global__ void poisson_kernel(typename fftdev::CT<T>::t *__restrict__ main_, typename fftdev::CT<T>::t *__restrict__ nyq,
                                int n, double inv_kf2, double gcoef)
 {
+    chain_begin();
     using C = typename fftdev::CT<T>::t;
     const int M = n / 2, h = n / 2;
     const int64_t nmain = (int64_t)n * n * M, ntot = nmain + (int64_t)n * n;
@@ -74,6 +75,7 @@ __global__ void poisson_kernel(typename fftdev::CT<T>::t *__restrict__ main_, ty
 template <typename T>
 __global__ void gradfindif_kernel(const T *__restrict__ in, T *__restrict__ out, int n, int64_t stride, double ideltaH)
 {
+    chain_begin();
     const int z = blockIdx.y * blockDim.x + threadIdx.x;
     if (z >= n) return;
     const int64_t row = blockIdx.x;

@@ -55,6 +55,7 @@ __global__ void __launch_bounds__(1024, 1)
 fft_cols_kernel(typename fftdev::CT<T>::t *base, int len, int ncols, int64_t jstride, int64_t pstride,
                 int64_t ccomp, Radices rd, const typename fftdev::CT<T>::t *__restrict__ tw, int twmul)
 {
+    chain_begin();
     using C = typename fftdev::CT<T>::t;
     constexpr int W = fftdev::CT<T>::kCols;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -106,6 +107,7 @@ __global__ void __launch_bounds__(fftdev::ct_threads(LEN, fftdev::CT<T>::kCols, 
 fft_cols_pipe_kernel(typename fftdev::CT<T>::t *base, int nct, int nplanes, int64_t ntiles, int64_t jstride,
                      int64_t pstride, int64_t ccomp, const typename fftdev::CT<T>::t *__restrict__ tw)
 {
+    chain_begin();
     using C = typename fftdev::CT<T>::t;
     constexpr int W = fftdev::CT<T>::kCols;
     constexpr int NTHR = fftdev::ct_threads(LEN, W, fftdev::CT<T>::kPPT);
@@ -161,6 +163,7 @@ fft_cols_move_kernel(const typename fftdev::CT<T>::t *__restrict__ src, ColSide 
                      typename fftdev::CT<T>::t *__restrict__ dst, ColSide di, int ncols, int nct, int64_t ntiles,
                      const typename fftdev::CT<T>::t *__restrict__ tw)
 {
+    chain_begin();
     using C = typename fftdev::CT<T>::t;
     constexpr int W = fftdev::CT<T>::kCols;
     constexpr int NTHR = fftdev::ct_threads(LEN, W, fftdev::CT<T>::kPPT);
@@ -231,6 +234,7 @@ __global__ void __launch_bounds__(fftdev::ct_threads(LEN, fftdev::CT<T>::kCols, 
 fft_cols_tma_kernel(const __grid_constant__ CUtensorMap map, TileDims td, int nct, int nplanes, int64_t ntiles,
                     const typename fftdev::CT<T>::t *__restrict__ tw, unsigned *__restrict__ err)
 {
+    chain_begin();
     using C = typename fftdev::CT<T>::t;
     constexpr int W = fftdev::CT<T>::kCols;
     constexpr int NTHR = fftdev::ct_threads(LEN, W, fftdev::CT<T>::kPPT);
@@ -359,6 +363,7 @@ fft_cols_tma_pk_kernel(const __grid_constant__ CUtensorMap map, TileDims td, int
                        const short *__restrict__ btab /* bin of q = |k|^2 / k_f^2 */, int store,
                        double *__restrict__ part /* [grid][nbins] */)
 {
+    chain_begin();
     using C = float2;
     constexpr int W = pk_pass_cols<LEN>();
     constexpr int RPW = 32 / W;  // rows a warp bins at a time
@@ -556,6 +561,7 @@ fft_rows_kernel(const void *in, void *out_main, typename fftdev::CT<T>::t *nyq, 
                 const typename fftdev::CT<T>::t *__restrict__ tw, const double *__restrict__ d_sub,
                 double scale)
 {
+    chain_begin();
     using C = typename fftdev::CT<T>::t;
     constexpr bool INV = (MODE == 1 || MODE == 3);
     constexpr bool PAD = LEN > 0;  // row tiles of the compile-time transforms are padded
@@ -661,6 +667,7 @@ fft_rows_r2c_pipe_kernel(const T *__restrict__ in, typename fftdev::CT<T>::t *__
                          typename fftdev::CT<T>::t *__restrict__ nyq, int64_t nrows,
                          const typename fftdev::CT<T>::t *__restrict__ tw, const double *__restrict__ d_sub)
 {
+    chain_begin();
     using C = typename fftdev::CT<T>::t;
     constexpr int M = LEN;
     constexpr int RPC = rows_rpc<T>(LEN);
@@ -712,6 +719,7 @@ __global__ void split_to_fftw_kernel(const typename fftdev::CT<T>::t *__restrict
                                      const typename fftdev::CT<T>::t *__restrict__ nyq,
                                      typename fftdev::CT<T>::t *__restrict__ dst, int64_t nrows, int M)
 {
+    chain_begin();
     const int64_t tot = nrows * (M + 1);
     for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < tot;
          e += (int64_t)gridDim.x * blockDim.x) {
@@ -726,6 +734,7 @@ __global__ void fftw_to_split_kernel(const typename fftdev::CT<T>::t *__restrict
                                      typename fftdev::CT<T>::t *__restrict__ main,
                                      typename fftdev::CT<T>::t *__restrict__ nyq, int64_t nrows, int M)
 {
+    chain_begin();
     const int64_t tot = nrows * (M + 1);
     for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < tot;
          e += (int64_t)gridDim.x * blockDim.x) {

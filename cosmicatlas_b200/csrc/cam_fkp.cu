@@ -24,6 +24,7 @@ __global__ void __launch_bounds__(kFkpThreads)
 fkp_weights_kernel(int64_t n, const float *__restrict__ nbar, double nbar_const, const float *__restrict__ w_in,
                    int fkp, double pest, float *__restrict__ w_out, double *__restrict__ part /* [grid][3] */)
 {
+    chain_begin();
     __shared__ double red[3][kFkpThreads];
     double sw = 0.0, sw2 = 0.0, snw2 = 0.0;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
@@ -50,6 +51,7 @@ fkp_weights_kernel(int64_t n, const float *__restrict__ nbar, double nbar_const,
 __global__ void __launch_bounds__(kFkpThreads)
 fkp_final_kernel(const double *__restrict__ part, int nparts, double *__restrict__ out /* [3] */)
 {
+    chain_begin();
     __shared__ double red[3][kFkpThreads];
     double s[3] = {0.0, 0.0, 0.0};
     for (int p = threadIdx.x; p < nparts; p += blockDim.x)

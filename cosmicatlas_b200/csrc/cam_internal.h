@@ -9,6 +9,7 @@
 #include <map>
 #include <mutex>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "../../include/cam.h"
@@ -38,18 +39,16 @@ struct Error {
 
 // Kernel launch with error check, launch accounting and (when enabled)
 // CUDA-event timing per kernel name.
-#define CAM_LAUNCH_NAMED(ctx, name, kernel, grid, block, smem, ...)                 \
-    do {                                                                            \
-        ::cam::prof_begin((ctx), (name));                                           \
-        kernel<<<(grid), (block), (smem), (ctx)->stream>>>(__VA_ARGS__);            \
-        {                                                                           \
-            const cudaError_t _le = cudaGetLastError();                             \
-            if (_le != cudaSuccess)                                                 \
-                throw ::cam::Error{CAM_E_CUDA, std::string("launch of ") + (name) + \
-                                                   ": " + cudaGetErrorString(_le)}; \
-        }                                                                           \
-        ::cam::prof_end(ctx);                                                       \
-        (ctx)->launches++;                                                          \
+#define CAM_LAUNCH_NAMED(ctx, name, kernel, grid, block, smem, ...)                           \
+    do {                                                                                      \
+        ::cam::prof_begin((ctx), (name));                                                     \
+        const cudaError_t _le = ::cam::launch_chained((ctx), kernel, dim3(grid), dim3(block), \
+                                                      (size_t)(smem), __VA_ARGS__);           \
+        if (_le != cudaSuccess)                                                               \
+            throw ::cam::Error{CAM_E_CUDA, std::string("launch of ") + (name) +               \
+                                               ": " + cudaGetErrorString(_le)};               \
+        ::cam::prof_end(ctx);                                                                 \
+        (ctx)->launches++;                                                                    \
     } while (0)
 #define CAM_LAUNCH(ctx, kernel, grid, block, smem, ...) \
     CAM_LAUNCH_NAMED(ctx, #kernel, kernel, grid, block, smem, __VA_ARGS__)
@@ -125,6 +124,38 @@ namespace cam {
 
 void prof_begin(cam_ctx *ctx, const char *name);
 void prof_end(cam_ctx *ctx);
+
+// First statement of every kernel launched by CAM_LAUNCH: wait until the
+// stream's previous kernel is complete and its writes are seen (at once for a
+// launch that was not chained), then let the next one's CTAs start.  A kernel
+// that left the wait out could overtake the one before the last.
+__device__ __forceinline__ void chain_begin()
+{
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+// A launch whose CTAs may take their places while the stream's previous
+// kernel runs its last ones (programmatic stream serialisation).  Not for
+// batches, whose jobs fill each other's gaps and need those places, nor on
+// the side stream, nor while kernels are timed one by one.
+template <typename... P, typename... A>
+cudaError_t launch_chained(cam_ctx *ctx, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, A &&...args)
+{
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = ctx->stream;
+    cfg.attrs = &at;
+    cfg.numAttrs = !ctx->sync_free && !ctx->capturing && !ctx->prof_on && ctx->stream != ctx->aux_stream;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
+    if (e != cudaSuccess) cudaGetLastError();
+    return e;
+}
 
 // Forks the side stream from the context's stream (the side stream then
 // runs after everything enqueued so far) and returns it; aux_join makes the

@@ -58,6 +58,7 @@ pk_bin_kernel(const C *__restrict__ main, const C *__restrict__ nyq, const C *__
               double *__restrict__ part /* [grid][nbins][2] */,
               unsigned long long *__restrict__ part_modes /* [grid][nbins] */)
 {
+    chain_begin();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int h = n / 2;
     const int M = h;
@@ -271,6 +272,7 @@ __global__ void __launch_bounds__(256)
 pk_final_kernel(const double *__restrict__ part, const unsigned long long *__restrict__ pm, int nparts,
                 int nbins, double *__restrict__ out /* [nbins][2] */, unsigned long long *__restrict__ modes)
 {
+    chain_begin();
     __shared__ double r0[256], r1[256];
     __shared__ unsigned long long rc[256];
     const int bn = blockIdx.x;
@@ -375,6 +377,7 @@ namespace {
 __global__ void pk_bintab_kernel(const double *__restrict__ E2, int nbins, float m_u, float inv_s, int qmax,
                                  short *__restrict__ out)
 {
+    chain_begin();
     for (int q = blockIdx.x * blockDim.x + threadIdx.x; q <= qmax; q += gridDim.x * blockDim.x)
         out[q] = (short)pk_bin((double)q, E2, nbins, m_u, inv_s);
 }
@@ -440,6 +443,7 @@ __global__ void __launch_bounds__(kNyqThreads)
 pk_nyq_kernel(const float2 *__restrict__ nyq, int n, const double *__restrict__ g_tab, int nbins,
               const short *__restrict__ btab, double *__restrict__ part)
 {
+    chain_begin();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int h = n / 2;
     double *tw2 = reinterpret_cast<double *>(smem_raw);  // [h+1]
@@ -491,6 +495,7 @@ pk_final_fused_kernel(const double *__restrict__ part, int nparts, int nbins, co
                       const unsigned long long *__restrict__ stat_modes, double *__restrict__ out,
                       unsigned long long *__restrict__ modes)
 {
+    chain_begin();
     __shared__ double r0[256];
     const int bn = blockIdx.x;
     double s0 = 0.0;

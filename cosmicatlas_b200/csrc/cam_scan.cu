@@ -45,6 +45,7 @@ __device__ __forceinline__ uint32_t block_exclusive(uint32_t v, uint32_t *warp_s
 __global__ void __launch_bounds__(kScanThreads) tile_sum_kernel(const uint32_t *__restrict__ in, int64_t n,
                                                                 uint32_t *__restrict__ sums)
 {
+    chain_begin();
     __shared__ uint32_t red[32];
     const int64_t base = (int64_t)blockIdx.x * kScanTile;
     uint32_t s = 0;
@@ -67,6 +68,7 @@ __global__ void __launch_bounds__(kScanThreads) tile_sum_kernel(const uint32_t *
 // Exclusive scan of the tile sums (one CTA, any count); sums[ntiles] = total.
 __global__ void __launch_bounds__(kScanThreads) tile_offsets_kernel(uint32_t *__restrict__ sums, int ntiles)
 {
+    chain_begin();
     __shared__ uint32_t warp_sums[32];
     __shared__ uint32_t tot;
     uint32_t carry = 0;
@@ -85,6 +87,7 @@ __global__ void __launch_bounds__(kScanThreads) tile_offsets_kernel(uint32_t *__
 __global__ void __launch_bounds__(kScanThreads) tile_scan_kernel(uint32_t *__restrict__ data, int64_t n,
                                                                  const uint32_t *__restrict__ offsets)
 {
+    chain_begin();
     __shared__ uint32_t warp_sums[32];
     __shared__ uint32_t tot;
     const int64_t base = (int64_t)blockIdx.x * kScanTile + (int64_t)threadIdx.x * kScanItems;

@@ -134,6 +134,7 @@ tidal_x_kernel(const typename CTw<T>::t *__restrict__ src, typename CTw<T>::t *_
                const typename CTw<T>::t *__restrict__ tw, double gauss_coef, const double *__restrict__ d_mean,
                int density_input, double scale, const typename CTw<T>::t *__restrict__ sf, int pot)
 {
+    chain_begin();
     using C = typename CTw<T>::t;
     constexpr int W = CTw<T>::kCols;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -191,6 +192,7 @@ tidal_y_kernel(typename CTw<T>::t *__restrict__ base, int n, int ncols, int64_t 
                int64_t pstride, int64_t ccomp, Radices rd, const typename CTw<T>::t *__restrict__ tw, int kz_fixed,
                const typename CTw<T>::t *__restrict__ sf)
 {
+    chain_begin();
     using C = typename CTw<T>::t;
     constexpr int W = CTw<T>::kCols;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -280,6 +282,7 @@ tidal_pipe_kernel(const typename CTw<T>::t *src, typename CTw<T>::t *dst, int n,
                   double gauss_coef, const double *__restrict__ d_mean, int density_input, double scale,
                   const typename CTw<T>::t *__restrict__ sf, int pot)
 {
+    chain_begin();
     using C = typename CTw<T>::t;
     constexpr int W = tpipe_cols<T, LEN>();
     constexpr int NTHR = tpipe_threads<T, LEN>();
@@ -691,6 +694,7 @@ tidal_z_kernel(const typename CTw<T>::t *__restrict__ src, const typename CTw<T>
                uint8_t *__restrict__ labels, float *__restrict__ lambdas, float *__restrict__ inv,
                unsigned long long *__restrict__ counts /* [5] */)
 {
+    chain_begin();
     using C = typename CTw<T>::t;
     constexpr bool PAD = LEN > 0;  // row tiles of the compile-time transforms are padded
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -827,6 +831,7 @@ tidal_z_pipe_kernel(const typename CTw<T>::t *__restrict__ src, const typename C
                     uint8_t *__restrict__ labels, float *__restrict__ lambdas, float *__restrict__ inv,
                     unsigned long long *__restrict__ counts /* [5] */)
 {
+    chain_begin();
     using C = typename CTw<T>::t;
     constexpr int M = LEN;
     constexpr int RPC = tweb_rpc<T>(LEN);
@@ -928,6 +933,7 @@ tidal_z_pipe_kernel(const typename CTw<T>::t *__restrict__ src, const typename C
 template <typename T>
 __global__ void fd_table_kernel(typename CTw<T>::t *__restrict__ sf, int n)
 {
+    chain_begin();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i > n) return;
     const double t = 2.0 * (double)(i - n / 2) / (double)n;  // sinpi(t) = sin(2 pi f / N)
