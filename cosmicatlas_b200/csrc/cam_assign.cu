@@ -991,6 +991,7 @@ AssignGeom make_geom(const cam_grid &gr, int scheme, int64_t np)
         g.L[a] = gr.L[a];
         g.d[a] = gr.d[a] != 0.f ? gr.d[a] : gr.L[a] / (float)gr.n[a];
         g.mn[a] = gr.min[a];
+        g.origin |= g.mn[a] != 0.0f;
         CAM_REQUIRE(std::isfinite(g.d[a]) && g.d[a] > 0.f, CAM_E_INVAL, "cell size must be > 0");
         CAM_REQUIRE(std::isfinite(g.mn[a]), CAM_E_INVAL, "box origin must be finite");
     }
@@ -1020,7 +1021,6 @@ AssignGeom make_geom(const cam_grid &gr, int scheme, int64_t np)
         g.nf[a] = (float)g.n[a];
         g.half_d[a] = 0.5f * g.d[a];
         g.off_scale[a] = g.inv_d[a] * 16777216.0f;
-        g.origin |= g.mn[a] != 0.0f;
         // an axis that one brick spans: brick 0 always, nothing crosses
         const bool whole = g.nb[a] == 1;
         const int reach = scheme == CAM_TSC ? 2 : 1;  // from the stencil's first to its last cell
@@ -1036,8 +1036,14 @@ AssignGeom make_geom(const cam_grid &gr, int scheme, int64_t np)
         const float thr = 4.2e-7f * (float)(g.n[a] + 1) + 1e-6f;
         const double end = (double)(g.mn[a] + g.L[a]) - (double)g.mn[a];
         const double nd = (double)g.n[a] * (double)g.d[a];
+        // How far n * d may be off L.  Without an origin locate() puts a CIC
+        // position v in [-d, 0) into cell n - 1, the reference into the cell
+        // of v + L: the same one if n - L / d is below thr less the roundings
+        // of v + L and of its quotient (1.2e-7 n cells); d = L / n rounded is
+        // off by 6e-8 n cells.  Nothing else here depends on n * d being L.
+        const double off = scheme == CAM_CIC && !g.origin ? 0.5 * thr : 1e-3 * std::max(1.0, 1e-3 * g.n[a]);
         const bool regular = g.n[a] >= 4 && std::isfinite(g.off_scale[a]) && std::isnormal(g.inv_d[a]) && ((double)g.n[a] - thr) * g.d[a] * (1.0 + 3e-7) < end &&
-                             std::fabs(nd - (double)g.L[a]) <= 1e-3 * g.d[a] * std::max(1.0, 1e-3 * g.n[a]);
+                             std::fabs(nd - (double)g.L[a]) <= off * g.d[a];
         g.safe[a] = regular ? 0.5f - thr : -1.0f;
     }
     for (int a = 0; a < 2; ++a)

@@ -381,3 +381,25 @@ def test_many_super_bricks_too_clumped_for_slabs(scheme):
         assert np.array_equal(np.asarray(first.mesh.cpu()), np.asarray(again.mesh.cpu()))
     finally:
         c.close()
+
+
+@pytest.mark.parametrize("mn", [0.0, 12.5])
+@pytest.mark.parametrize("n,box,d", [(256, 505.0, 1.97265), (256, 505.0, 1.97266), (64, 1000.0, 15.62494),
+                                     (64, 1000.0, 15.62506), (130, 777.7, 5.98232)])
+def test_cell_size_off_box_over_cells(ctx, n, box, d, mn):
+    # a cell size of one to four parts in 10^6 off L/N, as a caller that
+    # rounds it passes: positions in and around the first and the last half
+    # cell, where CIC takes periodic images, and anywhere
+    f = np.float32
+    rng = np.random.default_rng(n)
+    edge = np.concatenate([rng.uniform(0.0, 1.0, 20_000), 0.5 + rng.uniform(-2e-3, 2e-3, 20_000),
+                           n + rng.uniform(-1.0, 0.0, 20_000), n - 0.5 + rng.uniform(-2e-3, 2e-3, 20_000)]) * d
+    x = (np.concatenate([edge, rng.uniform(0.0, box, 40_000)]) + mn).astype(f)
+    y, z = (rng.permutation(x) for _ in range(2))
+    g = make_grid(n, box, d, mn)
+    og = orc.Grid((n,) * 3, (box,) * 3, tuple(g.d), (mn,) * 3)
+    for s in SCHEMES:
+        a = ctx.assign(x, y, z, None, g, s, F64)
+        ref, lost = orc.assign_f64_mt(s, x, y, z, None, og)
+        assert a.n_lost == lost
+        assert rel_err_cells(a.mesh, ref, 1.0) <= 1e-5
