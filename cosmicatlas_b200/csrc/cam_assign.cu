@@ -1011,10 +1011,21 @@ AssignGeom make_geom(const cam_grid &gr, int scheme, int64_t np)
         if (g.b[0] >= g.b[1] && g.b[0] > 4) g.b[0] = (g.b[0] + 1) / 2;
         else g.b[1] = (g.b[1] + 1) / 2;
     }
-    // A stencil of width <= 3 must never span three bricks: a partial last
-    // brick keeps at least 2 cells (shrink the brick until it does).
+    // A stencil of three cells must never span three bricks (its particle has
+    // records in two at most along an axis): a partial last brick keeps at
+    // least 2 cells.  The extent shrinks until it does, or grows where no
+    // smaller one leaves 0 or 2 (N = 13, 25, 37, 49, 61, ..., when many
+    // particles had made the bricks 4 or 3 cells).
+    constexpr int largest[3] = {16, 16, 32};
     for (int a = 0; a < 3; ++a) {
-        while (g.b[a] < g.n[a] && g.n[a] % g.b[a] != 0 && g.n[a] % g.b[a] < 2 && g.b[a] > 3) --g.b[a];
+        auto one_left = [&](int b) { return b < g.n[a] && g.n[a] % b == 1; };
+        int b = g.b[a];
+        while (one_left(b) && b > 3) --b;
+        if (one_left(b))
+            for (b = g.b[a]; one_left(b) && b < largest[a];) ++b;
+        CAM_REQUIRE(scheme != CAM_TSC || !one_left(b), CAM_E_UNSUPPORTED,
+                    "no brick extent leaves a TSC stencil within two bricks");  // N = 720721 alone
+        g.b[a] = b;
         g.nb[a] = (g.n[a] + g.b[a] - 1) / g.b[a];
         g.inv_d[a] = 1.0f / g.d[a];
         g.e_last[a] = g.n[a] - (g.nb[a] - 1) * g.b[a];

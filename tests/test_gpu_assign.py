@@ -403,3 +403,22 @@ def test_cell_size_off_box_over_cells(ctx, n, box, d, mn):
         ref, lost = orc.assign_f64_mt(s, x, y, z, None, og)
         assert a.n_lost == lost
         assert rel_err_cells(a.mesh, ref, 1.0) <= 1e-5
+
+
+@pytest.mark.parametrize("scheme", SCHEMES)
+@pytest.mark.parametrize("n", [(61, 61, 61), (49, 49, 49), (13, 25, 64), (37, 10, 33), (85, 73, 31)])
+def test_small_bricks_with_one_cell_left(ctx, scheme, n):
+    # particles enough to make the bricks 4 or 3 cells along axes that either
+    # leaves one cell of: a TSC stencil would span three bricks there
+    box = 1000.0
+    npart = 1_300_000
+    rng = np.random.default_rng(n[0])
+    x, y, z = (rng.uniform(0.0, box, npart).astype(np.float32) for _ in range(3))
+    x[:npart // 4] *= np.float32(0.02)  # and the cells beside the box face
+    y[npart // 8:npart // 2] = np.float32(box) - y[npart // 8:npart // 2] * np.float32(0.03)
+    g = make_grid(n, box)
+    r = ctx.assign(x, y, z, None, g, scheme, F64)
+    ref, lost = orc.assign_f64_mt(scheme, x, y, z, None, orc.Grid(n, (box,) * 3, tuple(g.d), (0.0,) * 3))
+    assert r.n_lost == lost
+    assert abs(r.sum_mesh - (npart - lost)) <= 1e-9 * npart
+    assert rel_err_cells(r.mesh, ref, 1.0) <= 1e-5
