@@ -267,3 +267,29 @@ def test_job_pk_binned_in_fft_equals_separate_binning(ctx, scheme, n, nbins, nde
     # and with the T-web, where the x pass also writes the spectrum back
     job2 = ctx.job(x, y, z, None, g, scheme, F32, pk=opts, tweb=Context.tweb_opts(8.0, 0.0, 1e-5))
     assert np.array_equal(job2["pk"].pk, job["pk"].pk)
+
+
+@pytest.mark.parametrize("n", [32, 64, 256])
+def test_job_pk_rows_of_opposite_kx_enter_fp64_apart(ctx, n):
+    # Two waves of period 4 along every axis, (k, k, k) and (-k, k, k) with
+    # k = n/4, the second 2^-13 as high: every value of the mesh and of its
+    # transform is an integer multiple of a power of two within 24 bits, so
+    # the spectrum is exact.  Both fall into one bin, from rows i and n - i of
+    # one plane; their powers are 1 to 2^-26, so an FP32 sum of the two rows
+    # loses the second and the FP64 bin does not.
+    i = np.arange(n, dtype=np.int64)
+    ijk = i[:, None, None], i[None, :, None], i[None, None, :]
+    cos4 = np.array([1.0, 0.0, -1.0, 0.0])
+    one = cos4[(ijk[0] + ijk[1] + ijk[2]) % 4]
+    two = cos4[(-ijk[0] + ijk[1] + ijk[2]) % 4] * 2.0 ** -13
+    pos = [np.ascontiguousarray(np.broadcast_to(a + 0.5, (n,) * 3).reshape(-1), dtype=np.float32) for a in ijk]
+    opts = Context.pk_opts(NGP, nbins=n // 2, mas_correction=False, sn_correction=False, input_type=1)
+
+    def power(mesh):
+        w = mesh.reshape(-1).astype(np.float32)
+        return ctx.job(*pos, w, make_grid(n, float(n)), NGP, F32, pk=opts)["pk"].pk
+
+    a, b, both = power(one), power(two), power(one + two)
+    k = int(np.argmax(a))
+    assert k == int(n / 4 * 3 ** 0.5) and b[k] == a[k] * 2.0 ** -26
+    assert abs(both[k] - (a[k] + b[k])) <= 1e-12 * a[k]
