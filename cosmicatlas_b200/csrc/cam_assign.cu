@@ -931,6 +931,10 @@ deposit_kernel(const uint4 *__restrict__ payload, const uint32_t *__restrict__ s
     const uint32_t end = slab ? beg + min(slab_count[(int64_t)B * g.cstride], slab) : min(start[B + 1], nrec);
     RecordStream rec;
     rec.open(payload, beg, end, warp, kDepositThreads / 32, lane);
+    // a weight that is not finite, or records that found no room (the call
+    // fails, or runs again exactly): the mesh, which may be the caller's, is
+    // left as it is
+    if ((weighted && wstat[0] >= 0x7f800000u) || wstat[4] != 0u) return;
     const bool nonneg = !weighted || wstat[1] == 0u;
     const int s = fixed_scale(wstat, weighted, end - beg);
     // 2^s as two exact factors (s may exceed the float exponent range)

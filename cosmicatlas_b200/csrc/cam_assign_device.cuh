@@ -643,6 +643,7 @@ __device__ __forceinline__ long long store_tile(const uint32_t *tile, const int 
 // 2^62.  Unit weights use s = 30; NGP counts convert by a shift.
 // wstat[0] = bits of max |w|, wstat[1] != 0 if some weight is negative,
 // wstat[6] = 0x7fffffff - bits of min nonzero |w| (0: no nonzero weight).
+// wstat[4] != 0 (deposit_kernel only): some records were not written.
 __device__ __forceinline__ int fixed_scale(const unsigned int *wstat, int weighted, uint32_t nrec)
 {
     float wmax = 1.0f, wmin = 1.0f;

@@ -422,3 +422,33 @@ def test_small_bricks_with_one_cell_left(ctx, scheme, n):
     assert r.n_lost == lost
     assert abs(r.sum_mesh - (npart - lost)) <= 1e-9 * npart
     assert rel_err_cells(r.mesh, ref, 1.0) <= 1e-5
+
+
+@pytest.mark.parametrize("n,npart", [(64, 200_000), (416, 1_200_000)])
+@pytest.mark.parametrize("bad", [np.inf, np.nan])
+def test_nonfinite_weight_leaves_the_mesh(n, npart, bad):
+    # the caller's device mesh is not written before the weights are refused:
+    # exact and slab runs, one and two levels, with and without an overflow
+    import torch
+    from cosmicatlas_b200.api import Context
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    xs = [torch.rand(npart, device="cuda", generator=gen) * 100.0 for _ in range(3)]
+    w = torch.ones(npart, device="cuda")
+    wrong = w.clone()
+    wrong[npart // 2] = float(bad)
+    clumped = [v * 0.1 for v in xs]
+    c = Context()
+    try:
+        g = make_grid(n, 100.0)
+        mesh = torch.full((n, n, n), -7.0, device="cuda")
+        for pos in (xs, xs, clumped):
+            with pytest.raises(CamError) as e:
+                c.assign(*pos, wrong, g, CIC, F32, out=mesh)
+            assert e.value.code == -8
+            assert bool((mesh == -7.0).all())
+            if pos is xs:
+                c.assign(*xs, w, g, CIC, F32)  # measures the slabs of the calls after it
+        c.assign(*xs, w, g, CIC, F32, out=mesh)
+        assert abs(float(mesh.double().sum()) - npart) <= 1e-5 * npart
+    finally:
+        c.close()
