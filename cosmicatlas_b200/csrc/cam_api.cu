@@ -1192,9 +1192,9 @@ int cam_job_run(cam_ctx *ctx, const cam_job_desc *job, cam_job_result *res)
         FftPlan *plan = get_plan(ctx, n, job->precision);
         const int nb = want_pk ? nbins_for(job->pk, n) : 0;
         // Readback of one run into pinned memory: assignment statistics [8],
-        // T-web counters [8], mesh sum and mean [2], the error word, P(k)
-        // sums [nb][2] and modes [nb].
-        constexpr size_t kTw = 64, kSum = 128, kErr = 144, kPk = 160;
+        // T-web counters [8], mesh sum and mean [2], the error word, the
+        // deposit's overflow word, P(k) sums [nb][2] and modes [nb].
+        constexpr size_t kTw = 64, kSum = 128, kErr = 144, kOvf = 148, kPk = 160;
         unsigned char *pin = pinned(ctx, kPk + (size_t)nb * 24);
         const auto *hstats = reinterpret_cast<const unsigned long long *>(pin);
         const auto *htw = reinterpret_cast<const unsigned long long *>(pin + kTw);
@@ -1213,6 +1213,9 @@ int cam_job_run(cam_ctx *ctx, const cam_job_desc *job, cam_job_result *res)
             auto *dsum = static_cast<double *>(scratch(ctx, "job.sum", 2 * sizeof(double)));
             out.d_sum = dsum;
             out.defer = defer;
+            volatile unsigned *const ovf = reinterpret_cast<volatile unsigned *>(pin + kOvf);
+            *ovf = 0u;
+            out.host_ovf = const_cast<unsigned *>(ovf);
             assign_device(ctx, d.x, d.y, d.z, d.w, d.n, g, job->scheme, out);
             // FFT of rho - mean, mean from the deposit's exact per-brick sums.
             Spectrum s = alloc_spectrum(ctx, n, job->precision, "job.spec");
@@ -1220,6 +1223,14 @@ int cam_job_run(cam_ctx *ctx, const cam_job_desc *job, cam_job_result *res)
                                             job->want_tweb != 0);
             uint8_t *dl = nullptr;
             if (job->want_tweb) {
+                // No T-web (half of a large job) of a mesh that fell short.
+                // The transform forked the side stream behind the assignment
+                // and its row pass; what follows that runs while the host
+                // waits and enqueues the T-web.
+                if (defer) {
+                    CAM_CUDA_TRY(cudaEventSynchronize(ctx->ev_fork));
+                    if (*ovf) return true;
+                }
                 if (res->labels) dl = static_cast<uint8_t *>(scratch(ctx, "tw.labels", ncell));
                 tweb_device(ctx, plan, s, g.L[0], dsum + 1, job->tweb.input_type, job->tweb, dl, nullptr, nullptr, nullptr,
                             job_tweb_counts(ctx));

@@ -910,7 +910,7 @@ __global__ void __launch_bounds__(kDepositThreads, 2)
 deposit_kernel(const uint4 *__restrict__ payload, const uint32_t *__restrict__ start, uint32_t nrec,
                AssignGeom g, const unsigned int *__restrict__ wstat, int weighted,
                OutT *__restrict__ mesh, double *__restrict__ brick_sum, uint32_t slab,
-               const uint32_t *__restrict__ slab_count)
+               const uint32_t *__restrict__ slab_count, unsigned int *__restrict__ host_ovf)
 {
     chain_begin();
     extern __shared__ __align__(16) uint32_t tile32[];
@@ -934,7 +934,10 @@ deposit_kernel(const uint4 *__restrict__ payload, const uint32_t *__restrict__ s
     // a weight that is not finite, or records that found no room (the call
     // fails, or runs again exactly): the mesh, which may be the caller's, is
     // left as it is
-    if ((weighted && wstat[0] >= 0x7f800000u) || wstat[4] != 0u) return;
+    if ((weighted && wstat[0] >= 0x7f800000u) || wstat[4] != 0u) {
+        if (host_ovf && blockIdx.x == 0 && threadIdx.x == 0 && wstat[4] != 0u) *host_ovf = 1u;
+        return;
+    }
     const bool nonneg = !weighted || wstat[1] == 0u;
     const int s = fixed_scale(wstat, weighted, end - beg);
     // 2^s as two exact factors (s may exceed the float exponent range)
@@ -1352,7 +1355,7 @@ static void assign_impl(cam_ctx *ctx, const float *x, const float *y, const floa
         smem_at_least(kern, smem);
         CAM_LAUNCH_NAMED(ctx, "assign_deposit", kern, (unsigned)nb, kDepositThreads, smem, payload, start,
                          (uint32_t)std::min<uint64_t>(total, 0xffffffffull), g, d_wmax, weighted, mesh, bsum, slab,
-                         table);
+                         table, out.host_ovf);
     };
     if (out.precision == CAM_F32)
         launch_dep(deposit_kernel<SCHEME, float>, static_cast<float *>(out.mesh));

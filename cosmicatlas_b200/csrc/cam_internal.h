@@ -158,7 +158,8 @@ cudaError_t launch_chained(cam_ctx *ctx, void (*kernel)(P...), dim3 grid, dim3 b
 }
 
 // Forks the side stream from the context's stream (the side stream then
-// runs after everything enqueued so far) and returns it; aux_join makes the
+// runs after everything enqueued so far, which ctx->ev_fork, recorded here,
+// marks the end of) and returns it; aux_join makes the
 // context's stream wait for everything enqueued on the side stream since.
 // Both are plain event record / wait, so they also work under stream
 // capture.
@@ -244,6 +245,10 @@ struct AssignOut {
     // written and raise the overflow word of the device statistics, in
     // which case the caller reruns without defer.  n_in / n_lost are -1.
     bool defer = false;
+    // A word of pinned host memory (may be null) that the deposit sets if
+    // records were not written: there for a host that waits for an event
+    // behind the assignment, before the statistics are published.
+    unsigned int *host_ovf = nullptr;
     // Set by exact (non-slab) runs: the records a brick of a uniform
     // catalogue expects, and (without defer) the fullest brick's records;
     // with defer the fullest brick is word [5] of the device statistics.

@@ -256,3 +256,38 @@ def test_two_level_slabs_overflow_reruns(scheme):
         # NGP loses the positions that round to the box side
         assert r["assign"].n_lost == fresh["assign"].n_lost
         assert r["assign"].sum_mesh == fresh["assign"].sum_mesh
+
+
+@pytest.mark.parametrize("n,prec", [(64, F32), (54, F32), (128, F64)])
+@pytest.mark.parametrize("want_pk", [True, False])
+def test_job_that_runs_again_makes_one_tweb(n, prec, want_pk):
+    # slabs sized by a uniform catalogue, then a clumped one that they do not
+    # hold: the job runs again from the assignment on, its T-web runs once
+    box, npart = 10.0 * n, 150_000
+    rng = np.random.default_rng(n)
+    even = [rng.uniform(0.0, box, npart).astype(np.float32) for _ in range(3)]
+    clumped = [np.concatenate([v[:npart // 2], v[npart // 2:] * np.float32(0.04)]) for v in even]
+    pk = Context.pk_opts(CIC, nbins=n // 2) if want_pk else None
+    args = (None, make_grid(n, box), CIC, prec)
+    kw = dict(pk=pk, tweb=Context.tweb_opts(8.0, 0.0, BAND), want_labels=True)
+    fresh = Context(0)
+    try:
+        want = fresh.job(*clumped, *args, **kw)
+    finally:
+        fresh.close()
+    c = Context(0)
+    try:
+        for _ in range(2):
+            c.job(*even, *args, **kw)
+        c.profile(True)
+        c.profile_read(True)
+        got = c.job(*clumped, *args, **kw)
+        launches = {k: v[0] for k, v in c.profile_read(True).items()}
+    finally:
+        c.close()
+    assert launches["assign_deposit"] == 2
+    assert launches["tweb_tidal_z_eigen"] == 1
+    assert np.array_equal(got["tweb"].labels, want["tweb"].labels)
+    assert np.array_equal(got["tweb"].counts, want["tweb"].counts)
+    if want_pk:
+        assert np.array_equal(got["pk"].pk, want["pk"].pk)
