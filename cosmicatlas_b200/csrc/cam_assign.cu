@@ -1147,7 +1147,7 @@ static void assign_impl(cam_ctx *ctx, const float *x, const float *y, const floa
     // budget was sized for; nor do slabs take more than a quarter of the
     // device's memory, or sorted particles a sixteenth.
     const double est_brick = (double)np * f / (double)nb;
-    const int64_t shape = ((int64_t)g.n[0] << 32) | ((int64_t)g.n[1] << 16) | (int64_t)g.n[2];
+    const AssignShape shape{g.n[0], g.n[1], g.n[2], g.b[0], g.b[1], g.b[2], SCHEME};
     double est_super = (double)np;
     for (int a = 0; a < 3 && sg.count > 0; ++a)
         est_super *= (double)std::min(sg.gs[a] * g.b[a], g.n[a]) / (double)g.n[a];

@@ -6,6 +6,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <array>
 #include <map>
 #include <mutex>
 #include <string>
@@ -62,6 +63,10 @@ struct DevBuf {
 
 struct FftPlan;  // cam_fft.cu
 
+// What the clumping of a catalogue was measured on: mesh sides, brick extents
+// (they depend on the number of particles) and scheme.
+using AssignShape = std::array<int64_t, 7>;
+
 struct ProfRecord {
     const char *name;
     cudaEvent_t start, stop;
@@ -93,7 +98,7 @@ struct cam_ctx {
     bool sync_free = false;
     bool capturing = false;  // inside stream capture: no allocation, no events
     uint64_t asg_cap = 0;    // payload records of deferred assignments (grow-only)
-    // Slabs of deferred assignments (cam_job_run), per mesh shape: the
+    // Slabs of deferred assignments, per mesh shape: the
     // fullest brick's expected records over those of a uniform catalogue,
     // as the last exact job run of that shape measured them (Poisson noise
     // taken out).  No entry until a job of the shape has run exactly.
@@ -101,7 +106,7 @@ struct cam_ctx {
     // admission budgets the exact payload); so does a context with an HBM
     // budget.
     // super_clump: the same for the super-bricks of two-level sorts.
-    std::map<int64_t, double> slab_clump, super_clump;
+    std::map<cam::AssignShape, double> slab_clump, super_clump;
     bool slabs_off = false;
     unsigned char *job_pin = nullptr;  // pinned readback buffer of cam_job_run
     size_t job_pin_bytes = 0;
@@ -254,7 +259,7 @@ struct AssignOut {
     // with defer the fullest brick is word [5] of the device statistics.
     double brick_est = 0.0;
     uint64_t brick_max = 0;
-    int64_t brick_shape = 0;  // slab_clump key of the mesh
+    AssignShape brick_shape{};  // slab_clump key of the mesh
     // The same for super-bricks (two-level sorts; word [6] with defer).
     double super_est = 0.0;
     uint64_t super_max = 0;

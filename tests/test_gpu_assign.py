@@ -452,3 +452,39 @@ def test_nonfinite_weight_leaves_the_mesh(n, npart, bad):
         assert abs(float(mesh.double().sum()) - npart) <= 1e-5 * npart
     finally:
         c.close()
+
+
+def _deposits(c, call):
+    """(result, deposit launches) of one call: two when it ran again exactly."""
+    c.profile(True)
+    c.profile_read(True)
+    r = call()
+    n = c.profile_read(True)["assign_deposit"][0]
+    c.profile(False)
+    return r, n
+
+
+def _layered(npart, box, period, seed):
+    """Uniform in x and z, the lower half of every `period` along y."""
+    import torch
+    gen = torch.Generator(device="cuda").manual_seed(seed)
+    xs = [torch.rand(npart, device="cuda", generator=gen) * box for _ in range(3)]
+    xs[1] = (xs[1] / period).floor() * period + (xs[1] % period) * 0.5
+    return xs
+
+
+def test_slabs_are_kept_by_brick_extent():
+    # layers 8 cells apart: even over bricks of 8 cells, which a million
+    # particles get, twice the mean in every second brick of 4, which five
+    # million get.  Calls of both in turn settle on slabs for the one and
+    # exact counts for the other, none runs twice.
+    from cosmicatlas_b200.api import Context
+    n, box = 64, 64.0
+    few, many = _layered(1_050_000, box, 8.0, 1), _layered(5_000_000, box, 8.0, 2)
+    g = make_grid(n, box)
+    c = Context()
+    try:
+        runs = [_deposits(c, lambda: c.assign(*xs, None, g, NGP, F32))[1] for _ in range(5) for xs in (few, many)]
+        assert runs[4:] == [1] * 6, runs
+    finally:
+        c.close()
