@@ -1136,9 +1136,9 @@ static void assign_impl(cam_ctx *ctx, const float *x, const float *y, const floa
         per *= 2;
     }
     // Slabs (deferred jobs): every brick gets a fixed slab of the payload,
-    // sized from the clumping the last exact job run of this mesh shape
-    // measured (a slab that overflows makes the job rerun exactly, which
-    // measures again); no count pass and no scan then, and the scatter
+    // sized from the clumping the exact runs of this mesh shape measured (a
+    // slab that overflows makes the call rerun exactly, which measures
+    // again); no count pass and no scan then, and the scatter
     // gathers the statistics.  With two levels the super-bricks get slabs of
     // their own the same way.  Only while the slabs stay within twice the
     // expected records (or 2^20 records), three times with two levels: one
@@ -1158,12 +1158,12 @@ static void assign_impl(cam_ctx *ctx, const float *x, const float *y, const floa
         const auto is = ctx->super_clump.find(shape);
         const bool two = sg.count > 0;
         if (it != ctx->slab_clump.end() && (!two || is != ctx->super_clump.end())) {
-            const uint64_t cap = slab_capacity(it->second * est_brick);
+            const uint64_t cap = slab_capacity(it->second.value * est_brick);
             const double room = std::max((two ? 3.0 : 2.0) * (double)np * f, (double)(1u << 20));
             bool fits = (double)nb * (double)cap <= room && (uint64_t)nb * cap < (1ull << 32) &&
                         (uint64_t)nb * cap * sizeof(uint4) <= ctx->device_bytes / 4;
             if (two) {
-                const uint64_t scap = slab_capacity(is->second * est_super);
+                const uint64_t scap = slab_capacity(is->second.value * est_super);
                 fits = fits && (double)sg.count * (double)scap <= 2.0 * (double)np + (double)(1u << 20) &&
                        (uint64_t)sg.count * scap + beyond < (1ull << 32);
                 if (fits) sg.cap = (uint32_t)scap;

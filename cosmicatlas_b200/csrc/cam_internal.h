@@ -67,6 +67,34 @@ struct FftPlan;  // cam_fft.cu
 // (they depend on the number of particles) and scheme.
 using AssignShape = std::array<int64_t, 7>;
 
+// The clumping that slabs are sized from.  A larger measurement counts at
+// once; a smaller one only after four in a row (then the largest of them):
+// where smooth and clumped catalogues of one shape come in turn, the smooth
+// one would otherwise shrink the slabs for the clumped one, which overflows
+// and runs twice.  An exact run costs a quarter of a run with slabs more (CIC,
+// 16.8 M particles onto 256^3: 423 us with slabs, 521 exact; 134 M onto 512^3:
+// 3.96 and 5.38 ms), so four exact runs cost about what one overflow does.
+struct Clump {
+    double value = 0.0;  // 0: not measured yet
+    void measured(double m)
+    {
+        if (m >= value) {
+            value = m;
+            lower = 0;
+            return;
+        }
+        seen = lower == 0 ? m : (m > seen ? m : seen);
+        if (++lower == 4) {
+            value = seen;
+            lower = 0;
+        }
+    }
+
+private:
+    double seen = 0.0;  // largest of the last `lower` measurements, all below value
+    int lower = 0;
+};
+
 struct ProfRecord {
     const char *name;
     cudaEvent_t start, stop;
@@ -100,13 +128,13 @@ struct cam_ctx {
     uint64_t asg_cap = 0;    // payload records of deferred assignments (grow-only)
     // Slabs of deferred assignments, per mesh shape: the
     // fullest brick's expected records over those of a uniform catalogue,
-    // as the last exact job run of that shape measured them (Poisson noise
-    // taken out).  No entry until a job of the shape has run exactly.
+    // as the exact runs of that shape measured them (Poisson noise taken
+    // out).  No entry until a call of the shape has run exactly.
     // slabs_off: always the exact path (the server's contexts, whose
     // admission budgets the exact payload); so does a context with an HBM
     // budget.
     // super_clump: the same for the super-bricks of two-level sorts.
-    std::map<cam::AssignShape, double> slab_clump, super_clump;
+    std::map<cam::AssignShape, cam::Clump> slab_clump, super_clump;
     bool slabs_off = false;
     unsigned char *job_pin = nullptr;  // pinned readback buffer of cam_job_run
     size_t job_pin_bytes = 0;

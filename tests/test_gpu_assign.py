@@ -488,3 +488,29 @@ def test_slabs_are_kept_by_brick_extent():
         assert runs[4:] == [1] * 6, runs
     finally:
         c.close()
+
+
+@pytest.mark.parametrize("n,npart", [(64, 1_050_000), (384, 1_200_000)])
+def test_alternating_catalogues_run_once(n, npart):
+    # a smooth and a clumped catalogue of one mesh in turn (one level of
+    # sorting and two): after the first pair none runs twice; once only
+    # smooth ones come, slabs are used again
+    import torch
+    from cosmicatlas_b200.api import Context
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    smooth = [torch.rand(npart, device="cuda", generator=gen) * 100.0 for _ in range(3)]
+    clumped = [v.clone() for v in smooth]
+    clumped[0][: npart // 2] *= 0.125
+    g = make_grid(n, 100.0)
+    c = Context()
+    try:
+        runs = [_deposits(c, lambda: c.assign(*xs, None, g, NGP, F32))[1] for _ in range(5) for xs in (smooth, clumped)]
+        assert runs[2:] == [1] * 8, runs
+        for _ in range(6):
+            c.assign(*smooth, None, g, NGP, F32)
+        c.profile(True)
+        c.profile_read(True)
+        c.assign(*smooth, None, g, NGP, F32)
+        assert "assign_bin_count" not in c.profile_read(True)
+    finally:
+        c.close()
