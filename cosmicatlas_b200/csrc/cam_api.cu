@@ -422,8 +422,14 @@ void keep_clumps(cam_ctx *ctx, const AssignOut &out, const unsigned long long *h
 {
     const uint64_t bmax = out.defer ? (hstats[5] & 0xffffffffu) : out.brick_max;
     const uint64_t smax = out.defer ? (hstats[6] & 0xffffffffu) : out.super_max;
-    if (bmax && out.brick_est > 0.0) ctx->slab_clump[out.brick_shape].measured(slab_clump_of(bmax, out.brick_est));
-    if (smax && out.super_est > 0.0) ctx->super_clump[out.brick_shape].measured(slab_clump_of(smax, out.super_est));
+    if (!bmax || out.brick_est <= 0.0) return;
+    SlabClump &c = ctx->slab_clump[out.brick_shape];
+    c.brick.measured(slab_clump_of(bmax, out.brick_est));
+    ++c.since_super;
+    if (smax && out.super_est > 0.0) {
+        c.super.measured(slab_clump_of(smax, out.super_est));
+        c.since_super = 0;
+    }
 }
 
 // One assignment call: a deferred run (see AssignOut) and, if its slabs or

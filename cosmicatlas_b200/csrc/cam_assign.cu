@@ -1155,26 +1155,30 @@ static void assign_impl(cam_ctx *ctx, const float *x, const float *y, const floa
     uint32_t slab = 0;
     if (out.defer && plain_ctx && np > 0) {
         const auto it = ctx->slab_clump.find(shape);
-        const auto is = ctx->super_clump.find(shape);
-        const bool two = sg.count > 0;
-        if (it != ctx->slab_clump.end() && (!two || is != ctx->super_clump.end())) {
-            const uint64_t cap = slab_capacity(it->second.value * est_brick);
+        if (it != ctx->slab_clump.end()) {
+            SlabClump &clump = it->second;
+            const bool two = sg.count > 0;
+            const uint64_t cap = slab_capacity(clump.brick.value * est_brick);
             const double room = std::max((two ? 3.0 : 2.0) * (double)np * f, (double)(1u << 20));
-            bool fits = (double)nb * (double)cap <= room && (uint64_t)nb * cap < (1ull << 32) &&
-                        (uint64_t)nb * cap * sizeof(uint4) <= ctx->device_bytes / 4;
-            if (two) {
-                const uint64_t scap = slab_capacity(is->second.value * est_super);
-                fits = fits && (double)sg.count * (double)scap <= 2.0 * (double)np + (double)(1u << 20) &&
-                       (uint64_t)sg.count * scap + beyond < (1ull << 32);
-                if (fits) sg.cap = (uint32_t)scap;
-            }
+            const bool bricks_fit = (double)nb * (double)cap <= room && (uint64_t)nb * cap < (1ull << 32) &&
+                                    (uint64_t)nb * cap * sizeof(uint4) <= ctx->device_bytes / 4;
             // With more than 128 super-bricks the exact counts of two levels
             // cost more than their longer runs save (768^3, 453 M TSC
             // particles, 216 of them: counts 5.0 ms, sort 3.4, records 8.0;
-            // one level 4.45 and 8.8), and a shape that has its clumping
-            // measured and is too clumped for slabs has no more use for them.
+            // one level 4.45 and 8.8), and a shape too clumped for slabs runs
+            // exactly in one level, which does not measure its super-bricks.
+            // If the bricks have come to fit since, they are measured anew.
+            if (sg.count > 128 && bricks_fit && clump.since_super >= 4) clump.super = Clump{};
+            bool fits = bricks_fit;
+            if (two) {
+                const uint64_t scap = slab_capacity(clump.super.value * est_super);
+                fits = fits && clump.super.value > 0.0 &&
+                       (double)sg.count * (double)scap <= 2.0 * (double)np + (double)(1u << 20) &&
+                       (uint64_t)sg.count * scap + beyond < (1ull << 32);
+                if (fits) sg.cap = (uint32_t)scap;
+            }
             if (fits) slab = (uint32_t)cap;
-            else if (sg.count > 128) sg = SuperGeom{};
+            else if (sg.count > 128 && clump.super.value > 0.0) sg = SuperGeom{};
         }
     }
     const bool two = sg.count > 0;

@@ -94,6 +94,11 @@ private:
     double seen = 0.0;  // largest of the last `lower` measurements, all below value
     int lower = 0;
 };
+// Of a shape's bricks and, for two-level sorts, its super-bricks.
+struct SlabClump {
+    Clump brick, super;
+    int since_super = 0;  // exact runs since one measured the super-bricks
+};
 
 struct ProfRecord {
     const char *name;
@@ -133,8 +138,7 @@ struct cam_ctx {
     // slabs_off: always the exact path (the server's contexts, whose
     // admission budgets the exact payload); so does a context with an HBM
     // budget.
-    // super_clump: the same for the super-bricks of two-level sorts.
-    std::map<cam::AssignShape, cam::Clump> slab_clump, super_clump;
+    std::map<cam::AssignShape, cam::SlabClump> slab_clump;
     bool slabs_off = false;
     unsigned char *job_pin = nullptr;  // pinned readback buffer of cam_job_run
     size_t job_pin_bytes = 0;

@@ -514,3 +514,27 @@ def test_alternating_catalogues_run_once(n, npart):
         assert "assign_bin_count" not in c.profile_read(True)
     finally:
         c.close()
+
+
+def test_super_bricks_are_measured_again():
+    # 768^3 sorts by more than 128 super-bricks: after clumped catalogues,
+    # which run exactly in one level, smooth ones come back to slabs
+    import torch
+    from cosmicatlas_b200.api import Context
+    n, npart = 768, 4_000_000
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    smooth = [torch.rand(npart, device="cuda", generator=gen) * 1000.0 for _ in range(3)]
+    clumped = [smooth[0] * 0.04, smooth[1], smooth[2]]
+    g = make_grid(n, 1000.0)
+    mesh = torch.empty((n, n, n), device="cuda")
+    c = Context()
+    try:
+        for xs in [clumped] * 2 + [smooth] * 8:
+            c.assign(*xs, None, g, NGP, F32, out=mesh)
+        c.profile(True)
+        c.profile_read(True)
+        c.assign(*smooth, None, g, NGP, F32, out=mesh)
+        names = c.profile_read(True)
+        assert "assign_super_sort" in names and "assign_bin_count" not in names, sorted(names)
+    finally:
+        c.close()
