@@ -109,6 +109,17 @@ void *scratch(cam_ctx *ctx, const char *name, size_t bytes)
     return p;
 }
 
+void drop_scratch(cam_ctx *ctx, const char *name)
+{
+    const auto it = ctx->bufs.find(name);
+    if (it == ctx->bufs.end() || !it->second.ptr) return;
+    std::lock_guard<std::mutex> lk(alloc_mutex());
+    ctx->gen++;
+    CAM_CUDA_TRY(cudaFreeAsync(it->second.ptr, ctx->stream));
+    ctx->used -= it->second.cap;
+    it->second = DevBuf{};
+}
+
 unsigned *device_error_word(cam_ctx *ctx)
 {
     if (!ctx->err_word) {
@@ -432,9 +443,39 @@ void keep_clumps(cam_ctx *ctx, const AssignOut &out, const unsigned long long *h
     }
 }
 
-// One assignment call: a deferred run (see AssignOut) and, if its slabs or
-// its payload estimate fell short, an exact one; the host waits once in the
-// common case.
+// One call of an assignment or a job: a deferred run (see AssignOut), unless
+// `exact`, and an exact one if attempt(true) returns that its slabs or its
+// payload estimate fell short.  Slabs, the payload estimate and the particles
+// sorted by super-brick take memory for speed alone, up to a fixed share of
+// the device, which others may have filled: where an allocation fails they
+// are given back, and this call and the next 63 run exactly in one level.
+// Not with an HBM budget, which sizes the exact path by itself.
+template <typename F>
+void run_as_fits(cam_ctx *ctx, bool exact, F &&attempt)
+{
+    auto fits = [&](bool defer, bool &again) {
+        try {
+            again = attempt(defer);
+            return true;
+        } catch (const Error &e) {
+            if (e.code != CAM_E_NOMEM || ctx->budget || ctx->lean) throw;
+        }
+        drop_scratch(ctx, "asg.part");
+        drop_scratch(ctx, "asg.payload");
+        ctx->asg_cap = 0;
+        ctx->lean = 64;
+        return false;
+    };
+    struct Count {
+        cam_ctx *c;
+        ~Count() { c->lean -= c->lean > 0; }
+    } count{ctx};
+    bool again = true;
+    if (!exact && !ctx->lean) fits(true, again);
+    if (again && !fits(false, again)) attempt(false);
+}
+
+// One assignment call; the host waits once in the common case.
 void assign_call(cam_ctx *ctx, const DevParticles &d, const cam_grid &g, int scheme, AssignOut &out, size_t out_bytes,
                  void *host_out, cam_assign_stats *stats)
 {
@@ -443,8 +484,8 @@ void assign_call(cam_ctx *ctx, const DevParticles &d, const cam_grid &g, int sch
     // a context with a budget, and a catalogue whose records would fill a
     // quarter of the device, sizes its payload exactly
     const bool exact = ctx->budget || (uint64_t)d.n * 8 * sizeof(uint4) > ctx->device_bytes / 4;
-    for (int pass = exact ? 1 : 0; pass < 2; ++pass) {
-        out.defer = pass == 0;
+    run_as_fits(ctx, exact, [&](bool defer) {
+        out.defer = defer;
         assign_device(ctx, d.x, d.y, d.z, d.w, d.n, g, scheme, out);
         Publish p;
         p.add(assign_stats(ctx), 64, 0);
@@ -452,8 +493,8 @@ void assign_call(cam_ctx *ctx, const DevParticles &d, const cam_grid &g, int sch
         publish(ctx, p, pin);
         CAM_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
         keep_clumps(ctx, out, hstats);
-        if (!(out.defer && (hstats[3] & 0xffffffffu))) break;
-    }
+        return defer && (hstats[3] & 0xffffffffu) != 0;
+    });
     CAM_REQUIRE(!d.w || (unsigned)(hstats[1] & 0xffffffffu) < 0x7f800000u, CAM_E_NONFINITE,
                 "a particle weight is NaN or infinite");
     if (host_out) {
@@ -1286,7 +1327,7 @@ int cam_job_run(cam_ctx *ctx, const cam_job_desc *job, cam_job_result *res)
             }
             return false;
         };
-        if (run(true)) run(false);
+        run_as_fits(ctx, false, run);
     });
 }
 

@@ -1113,7 +1113,7 @@ static void assign_impl(cam_ctx *ctx, const float *x, const float *y, const floa
     const bool smem_hist = nb <= kSmemBricks;
     // Two levels of sorting when the records would otherwise leave a tile in
     // runs of a few per brick.
-    const bool plain_ctx = !ctx->sync_free && !ctx->slabs_off && !ctx->budget;
+    const bool plain_ctx = !ctx->sync_free && !ctx->slabs_off && !ctx->budget && !ctx->lean;
     SuperGeom sg{};
     if (plain_ctx && nb > kStageBins && np >= kTwoLevelParticles &&
         (uint64_t)np * sizeof(float4) <= ctx->device_bytes / 16 && geom.safe[0] > 0.f && geom.safe[1] > 0.f &&
@@ -1144,7 +1144,8 @@ static void assign_impl(cam_ctx *ctx, const float *x, const float *y, const floa
     // expected records (or 2^20 records), three times with two levels: one
     // level's short runs slow down as the slabs spread them over more memory.
     // A context with an HBM budget keeps the exact path, whose payload the
-    // budget was sized for; nor do slabs take more than a quarter of the
+    // budget was sized for, and so does one whose device is short of memory
+    // (run_as_fits); nor do slabs take more than a quarter of the
     // device's memory, or sorted particles a sixteenth.
     const double est_brick = (double)np * f / (double)nb;
     const AssignShape shape{g.n[0], g.n[1], g.n[2], g.b[0], g.b[1], g.b[2], SCHEME};

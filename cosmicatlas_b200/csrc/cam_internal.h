@@ -140,6 +140,7 @@ struct cam_ctx {
     // budget.
     std::map<cam::AssignShape, cam::SlabClump> slab_clump;
     bool slabs_off = false;
+    int lean = 0;  // calls left that spend no memory on speed (run_as_fits)
     unsigned char *job_pin = nullptr;  // pinned readback buffer of cam_job_run
     size_t job_pin_bytes = 0;
     // bumped whenever a scratch buffer is (re)allocated or freed, so that
@@ -223,6 +224,8 @@ void check_device_error(cam_ctx *ctx);
 // Returns a device buffer of at least `bytes`, reallocating (and
 // synchronising the stream) if the cached one is too small.
 void *scratch(cam_ctx *ctx, const char *name, size_t bytes);
+// Frees one such buffer, in stream order.
+void drop_scratch(cam_ctx *ctx, const char *name);
 void release_all(cam_ctx *ctx);
 // Serialises device allocation/free against stream capture in other threads.
 std::mutex &alloc_mutex();

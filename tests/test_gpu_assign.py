@@ -538,3 +538,47 @@ def test_super_bricks_are_measured_again():
         assert "assign_super_sort" in names and "assign_bin_count" not in names, sorted(names)
     finally:
         c.close()
+
+
+@pytest.mark.parametrize("job", [False, True])
+def test_short_of_memory_runs_exactly(job):
+    # All but 0.9 GB of the device is taken.  30 M particles: 0.56 GB of CIC
+    # records on 512^3, for which the two-level sort wants 0.48 GB beside
+    # them and the payload estimate a quarter more; 0.65 GB of TSC records and
+    # 0.14 GB of mesh and spectrum of a 256^3 job.
+    import torch
+    from cosmicatlas_b200 import _lib as L
+    from cosmicatlas_b200.api import Context, alloc_stats
+    npart = 30_000_000
+    gen = torch.Generator(device="cuda").manual_seed(8)
+    xs = [torch.rand(npart, device="cuda", generator=gen) * 1000.0 for _ in range(3)]
+    mesh = None if job else torch.empty((512, 512, 512), device="cuda")
+
+    def call(c):
+        if job:
+            return c.job(*xs, None, make_grid(256, 1000.0), TSC, F32, pk=Context.pk_opts(TSC, nbins=128))["pk"].pk
+        c.assign(*xs, None, make_grid(512, 1000.0), CIC, F32, out=mesh)
+        return mesh.cpu().numpy()
+
+    c = Context()
+    want = call(c)
+    c.close()
+    c = Context()
+    hog = None
+    try:
+        torch.cuda.synchronize()
+        torch.cuda.empty_cache()
+        assert L.lib().cam_pool_trim(0) == L.CAM_OK
+        hog = torch.empty(torch.cuda.mem_get_info()[0] - 900_000_000, dtype=torch.uint8, device="cuda")
+        alloc_stats(reset=True)
+        got = [call(c) for _ in range(3)]
+        assert alloc_stats()["failures"] > 0
+        del hog
+        torch.cuda.empty_cache()
+        got.append(call(c))
+        assert all(np.array_equal(g, want) for g in got)
+    finally:
+        hog = None
+        c.close()
+        torch.cuda.empty_cache()
+        L.lib().cam_pool_trim(0)
