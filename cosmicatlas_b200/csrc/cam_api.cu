@@ -84,6 +84,12 @@ void *scratch(cam_ctx *ctx, const char *name, size_t bytes)
         // it back to the device and try once more
         cudaGetLastError();
         alloc_counters().failures++;
+        const auto part = ctx->bufs.find("asg.part");
+        if (!ctx->assigning && part != ctx->bufs.end() && part->second.ptr) {
+            CAM_CUDA_TRY(cudaFreeAsync(part->second.ptr, ctx->stream));
+            ctx->used -= part->second.cap;
+            part->second = DevBuf{};
+        }
         cudaDeviceSynchronize();
         cudaMemPoolTrimTo(pool, 0);
         e = cudaMallocFromPoolAsync(&p, want, pool, ctx->stream);

@@ -1384,6 +1384,11 @@ void assign_device(cam_ctx *ctx, const float *x, const float *y, const float *z,
     CAM_REQUIRE(np == 0 || (x && y && z), CAM_E_INVAL, "null particle coordinates");
     CAM_REQUIRE(np < (1ll << 31), CAM_E_UNSUPPORTED, "more than 2^31 particles per call");
     const AssignGeom g = make_geom(grid, scheme, np);
+    struct Assigning {
+        cam_ctx *c;
+        explicit Assigning(cam_ctx *ctx) : c(ctx) { c->assigning = true; }
+        ~Assigning() { c->assigning = false; }
+    } assigning(ctx);
     if (out.precision == -1)
         CAM_REQUIRE(scheme == CAM_NGP && w == nullptr, CAM_E_INVAL, "integer counts need unweighted NGP");
     switch (scheme) {

@@ -140,6 +140,7 @@ struct cam_ctx {
     // budget.
     std::map<cam::AssignShape, cam::SlabClump> slab_clump;
     bool slabs_off = false;
+    bool assigning = false;  // asg.part is being written or read (assign_device)
     int lean = 0;  // calls left that spend no memory on speed (run_as_fits)
     unsigned char *job_pin = nullptr;  // pinned readback buffer of cam_job_run
     size_t job_pin_bytes = 0;
@@ -221,8 +222,9 @@ struct StreamScope {
 unsigned *device_error_word(cam_ctx *ctx);
 void check_device_error(cam_ctx *ctx);
 
-// Returns a device buffer of at least `bytes`, reallocating (and
-// synchronising the stream) if the cached one is too small.
+// Returns a device buffer of at least `bytes`, reallocating (in stream order)
+// if the cached one is too small.  Where that fails, the particles sorted by
+// super-brick, kept for speed alone, are given up first.
 void *scratch(cam_ctx *ctx, const char *name, size_t bytes);
 // Frees one such buffer, in stream order.
 void drop_scratch(cam_ctx *ctx, const char *name);

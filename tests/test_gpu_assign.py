@@ -582,3 +582,47 @@ def test_short_of_memory_runs_exactly(job):
         c.close()
         torch.cuda.empty_cache()
         L.lib().cam_pool_trim(0)
+
+
+def test_sorted_particles_make_room_for_other_calls():
+    # a 512^3 assignment leaves 0.5 GB of sorted particles in its context;
+    # with 0.15 GB free the 0.23 GB spectrum of a 384^3 transform takes
+    # their place, and the next assignment is the same again
+    import torch
+    from cosmicatlas_b200 import _lib as L
+    from cosmicatlas_b200.api import Context
+    gen = torch.Generator(device="cuda").manual_seed(9)
+    xs = [torch.rand(30_000_000, device="cuda", generator=gen) * 1000.0 for _ in range(3)]
+    mesh = torch.empty((512, 512, 512), device="cuda")
+    field = torch.randn((384, 384, 384), device="cuda", generator=gen)
+    spec = torch.empty((384, 384, 193), dtype=torch.complex64, device="cuda")
+    g = make_grid(512, 1000.0)
+    c = Context()
+    hog = None
+
+    def transform():
+        c._check(c._lib.cam_fft_r2c(c.h, 384, F32, L.ptr(field), L.ptr(spec), L.MEM_DEVICE))
+        return spec.cpu().numpy()
+
+    try:
+        want = Context()
+        try:
+            want_spec = want.fft_r2c(field).cpu().numpy()
+        finally:
+            want.close()
+        c.assign(*xs, None, g, CIC, F32, out=mesh)
+        want_mesh = mesh.cpu().numpy()
+        torch.cuda.synchronize()
+        torch.cuda.empty_cache()
+        assert L.lib().cam_pool_trim(0) == L.CAM_OK
+        hog = torch.empty(torch.cuda.mem_get_info()[0] - 150_000_000, dtype=torch.uint8, device="cuda")
+        assert np.array_equal(transform().view(np.float32), want_spec.view(np.float32))
+        del hog
+        torch.cuda.empty_cache()
+        c.assign(*xs, None, g, CIC, F32, out=mesh)
+        assert np.array_equal(mesh.cpu().numpy(), want_mesh)
+    finally:
+        hog = None
+        c.close()
+        torch.cuda.empty_cache()
+        L.lib().cam_pool_trim(0)
