@@ -62,6 +62,10 @@ constexpr int kDlMaxN = 128;
 constexpr int kDlMaxBricks = 1024;  // bricks of one job (shared counters)
 constexpr int kDlPoints = 8192;     // complex points of one FFT tile (8 per thread)
 constexpr size_t kDlSmem = 104 * 1024;
+// the deposit tile of the largest brick (16 cells along x, see make_geom) and
+// the warps' sums behind it
+static_assert((size_t)asg::tile_words(16) * sizeof(uint32_t) + kDlWarps * sizeof(long long) <= kDlSmem,
+              "a brick's deposit tile does not fit the job's shared memory");
 
 enum : unsigned { DL_RUNNING = 0, DL_STOPPED = 1, DL_IDLE = 2 };
 
@@ -803,8 +807,6 @@ int cam_devloop_submit(cam_devloop *l, const cam_job_desc *job, uint64_t *id)
         const cam_grid g = resolved_grid(job->grid);
         J.g = make_geom(g, job->scheme, job->parts.n);
         CAM_REQUIRE((int64_t)J.g.nb[0] * J.g.nb[1] * J.g.nb[2] <= kDlMaxBricks, CAM_E_UNSUPPORTED, "too many bricks");
-        CAM_REQUIRE((size_t)(J.g.b[0] + 2) * (J.g.b[1] + 2) * (J.g.b[2] + 2) * 8 <= kDlSmem, CAM_E_UNSUPPORTED,
-                    "brick tile too large");
         J.x = job->parts.x;
         J.y = job->parts.y;
         J.z = job->parts.z;
