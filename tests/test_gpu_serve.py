@@ -188,3 +188,20 @@ def test_server_failed_job_and_poll(ctx):
         st = srv.stats(reset=True)
         assert st["failed"] == 1
         assert srv.stats()["completed"] == 0
+
+
+def test_batch_refuses_host_arrays_called_device(ctx):
+    # checked on the host before anything is launched; the context goes on
+    n, box = 32, 320.0
+    x, y, z = synth.clumped(20_000, box, 200, 2.0, 0.8, seed=3)
+    specs = [JobSpec(x, y, z, None, grid=make_grid(n, box), scheme=CIC, pk=Context.pk_opts(CIC, nbins=16))
+             for _ in range(3)]
+    want = ctx.batch(specs)[0]["pk"].pk.copy()
+    wrong = [JobSpec(x, y, z, None, grid=make_grid(n, box), scheme=CIC, pk=Context.pk_opts(CIC, nbins=16))
+             for _ in range(3)]
+    for s in wrong:
+        s.desc.parts.mem = L.MEM_DEVICE
+    with pytest.raises(CamError) as e:
+        ctx.batch(wrong)
+    assert e.value.code == -1
+    assert np.array_equal(ctx.batch(specs)[0]["pk"].pk, want)
