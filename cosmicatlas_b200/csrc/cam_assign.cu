@@ -161,9 +161,9 @@ append_kernel(const float *__restrict__ x, const float *__restrict__ y, const fl
 // tile (4.6 records at 256^3 with tiles of 8192); two levels write the
 // particles once more but both in long runs.  16.8 M particles onto 256^3
 // (2048 bricks), NGP, CIC, TSC: one level 216, 284, 325 us, two levels 316,
-// 410, 443, record by record 345, 441, 530.  134 M CIC particles onto 512^3
-// (16384 bricks, more than a tile counts): two levels 3.09 ms, record by
-// record 4.64.
+// 410, 443, record by record 345, 441, 530 (one level 190, 271, 306 with the
+// next tile's particles prefetched).  134 M CIC particles onto 512^3 (16384
+// bricks, more than a tile counts): two levels 3.09 ms, record by record 4.64.
 // Steps of a tile:
 //   1. each particle's record for its first brick (LEVEL 1: the particle)
 //      goes to its stage slot, and a shared counter per bin gives its rank
@@ -195,10 +195,14 @@ constexpr int kStageTile = 8192;   // particles per tile (13 bits in the queue)
 constexpr int stage_threads(int level) { return level == 0 ? 1024 : 256; }
 constexpr int stage_ctas(int level) { return 1024 / stage_threads(level); }
 constexpr size_t stage_budget(int level) { return (226 / stage_ctas(level) - 1) * 1024; }
-// bytes besides the 20 per record
-// Two levels where one level's tiles cannot count the bricks, for jobs with
-// tiles enough to fill the GPU twice.
+// Two levels where one level's tiles cannot count the bricks, from a million
+// particles on.  Uniform particles in slabs, two levels against record by
+// record: 384^3 CIC 260 and 236 us at 1 M, 325 and 308 at 4 M; 512^3 TSC 505
+// and 495 at 1 M, 605 and 591 at 4 M.  Both sides cross between 4 M and 30 M
+// (512^3, 67 M, counted exactly: CIC 2.94 and 3.32 ms, TSC 3.75 and 4.34), so
+// the line lies low: up to a tenth of a call is lost below the crossing.
 constexpr int64_t kTwoLevelParticles = 1000000;
+// bytes besides the 20 per record
 inline size_t stage_fixed(int level, int nbins)
 {
     return (size_t)nbins * 4 + (level == 2 ? (size_t)nbins * 8 + (kMaxSupers + 2) * 4 : 0);
@@ -1141,12 +1145,15 @@ static void assign_impl(cam_ctx *ctx, const float *x, const float *y, const floa
     // again); no count pass and no scan then, and the scatter
     // gathers the statistics.  With two levels the super-bricks get slabs of
     // their own the same way.  Only while the slabs stay within twice the
-    // expected records (or 2^20 records), three times with two levels: one
-    // level's short runs slow down as the slabs spread them over more memory.
+    // expected records (or 2^20 records), three times with two levels, which
+    // limits memory: slabs are the faster at any size (a layer of 1 to 6
+    // times the mean density: 16.8 M TSC particles onto 256^3 640-650 us with
+    // slabs of 1.1 to 6.8 times the records, 735-747 counted exactly; 67 M
+    // onto 512^3 2.99-3.00 and 3.75 ms).
     // A context with an HBM budget keeps the exact path, whose payload the
     // budget was sized for, and so does one whose device is short of memory
-    // (run_as_fits); nor do slabs take more than a quarter of the
-    // device's memory, or sorted particles a sixteenth.
+    // (run_as_fits); nor do slabs take more than a quarter of the device's
+    // memory, or sorted particles a sixteenth, an eighth in slabs.
     const double est_brick = (double)np * f / (double)nb;
     const AssignShape shape{g.n[0], g.n[1], g.n[2], g.b[0], g.b[1], g.b[2], SCHEME};
     double est_super = (double)np;
@@ -1163,11 +1170,13 @@ static void assign_impl(cam_ctx *ctx, const float *x, const float *y, const floa
             const double room = std::max((two ? 3.0 : 2.0) * (double)np * f, (double)(1u << 20));
             const bool bricks_fit = (double)nb * (double)cap <= room && (uint64_t)nb * cap < (1ull << 32) &&
                                     (uint64_t)nb * cap * sizeof(uint4) <= ctx->device_bytes / 4;
-            // With more than 128 super-bricks the exact counts of two levels
-            // cost more than their longer runs save (768^3, 453 M TSC
-            // particles, 216 of them: counts 5.0 ms, sort 3.4, records 8.0;
-            // one level 4.45 and 8.8), and a shape too clumped for slabs runs
-            // exactly in one level, which does not measure its super-bricks.
+            // With more than 128 super-bricks a shape too clumped for slabs
+            // runs exactly in one level, which does not measure its
+            // super-bricks.  Particles in lattice order, whose records append
+            // to a few bricks at a time, gain by it (768^3, 453 M TSC
+            // particles: counts 4.45 ms and records 8.8, in two levels 5.0 +
+            // 3.4 + 8.0), particles in random order lose (226 M CIC onto
+            // 768^3 11.9 and 10.0 ms, 131 M onto 640^3 6.8 and 5.7).
             // If the bricks have come to fit since, they are measured anew.
             if (sg.count > 128 && bricks_fit && clump.since_super >= 4) clump.super = Clump{};
             bool fits = bricks_fit;
@@ -1220,7 +1229,9 @@ static void assign_impl(cam_ctx *ctx, const float *x, const float *y, const floa
         const double each = 20.0 * fr + (level == 1 ? 0.0 : 2.0);
         const int64_t most = std::max<int64_t>(512, std::min<int64_t>(kStageTile, (int64_t)((double)bytes / each)));
         // a batch's jobs run beside each other: fewer, larger tiles cost less
-        // in all (64 jobs of 64^3: 4.82 ms split over 148, 4.51 over 32)
+        // in all (32 jobs, CIC, split over 16, 32, 64, 148 CTAs: 32^3 with
+        // 300,000 particles 1.09, 1.10, 1.10, 1.16 ms; 64^3 with 262,144 1.02,
+        // 1.02, 1.05, 1.14; 128^3 with 600,000 1.93, 1.94, 1.98, 1.98)
         const int64_t ctas = ctx->sync_free ? 32 : stage_ctas(level) * kNumSMs;
         const int64_t rounds = std::max<int64_t>(1, (np + ctas * most - 1) / (ctas * most));
         const int64_t even = (np + ctas * rounds - 1) / (ctas * rounds);

@@ -320,9 +320,9 @@ __device__ __forceinline__ bool append_one(float px, float py, float pz, float w
     return true;
 }
 
-// Cell sum q (units of 2^-s) as the output type; sc = 2^-s, so q * sc is
-// exact in double (|q| < 2^63, -97 <= s <= 180) and the float output is one
-// rounding of the exact value.
+// Cell sum q (units of 2^-s) as the output type; sc = 2^-s (-97 <= s <= 180).
+// Up to |q| = 2^53 q * sc is exact in double and the float output one rounding
+// of the exact value; a larger sum is rounded to double first.
 template <typename OutT>
 __device__ __forceinline__ OutT convert_out(long long q, int s, double sc);
 template <>

@@ -878,8 +878,9 @@ void rows_impl(cam_ctx *ctx, FftPlan *p, const void *in, void *out, void *nyq, i
                   ((LEN & (LEN - 1)) == 0 || (sizeof(T) == 4 && LEN >= 192))) {
         // pipelined r2c rows for the half lengths whose transforms fit the
         // register bound (192 and 384 spill a few words and still gain: 768^3
-        // 1454 -> 1398 us): one component, 16-byte aligned input, raw + padded
-        // tile within 200 KB
+        // 1454 -> 1398 us; rows of 24 and 48 would gain under 1 us of 13, at 48^3
+        // and 96^3): one component, 16-byte aligned input, raw + padded tile
+        // within 200 KB
         const size_t psmem = (size_t)rpc * len * sizeof(C) + smem;
         if (ncomp == 1 && ((uintptr_t)in % 16) == 0 && (len * sizeof(C)) % 16 == 0 && psmem <= 200 * 1024) {
             auto kp = fft_rows_r2c_pipe_kernel<T, LEN>;
