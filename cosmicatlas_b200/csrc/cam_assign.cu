@@ -1166,10 +1166,10 @@ static void assign_impl(cam_ctx *ctx, const float *x, const float *y, const floa
         if (it != ctx->slab_clump.end()) {
             SlabClump &clump = it->second;
             const bool two = sg.count > 0;
-            const uint64_t cap = slab_capacity(clump.brick.value * est_brick);
-            const double room = std::max((two ? 3.0 : 2.0) * (double)np * f, (double)(1u << 20));
-            const bool bricks_fit = (double)nb * (double)cap <= room && (uint64_t)nb * cap < (1ull << 32) &&
-                                    (uint64_t)nb * cap * sizeof(uint4) <= ctx->device_bytes / 4;
+            const double room = std::min({std::max((two ? 3.0 : 2.0) * (double)np * f, (double)(1u << 20)), 4294967295.0,
+                                          (double)(ctx->device_bytes / 4 / sizeof(uint4))});
+            const uint64_t cap = slab_within(clump.brick.value * est_brick, (uint64_t)(room / (double)nb) & ~(uint64_t)3);
+            const bool bricks_fit = cap > 0;
             // With more than 128 super-bricks a shape too clumped for slabs
             // runs exactly in one level, which does not measure its
             // super-bricks.  Particles in lattice order, whose records append
@@ -1181,11 +1181,11 @@ static void assign_impl(cam_ctx *ctx, const float *x, const float *y, const floa
             if (sg.count > 128 && bricks_fit && clump.since_super >= 4) clump.super = Clump{};
             bool fits = bricks_fit;
             if (two) {
-                const uint64_t scap = slab_capacity(clump.super.value * est_super);
-                fits = fits && clump.super.value > 0.0 &&
-                       (double)sg.count * (double)scap <= 2.0 * (double)np + (double)(1u << 20) &&
-                       (uint64_t)sg.count * scap + beyond < (1ull << 32);
-                if (fits) sg.cap = (uint32_t)scap;
+                const double sroom = std::min(2.0 * (double)np + (double)(1u << 20), 4294967295.0 - (double)beyond);
+                sg.cap = fits && clump.super.value > 0.0
+                             ? (uint32_t)slab_within(clump.super.value * est_super, (uint64_t)(sroom / sg.count) & ~(uint64_t)3)
+                             : 0u;
+                fits = sg.cap > 0;
             }
             if (fits) slab = (uint32_t)cap;
             else if (sg.count > 128 && clump.super.value > 0.0) sg = SuperGeom{};

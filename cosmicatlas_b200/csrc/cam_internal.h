@@ -319,6 +319,19 @@ inline double slab_clump_of(uint64_t m, double est)
     return std::max(1.0, (md - 4.0 * std::sqrt(md)) / est);
 }
 
+// Records per slab where at most `most` are allowed: slab_capacity of mu, or
+// all that is allowed if that still holds a fullest brick like the measured
+// one, or 0.  Catalogues near the limit differ by less than the margin of
+// 9/8: without the middle case the fullest of three made all of them count
+// exactly (density mesh of 235 us with slabs, 272 without).
+inline uint64_t slab_within(double mu, uint64_t most)
+{
+    const uint64_t want = slab_capacity(mu);
+    if (want <= most) return want;
+    const double root = 2.0 + std::sqrt(4.0 + mu);  // slab_clump_of undone
+    return root * root <= (double)most ? most : 0;
+}
+
 // Device statistics of the last assignment of a context:
 // [0] lost particles, [1] low word: bits of max |w|, [2] low word: payload
 // records, [3] low word: nonzero if the deferred payload overflowed,

@@ -626,3 +626,34 @@ def test_sorted_particles_make_room_for_other_calls():
         c.close()
         torch.cuda.empty_cache()
         L.lib().cam_pool_trim(0)
+
+
+def test_slabs_near_their_limit():
+    # bricks of 4 cells along x whose fullest holds 1.9 times the mean: more
+    # than the limit of two with the margin of 9/8, less without it.  In turn
+    # with an even catalogue both use slabs, the exact mesh is the same.
+    import torch
+    from cosmicatlas_b200.api import Context
+    npart = 1_050_000
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    even = [torch.rand(npart, device="cuda", generator=gen) * 64.0 for _ in range(3)]
+    layer = [v.clone() for v in even]
+    layer[0][: int(0.06 * npart)] /= 16.0
+    g = make_grid(64, 64.0)
+    c, exact = Context(), Context()
+    try:
+        want = {id(xs): exact.assign(*xs, None, g, NGP, F32).mesh for xs in (even, layer)}
+        for _ in range(2):
+            for xs in (even, layer):
+                c.assign(*xs, None, g, NGP, F32)
+        for xs in (even, layer) * 2:
+            c.profile(True)
+            c.profile_read(True)
+            got = c.assign(*xs, None, g, NGP, F32).mesh
+            names = c.profile_read(True)
+            c.profile(False)
+            assert names["assign_deposit"][0] == 1 and "assign_bin_count" not in names
+            assert bool((got == want[id(xs)]).all())
+    finally:
+        c.close()
+        exact.close()
