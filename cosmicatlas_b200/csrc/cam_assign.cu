@@ -935,17 +935,18 @@ deposit_kernel(const uint4 *__restrict__ payload, const uint32_t *__restrict__ s
     const uint32_t end = slab ? beg + min(slab_count[(int64_t)B * g.cstride], slab) : min(start[B + 1], nrec);
     RecordStream rec;
     rec.open(payload, beg, end, warp, kDepositThreads / 32, lane);
-    // a weight that is not finite, or records that found no room (the call
-    // fails, or runs again exactly): the mesh, which may be the caller's, is
-    // left as it is
-    if ((weighted && wstat[0] >= 0x7f800000u) || wstat[4] != 0u) {
-        if (host_ovf && blockIdx.x == 0 && threadIdx.x == 0 && wstat[4] != 0u) *host_ovf = 1u;
-        return;
-    }
+    const unsigned heaviest = weighted ? wstat[0] : 0u, overflow = wstat[4];
     const bool nonneg = !weighted || wstat[1] == 0u;
     const int s = fixed_scale(wstat, weighted, end - beg);
     // 2^s as two exact factors (s may exceed the float exponent range)
     const float f1 = scalbnf(1.0f, s / 2), f2 = scalbnf(1.0f, s - s / 2);
+    // a weight that is not finite, or records that found no room (the call
+    // fails, or runs again exactly): the mesh, which may be the caller's, is
+    // left as it is
+    if (heaviest >= 0x7f800000u || overflow != 0u) {
+        if (host_ovf && blockIdx.x == 0 && threadIdx.x == 0 && overflow != 0u) *host_ovf = 1u;
+        return;
+    }
     zero_tile(tile32, e, threadIdx.x, kDepositThreads);
     __syncthreads();
     deposit_records<SCHEME>(rec, e, f1, f2, nonneg, tile32);
