@@ -171,7 +171,8 @@ const char *cam_version(void);
  * Headers/massFunctions.h:12,18,26).  mesh_out (N1*N2*N3 values of the
  * chosen precision) is overwritten (the reference zeroes delta first).
  * Deterministic: integer keys, counting sort into mesh bricks, exact
- * fixed-point accumulation per cell; no float atomics. */
+ * fixed-point accumulation per cell; no float atomics.  A weight that is NaN
+ * or infinite returns CAM_E_NONFINITE and leaves mesh_out as it was. */
 int cam_assign(cam_ctx *ctx, const cam_particles *parts, const cam_grid *grid,
                int scheme, int precision, void *mesh_out, int out_mem,
                cam_assign_stats *stats);
@@ -305,13 +306,17 @@ int cam_konvolve(cam_ctx *ctx, const cam_grid *grid, const void *in, int precisi
 /* ---- one mesh job: particles -> mesh -> FFT -> P(k) [-> T-web] ----------
  * The plain per-call GPU path of one BAM iteration: the mesh and its
  * spectrum stay resident on the device between the stages, and the host
- * waits once, for the statistics and P(k) at the end.  A context's first
- * job of a mesh shape sorts the particles into mesh bricks exactly (count,
- * scan, scatter) and measures its fullest brick (and, on meshes of more than
- * 4096 bricks, its fullest group of bricks); later jobs and cam_assign calls
- * of that shape write every brick's records into a fixed slab sized from it
- * and skip the count.  A job whose records do not fit (its slabs or the
- * payload estimate) runs again exactly, so results never depend on the path. */
+ * waits once, for the statistics and P(k) at the end (with a T-web also for
+ * the assignment, while the transform runs).  A context's first call of a
+ * mesh shape -- sides, scheme, and the brick extents that go with the number
+ * of particles -- sorts the particles into mesh bricks exactly (count, scan,
+ * scatter) and measures its fullest brick (and, on meshes of more than 4096
+ * bricks, its fullest group of bricks); later jobs and cam_assign calls of
+ * that shape write every brick's records into a fixed slab sized from it and
+ * skip the count.  A job whose records do not fit (its slabs or the payload
+ * estimate) runs again exactly, so results never depend on the path; one
+ * that finds no device memory for it runs exactly at once.
+ */
 typedef struct {
     cam_particles parts;
     cam_grid grid;
